@@ -378,6 +378,23 @@ int rcv_render_backward_volpathsimple(const rcv_medium* medium, const rcv_sensor
                                       int32_t spp, const float* grad_img, float* grad_density,
                                       float* grad_albedo, void* stream);
 
+/* The same adjoint with scratch (device, 256-byte aligned, any contents):
+ * paths are traced once by a persistent launch that records their segments
+ * and shadow-walk steps, from which flat passes form the gradient (several
+ * times faster than one thread per path).  Films whose records do not fit go
+ * in several passes, and without enough scratch for one (or with DRT and no
+ * subsampling, whose second random stream has no fixed length) the call does
+ * what rcv_render_backward_volpathsimple does.  opts->tape_events_per_path
+ * bounds the recorded shadow steps (0 = 48 per path).  The _bytes function
+ * gives the scratch for the fewest passes (at most about 6 GB). */
+uint64_t rcv_volpathsimple_adjoint_workspace_bytes(int32_t width, int32_t height, int32_t spp);
+int rcv_render_backward_volpathsimple_ws(const rcv_medium* medium, const rcv_sensor* sensor,
+                                         const rcv_volpath_options* opts,
+                                         const rcv_volpathsimple_flags* flags, uint32_t seed,
+                                         int32_t spp, const float* grad_img, float* grad_density,
+                                         float* grad_albedo, void* workspace,
+                                         uint64_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------- surface scenes */
 #define RCV_MAX_SPHERES 8
 

@@ -263,6 +263,11 @@ SIGNATURES = {
         C.c_int,
         [P(Medium), P(Sensor), P(VolpathOptions), P(VpsFlags), C.c_uint32, C.c_int32, vp, vp, vp, vp],
     ),
+    "rcv_volpathsimple_adjoint_workspace_bytes": (C.c_uint64, [C.c_int32, C.c_int32, C.c_int32]),
+    "rcv_render_backward_volpathsimple_ws": (
+        C.c_int,
+        [P(Medium), P(Sensor), P(VolpathOptions), P(VpsFlags), C.c_uint32, C.c_int32, vp, vp, vp, vp, C.c_uint64, vp],
+    ),
     "rcv_surface_workspace_bytes": (C.c_uint64, [C.c_int32, C.c_int32]),
     "rcv_surface_prepare": (C.c_int, [P(SurfaceScene), vp]),
     "rcv_render_twostates_surface": (

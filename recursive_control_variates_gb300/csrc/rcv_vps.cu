@@ -28,9 +28,12 @@
 // on; it is restated as a distance from the majorant's exponential truncated
 // to the segment, weight = ratio-tracking transmittance / pdf.
 //
-// One thread per path, sequential: this integrator is the alternative
-// adjoint, and its recursive DRT paths do not fit the persistent queue's
-// phase machine.  The arithmetic follows the oracle's float sequence.
+// The arithmetic follows the oracle's float sequence.  The adjoint runs as
+// two persistent tracers and two flat gradient passes over what they record
+// (rcv_vps_trace.cuh); vps_kernel, one thread per path, renders the primal and
+// takes the adjoints whose second stream has no fixed number of draws per
+// segment (DRT without subsampling), the paths that a recording lost, and
+// callers without a workspace.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -38,16 +41,9 @@
 
 #include "rcv_common.h"
 #include "rcv_pack.cuh"
-#include "rcv_volume.cuh"
+#include "rcv_vps_trace.cuh"
 
 namespace rcv {
-
-struct VpsParams {
-  int32_t use_nee, use_drt, use_drt_subsampling, use_drt_mis;
-  uint32_t alt_seed;   // seed of the adjoint's second stream
-  int32_t pad;
-  float4* path_out;    // primal: per-path radiance
-};
 
 struct VpsSeg {
   V3 o, d;
@@ -393,9 +389,11 @@ __global__ void __launch_bounds__(128) vps_kernel(const __grid_constant__ VolJob
   const float mu = J.scale * bits_to_float(__ldg(J.maxbits + 1));
   const Vps<kEnv> v{J, P, mu, 1.0f / mu};
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t path = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; path < J.path_count; path += stride) {
-    const int pix = (int)(path / J.spp);
-    const uint32_t sid = (uint32_t)path;  // pixel * spp + sample
+  const bool listed = kAdj && P.lost_list != nullptr;
+  const int64_t n = listed ? (int64_t)*P.lost_count : J.path_count;
+  for (int64_t path = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; path < n; path += stride) {
+    const uint32_t sid = listed ? P.lost_list[path] : (uint32_t)path;  // pixel * spp + sample
+    const int pix = (int)(sid / (uint32_t)J.spp);
     if (kAdj) {
       const float* g = J.grad_img + (int64_t)pix * 3;
       const float fs = (float)J.spp;
@@ -405,6 +403,169 @@ __global__ void __launch_bounds__(128) vps_kernel(const __grid_constant__ VolJob
       P.path_out[path] = make_float4(L.x, L.y, L.z, 0.0f);
     }
   }
+}
+
+template <int kMode, bool kSG, bool kEnv>
+__global__ void __launch_bounds__(kVpsBlock, 5) vps_trace_kernel(const __grid_constant__ VolJob J,
+                                                                 const __grid_constant__ VpsParams P,
+                                                                 const __grid_constant__ Queue Q) {
+  trace_vps<kMode, kSG, kEnv>(J, P, Q);
+}
+
+__device__ __forceinline__ V3 vps_dL(const VolJob& J, int pix) {
+  const float* g = J.grad_img + (int64_t)pix * 3;
+  const float fs = (float)J.spp;
+  return V3{g[0] / fs, g[1] / fs, g[2] / fs};
+}
+
+// Flat pass over the segment records and the DRT tasks: the transmittance
+// term of every segment (4 uniform samples of the second stream), the
+// scattering term at its end, the weight of its shadow walk (for the pass
+// over the tape), and the DRT term of every task.
+__global__ void __launch_bounds__(256) vps_segments_kernel(const __grid_constant__ VolJob J,
+                                                           const __grid_constant__ VpsParams P,
+                                                           const __grid_constant__ Queue Q, float* __restrict__ wn) {
+  const int64_t nrec = min((int64_t)*Q.ckpt_count, Q.ckpt_cap), ntask = P.use_drt ? (int64_t)*P.task_count : 0;
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x, first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int64_t i = first; i < nrec; i += stride) {
+    const float4* r = Q.ckpt + i * kVpsRec;
+    const float4 r0 = __ldcs(r), r1 = __ldcs(r + 1), r2 = __ldcs(r + 2), r3 = __ldcs(r + 3);
+    const uint32_t path = __float_as_uint(r0.x);
+    const float4 lt = __ldg(Q.path_ltot + path);
+    if (lt.w != 0.0f) {  // lost: the path is taken whole by vps_kernel
+      wn[i] = 0.0f;
+      continue;
+    }
+    int pix;
+    const uint32_t sid = vps_sid(J, path, pix);
+    const V3 dL = vps_dL(J, pix);
+    const V3 res{lt.x - r0.y, lt.y - r0.z, lt.z - r0.w};
+    wn[i] = (dL.x * r3.x + dL.y * r3.y) + dL.z * r3.z;
+    const V3 o{r1.x, r1.y, r1.z}, d{r2.x, r2.y, r2.z};
+    const float interval = r1.w;
+    const uint32_t kf = __float_as_uint(r2.w);
+    if ((kf & 1u) == 0u && (!P.use_drt || P.use_drt_mis)) {
+      const V3 x = advance(o, interval, d);
+      const Lookup l = locate(J, x);
+      const AlbedoLookup al = albedo_lookup(J, l, x);
+      const float st = J.scale * density_new(J, l);
+      const V3 a = albedo_at(J, al, 1);
+      const float mis = P.use_drt ? (st * st) / (1.0f + st * st) : 1.0f;
+      const float inv_pdf = 1.0f / st;
+      const V3 k{((mis * dL.x) * (res.x / fmaxf(1e-8f, a.x))) * inv_pdf,
+                 ((mis * dL.y) * (res.y / fmaxf(1e-8f, a.y))) * inv_pdf,
+                 ((mis * dL.z) * (res.z / fmaxf(1e-8f, a.z))) * inv_pdf};
+      scatter_density(J, l, J.scale * ((k.x * a.x + k.y * a.y) + k.z * a.z));
+      if (J.grad_albedo != nullptr) scatter_albedo(J, al, V3{k.x * st, k.y * st, k.z * st});
+    }
+    Pcg32 alt;
+    seed_lane(alt, P.alt_seed, sid);
+    alt.state = pcg_jump(alt.state, alt.inc, (uint32_t)P.draws * (kf >> 1) + (uint32_t)(P.draws - 4));
+    const float w = (dL.x * res.x + dL.y * res.y) + dL.z * res.z;
+    const float coef = -(w * (interval * 0.25f));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float tj = next1d(alt) * interval;
+      scatter_density(J, locate(J, advance(o, tj, d)), J.scale * coef);
+    }
+  }
+  if (!(J.scale * bits_to_float(__ldg(J.maxbits + 1)) > 0.0f)) return;  // empty medium: no DRT
+  for (int64_t i = first; i < ntask; i += stride) {
+    const float4* t = P.task + i * kVpsTask;
+    const float4 t0 = __ldcs(t), t1 = __ldcs(t + 1), t2 = __ldcs(t + 2);
+    int pix;
+    vps_sid(J, __float_as_uint(t0.x), pix);
+    const V3 dL = vps_dL(J, pix), x{t2.x, t2.y, t2.z};
+    const Lookup l = locate(J, x);
+    const AlbedoLookup al = albedo_lookup(J, l, x);
+    const float st = J.scale * density_new(J, l);
+    const V3 a = albedo_at(J, al, 1);
+    const float mis = P.use_drt_mis ? 1.0f / (1.0f + st * st) : 1.0f;
+    const float k0 = mis * t1.w;
+    const V3 k{(k0 * (t1.x * dL.x)) * t0.y, (k0 * (t1.y * dL.y)) * t0.z, (k0 * (t1.z * dL.z)) * t0.w};
+    scatter_density(J, l, J.scale * ((k.x * a.x + k.y * a.y) + k.z * a.z));
+    if (J.grad_albedo != nullptr) scatter_albedo(J, al, V3{k.x * st, k.y * st, k.z * st});
+  }
+}
+
+// Flat pass over the shadow-walk steps on the tape: -(weight of the walk) /
+// sigma_n at each.
+__global__ void __launch_bounds__(256) vps_shadow_kernel(const __grid_constant__ VolJob J,
+                                                         const __grid_constant__ Queue Q,
+                                                         const float* __restrict__ wn) {
+  const int64_t n = min((int64_t)*Q.tape_count, Q.tape_cap);
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    const float4 ev = __ldcs(Q.tape + i);
+    const uint32_t ref = __float_as_uint(ev.w);
+    if (ref == kTapeEmpty) continue;
+    const float w = __ldg(wn + ref);
+    if (w == 0.0f) continue;
+    const float sn = __ldcs(Q.tape_f + i);
+    scatter_density(J, locate(J, V3{ev.x, ev.y, ev.z}), -(J.scale * w) / sn);
+  }
+}
+
+// Workspace of the recorded adjoint over `paths` paths at a time (256-byte
+// aligned sections): counters (hand-out of both tracers, records, tape slots,
+// lost paths, tasks) | order buckets | pixel order | per-path radiance |
+// segment records | their shadow weights | tape (16 + 4 bytes a slot) | tasks
+// | lost list.
+// Room per path: 6 segments and 48 shadow steps.  A path of a medium that
+// fills the view takes about 3 segments and 20 steps at the albedos and
+// depths of the test scenes; what does not fit is traced by vps_kernel.
+constexpr int kVpsRecsPerPath = 6, kVpsSlotsPerPath = 48;
+constexpr int64_t kVpsMaxPaths = int64_t(1) << 22;  // 6 GB of workspace: larger films go in several passes
+constexpr int64_t kVpsMinPaths = int64_t(1) << 16;
+
+struct VpsLayout {
+  uint64_t counters, buckets, order, ltot, rec, wn, tape, task, lost, total;
+};
+
+static VpsLayout vps_layout(int64_t npix, int64_t paths) {
+  VpsLayout L;
+  const uint64_t n = (uint64_t)paths;
+  L.counters = 0;
+  L.buckets = 256;
+  L.order = align256(L.buckets + kRenderOrderBuckets * sizeof(uint32_t));
+  L.ltot = align256(L.order + uint64_t(npix) * sizeof(uint32_t));
+  L.rec = align256(L.ltot + n * 16u);
+  L.wn = align256(L.rec + n * kVpsRecsPerPath * 64u);
+  L.tape = align256(L.wn + n * kVpsRecsPerPath * 4u);
+  L.task = align256(L.tape + uint64_t(tape_capacity(paths, kVpsSlotsPerPath)) * 20u);
+  L.lost = align256(L.task + n * kVpsTask * 16u);
+  L.total = align256(L.lost + n * 4u);
+  return L;
+}
+
+// Paths that a workspace of `bytes` takes at a time (0: too small).
+static int64_t vps_paths_for(int64_t npix, int64_t paths, uint64_t bytes) {
+  int64_t n = paths < kVpsMaxPaths ? paths : kVpsMaxPaths;
+  while (vps_layout(npix, n).total > bytes) {
+    if (n <= kVpsMinPaths) return 0;
+    n = n / 2 > kVpsMinPaths ? n / 2 : kVpsMinPaths;
+  }
+  return n;
+}
+
+using VpsKernel = void (*)(VolJob, VpsParams, Queue);
+static const VpsKernel kVpsKernels[2][4] = {
+    {vps_trace_kernel<kVpsTape, false, false>, vps_trace_kernel<kVpsTape, true, false>,
+     vps_trace_kernel<kVpsTape, false, true>, vps_trace_kernel<kVpsTape, true, true>},
+    {vps_trace_kernel<kVpsDrt, false, false>, vps_trace_kernel<kVpsDrt, true, false>,
+     vps_trace_kernel<kVpsDrt, false, true>, vps_trace_kernel<kVpsDrt, true, true>}};
+
+static int vps_resident(int mode, int variant) {
+  static std::once_flag once;
+  static int blocks[2][4];
+  std::call_once(once, [] {
+    for (int k = 0; k < 8; ++k) {
+      int& b = blocks[k / 4][k % 4];
+      b = 1;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kVpsKernels[k / 4][k % 4], kVpsBlock, 0);
+      if (b < 1) b = 1;
+    }
+  });
+  return blocks[mode][variant];
 }
 
 // sample_tea_32(bits of lane 0's fourth draw, 1)[0] (:108-113).
@@ -452,6 +613,83 @@ static unsigned vps_grid(int64_t paths) {
   return (unsigned)(blocks < 1 ? 1 : blocks);
 }
 
+static int vps_whole(const VolJob& J, const VpsParams& P, unsigned grid, cudaStream_t st) {
+  if (J.env.valid)
+    vps_kernel<true, true><<<grid, 128, 0, st>>>(J, P);
+  else
+    vps_kernel<true, false><<<grid, 128, 0, st>>>(J, P);
+  return launched("volpathsimple adjoint launch");
+}
+
+// The recorded adjoint of all paths, `chunk` at a time.
+static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, char* ws, int64_t npix, int64_t chunk,
+                        cudaStream_t st) {
+  const VpsLayout L = vps_layout(npix, chunk);
+  unsigned long long* qc = reinterpret_cast<unsigned long long*>(ws + L.counters);
+  int rc = RCV_OK;
+  if (o->order != RCV_ORDER_ROW_MAJOR) {
+    // longest chord through the medium first: the path lengths of an earlier
+    // call would order a little better but would tie the scratch to the caller
+    uint32_t* order = reinterpret_cast<uint32_t*>(ws + L.order);
+    rc = order_pixels(J, reinterpret_cast<uint32_t*>(ws + L.buckets), order, nullptr, st);
+    if (rc) return rc;
+    J.pixel_order = order;
+  }
+  P.draws = P.use_drt ? 5 : 4;
+  P.task = reinterpret_cast<float4*>(ws + L.task);
+  P.task_count = qc + 5;
+  Queue Q;
+  std::memset(&Q, 0, sizeof(Q));
+  Q.ckpt = reinterpret_cast<float4*>(ws + L.rec);
+  Q.ckpt_count = qc + 2;
+  Q.ckpt_cap = chunk * kVpsRecsPerPath;
+  Q.tape = reinterpret_cast<float4*>(ws + L.tape);
+  Q.tape_f = reinterpret_cast<float*>(ws + L.tape + uint64_t(tape_capacity(chunk, kVpsSlotsPerPath)) * 16u);
+  Q.tape_count = qc + 3;
+  const int per_path = o->tape_events_per_path;
+  Q.tape_cap = tape_capacity(chunk, per_path >= 1 && per_path < kVpsSlotsPerPath ? per_path : kVpsSlotsPerPath);
+  Q.path_ltot = reinterpret_cast<float4*>(ws + L.ltot);
+  Q.lost_list = reinterpret_cast<uint32_t*>(ws + L.lost);
+  Q.lost_count = qc + 4;
+  // launch options beyond a warp's means are brought into range (the adjoint
+  // of one thread per path ignored them)
+  Q.defer = o->defer > 0 ? (o->defer < 32 ? o->defer : 32) : 8;
+  float* wn = reinterpret_cast<float*>(ws + L.wn);
+  const int variant = (J.sg[0] > 0 ? 1 : 0) + (J.env.valid ? 2 : 0);
+  const int sms = tracer_sm_count();
+  for (int64_t base = 0; base < J.path_count; base += chunk) {
+    const int64_t n = J.path_count - base < chunk ? J.path_count - base : chunk;
+    J.path_begin = -base;  // path p of the pass is path base + p of the film
+    RCV_TRY_CUDA(cudaMemsetAsync(qc, 0, 8 * sizeof(unsigned long long), st), "counters reset");
+    for (int mode = kVpsTape; mode <= (P.use_drt ? kVpsDrt : kVpsTape); ++mode) {
+      Q.counter = qc + mode;
+      Q.total = n;
+      const int64_t cap = int64_t(sms) * vps_resident(mode, variant);
+      // paths per fetch: 64, or fewer so that a small film reaches every warp
+      int64_t batch = n / (cap * kVpsWarps * 2);
+      batch = batch < 1 ? 1 : (batch > 64 ? 64 : batch);
+      Q.batch = (int32_t)batch;
+      int64_t blocks = (n + batch * kVpsWarps - 1) / (batch * kVpsWarps);
+      if (blocks > cap) blocks = cap;
+      kVpsKernels[mode][variant]<<<(unsigned)blocks, kVpsBlock, 0, st>>>(J, P, Q);
+      rc = launched("volpathsimple tracer launch");
+      if (rc) return rc;
+    }
+    vps_segments_kernel<<<(unsigned)sms * 8u, 256, 0, st>>>(J, P, Q, wn);
+    rc = launched("volpathsimple segments launch");
+    if (rc) return rc;
+    vps_shadow_kernel<<<(unsigned)sms * 8u, 256, 0, st>>>(J, Q, wn);
+    rc = launched("volpathsimple shadow launch");
+    if (rc) return rc;
+    VpsParams R = P;
+    R.lost_list = Q.lost_list;
+    R.lost_count = Q.lost_count;
+    rc = vps_whole(J, R, vps_grid(n) < (unsigned)sms ? vps_grid(n) : (unsigned)sms * 4u, st);
+    if (rc) return rc;
+  }
+  return RCV_OK;
+}
+
 }  // namespace rcv
 
 using namespace rcv;
@@ -485,7 +723,23 @@ extern "C" int rcv_render_backward_volpathsimple(const rcv_medium* m, const rcv_
                                                  const rcv_volpath_options* o, const rcv_volpathsimple_flags* f,
                                                  uint32_t seed, int32_t spp, const float* grad_img,
                                                  float* grad_density, float* grad_albedo, void* stream) {
+  return rcv_render_backward_volpathsimple_ws(m, s, o, f, seed, spp, grad_img, grad_density, grad_albedo, nullptr, 0,
+                                              stream);
+}
+
+extern "C" uint64_t rcv_volpathsimple_adjoint_workspace_bytes(int32_t width, int32_t height, int32_t spp) {
+  if (width <= 0 || height <= 0 || spp <= 0) return 0;
+  const int64_t npix = int64_t(width) * height, paths = npix * spp;
+  return vps_layout(npix, paths < kVpsMaxPaths ? paths : kVpsMaxPaths).total;
+}
+
+extern "C" int rcv_render_backward_volpathsimple_ws(const rcv_medium* m, const rcv_sensor* s,
+                                                    const rcv_volpath_options* o, const rcv_volpathsimple_flags* f,
+                                                    uint32_t seed, int32_t spp, const float* grad_img,
+                                                    float* grad_density, float* grad_albedo, void* workspace,
+                                                    uint64_t workspace_bytes, void* stream) {
   RCV_REQUIRE(grad_img != nullptr && grad_density != nullptr, "gradient buffers are NULL");
+  RCV_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255u) == 0, "workspace must be 256-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   VolJob J;
   VpsParams P;
@@ -496,11 +750,13 @@ extern "C" int rcv_render_backward_volpathsimple(const rcv_medium* m, const rcv_
   if (rc) return rc;
   if (!want_albedo) J.grad_albedo = nullptr;
   J.grad_img = grad_img;
-  if (J.env.valid)
-    vps_kernel<true, true><<<vps_grid(J.path_count), 128, 0, st>>>(J, P);
+  const int64_t npix = int64_t(J.width) * J.height;
+  const bool recorded = workspace != nullptr && (!P.use_drt || P.use_drt_subsampling);
+  const int64_t chunk = recorded ? vps_paths_for(npix, J.path_count, workspace_bytes) : 0;
+  if (chunk > 0)
+    rc = vps_recorded(J, P, o, static_cast<char*>(workspace), npix, chunk, st);
   else
-    vps_kernel<true, false><<<vps_grid(J.path_count), 128, 0, st>>>(J, P);
-  rc = launched("volpathsimple adjoint launch");
+    rc = vps_whole(J, P, vps_grid(J.path_count), st);
   if (rc) return rc;
   return launch_fold(m, grad_density, want_albedo ? grad_albedo : nullptr, st);
 }

@@ -60,6 +60,20 @@ class VolpathSimpleIntegrator(PRBVolpathIntegrator):
             self._vps_scratch[device] = buf
         return (buf.data_ptr() + 255) & ~255
 
+    @staticmethod
+    def _adjoint_scratch(device, sensor, spp: int):
+        """Scratch of one adjoint call: torch's allocator keeps it for the next
+        call on the stream, or hands it to others.  On a nearly full GPU a
+        smaller one (more passes; too small for any, one thread per path)."""
+        f = sensor.film()
+        need = int(_lib.load().rcv_volpathsimple_adjoint_workspace_bytes(f.width, f.height, spp)) + 256
+        while need > (1 << 22):
+            try:
+                return torch.empty(need, dtype=torch.uint8, device=device)
+            except torch.cuda.OutOfMemoryError:
+                need //= 4
+        return torch.empty(need, dtype=torch.uint8, device=device)
+
     def render(self, scene, sensor=0, seed: int = 0, spp: int = 0, develop: bool = True, evaluate: bool = True):
         """Primal image of the current parameters
         (VolpathSimpleIntegrator.sample in primal mode, :53-327)."""
@@ -102,13 +116,16 @@ class VolpathSimpleIntegrator(PRBVolpathIntegrator):
         dx, dy, dz = medium.dims
         gd = torch.zeros((dz, dy, dx, 1), dtype=torch.float32, device=medium.device)
         ga = medium.albedo_grad_buffer()
+        ws = self._adjoint_scratch(medium.device, sensor, spp)
+        base = (ws.data_ptr() + 255) & ~255
         with profiling.region("vps_adjoint", medium.device):
             _lib.check(
-                _lib.load().rcv_render_backward_volpathsimple(
+                _lib.load().rcv_render_backward_volpathsimple_ws(
                     C.byref(m), C.byref(s), C.byref(o), C.byref(fl), seed & 0xFFFFFFFF, spp, g.data_ptr(),
-                    gd.data_ptr(), ga.data_ptr() if ga is not None else None, st,
+                    gd.data_ptr(), ga.data_ptr() if ga is not None else None, base,
+                    ws.numel() - (base - ws.data_ptr()), st,
                 ),
-                "rcv_render_backward_volpathsimple",
+                "rcv_render_backward_volpathsimple_ws",
             )
         out = {}
         keys = list(params.keys()) if params is not None else []
