@@ -159,8 +159,9 @@ typedef struct rcv_volpath_options {
    * and jobs (or batches) of 2^28 gradient paths or more always replay.  The
    * batched engine takes the same choice. */
   int32_t adjoint;
-  /* Tape slots per path, 1..16 (0 = 16, the room the adjoint workspace
-   * holds): paths whose events do not fit are replayed whole. */
+  /* Tape slots per path, 1..16 (0 = the room that the adjoint workspace
+   * holds: 16 per path, up to 64 in single-job calls of 4.2 M paths or
+   * fewer): paths whose events do not fit are replayed whole. */
   int32_t tape_events_per_path;
   /* The two-state pass and the adjoint's radiance pass of a step as two
    * launches (1; the batched engine runs them on two streams) instead of one

@@ -390,6 +390,10 @@ struct PlanLayout {
   uint64_t entries, two, adj, prefix, queue, counters, path_out, ltot, ckpt, tape, cam_w, lost, total;
 };
 
+// A plan's scratch grows with its paths alone (the serving budget adds its
+// jobs' shares up): 2 checkpoints and kTapeSlotsPerPath tape slots per path.
+static int64_t batch_ckpt_capacity(int64_t paths) { return kTapeSlotsPerPath / 8 * paths + kCkptMargin; }
+
 static PlanLayout plan_layout(int n, int64_t total_two_paths, int64_t total_adj_paths) {
   PlanLayout L;
   uint64_t off = 0;
@@ -410,7 +414,7 @@ static PlanLayout plan_layout(int n, int64_t total_two_paths, int64_t total_adj_
   L.ltot = off;
   off = align256(off + uint64_t(total_adj_paths) * 16u);
   L.ckpt = off;
-  off = align256(off + uint64_t(ckpt_capacity(total_adj_paths)) * 64u);
+  off = align256(off + uint64_t(batch_ckpt_capacity(total_adj_paths)) * 64u);
   L.tape = off;
   off = align256(off + uint64_t(tape_capacity(total_adj_paths, kTapeSlotsPerPath)) * 20u);
   L.cam_w = off;
@@ -664,7 +668,7 @@ extern "C" int rcv_batch_create(const rcv_batch_job* jobs, int32_t n, const rcv_
   b->path_out = reinterpret_cast<float4*>(w + P.path_out);
   b->adjbuf.ckpt = reinterpret_cast<float4*>(w + P.ckpt);
   b->adjbuf.ckpt_count = b->queue + 3;
-  b->adjbuf.ckpt_cap = ckpt_capacity(adj_total);
+  b->adjbuf.ckpt_cap = batch_ckpt_capacity(adj_total);
   b->adjbuf.path_ltot = reinterpret_cast<float4*>(w + P.ltot);
   // (tape slots are 32-bit indices: batches of 2^28 gradient paths or more replay)
   b->tape = b->opt.adjoint == RCV_ADJOINT_TAPE && adj_total < (int64_t(1) << 28);
@@ -676,7 +680,7 @@ extern "C" int rcv_batch_create(const rcv_batch_job* jobs, int32_t n, const rcv_
     b->adjbuf.tape_cap = tape_capacity(adj_total, per_path);
     b->adjbuf.lost_list = reinterpret_cast<uint32_t*>(w + P.lost);
     b->adjbuf.lost_count = b->queue + 5;
-    b->adjbuf.tape_f = tape_terms(w + P.tape, adj_total);
+    b->adjbuf.tape_f = tape_terms(w + P.tape, tape_capacity(adj_total, kTapeSlotsPerPath));
     b->tape_weights = reinterpret_cast<float4*>(w + P.ckpt + uint64_t(b->adjbuf.ckpt_cap) * 32u);
     b->cam_w = reinterpret_cast<float2*>(w + P.cam_w);
   }

@@ -126,20 +126,39 @@ struct RenderLayout {
   uint64_t counter, buckets, order, cost, path_out, ltot, ckpt, tape, cam_w, lost, total;
 };
 
-// Adjoint scatter checkpoints: 64 bytes each, room for 2 per path plus a
-// margin; paths whose checkpoints do not fit are replayed whole.  The tape
-// adjoint keeps its 32-byte event records in the first half of the same
-// buffer and their 32-byte weights in the second.
-inline int64_t ckpt_capacity(int64_t paths) { return 2 * paths + 65536; }
-
-// Event tape of the adjoint: 16 bytes per event, kTapeSlotsPerPath per path
-// (whole chunks of kTapeChunkSlots, the unit a warp claims), followed by one
-// 4-byte extinction term per slot (volume tape).
+// Event tape of the adjoint: 16 bytes per event (whole chunks of
+// kTapeChunkSlots, the unit a warp claims), followed by one 4-byte extinction
+// term per slot (volume tape).  A launch has 16 slots per path, and one of
+// fewer paths up to 64 from a budget of 2^28 slots (5.4 GB, reached at 4.2 M
+// paths; the total never falls as paths are added).  Where the camera sees
+// little else than the medium, a path makes 30 to 60 events instead of the 8
+// of a film that it covers to a fifth; with 16 slots such launches lost most
+// of their paths to the whole-path replay (five 107 x 83 views at 6 spp:
+// 4.8 ms of replay beside a 1.2-ms tracer launch).
 constexpr int64_t kTapeSlotsPerPath = 16;
+constexpr int64_t kTapeSlotsMost = 64;
+constexpr int64_t kTapeSlotBudget = int64_t(1) << 28;
 constexpr int64_t kTapeChunkSlots = 256;
-inline int64_t tape_capacity(int64_t paths, int per_path) {
-  const int64_t slots = paths * (int64_t)per_path;
+inline int64_t tape_capacity(int64_t paths, int64_t per_path) {
+  const int64_t slots = paths * per_path;
   return (slots + kTapeChunkSlots - 1) / kTapeChunkSlots * kTapeChunkSlots;
+}
+// n per path, up to `most` per path within the budget
+inline int64_t within_budget(int64_t paths, int64_t n, int64_t most, int64_t budget) {
+  const int64_t up = most * paths < budget ? most * paths : budget;
+  return n * paths > up ? n * paths : up;
+}
+inline int64_t tape_room(int64_t paths) {
+  return tape_capacity(within_budget(paths, kTapeSlotsPerPath, kTapeSlotsMost, kTapeSlotBudget), 1);
+}
+
+// Adjoint scatter checkpoints: 64 bytes each, room for one per 8 tape slots (2
+// to 8 per path) plus a margin; paths whose checkpoints do not fit are
+// replayed whole.  The tape adjoint keeps its 32-byte event records in the
+// first half of the same buffer and their 32-byte weights in the second.
+constexpr int64_t kCkptMargin = 65536;
+inline int64_t ckpt_capacity(int64_t paths) {
+  return within_budget(paths, kTapeSlotsPerPath / 8, kTapeSlotsMost / 8, kTapeSlotBudget / 8) + kCkptMargin;
 }
 
 inline uint64_t path_out_bytes(int64_t paths, int mode) {
@@ -157,7 +176,7 @@ inline RenderLayout render_layout(int64_t npix, int64_t paths, int mode) {
   L.ltot = align256(L.path_out + path_out_bytes(paths, mode));
   L.ckpt = align256(L.ltot + (adj ? uint64_t(paths) * 16u : 0u));
   L.tape = align256(L.ckpt + (adj ? uint64_t(ckpt_capacity(paths)) * 64u : 0u));
-  L.cam_w = align256(L.tape + (adj ? uint64_t(tape_capacity(paths, kTapeSlotsPerPath)) * 20u : 0u));
+  L.cam_w = align256(L.tape + (adj ? uint64_t(tape_room(paths)) * 20u : 0u));
   L.lost = align256(L.cam_w + (adj ? uint64_t(paths) * 8u : 0u));
   L.total = align256(L.lost + (adj ? uint64_t(paths) * 4u : 0u));
   return L;

@@ -169,7 +169,11 @@ __global__ void __launch_bounds__(256) tape_scatter_kernel(const __grid_constant
 int launch_tape_gradient(const VolJob& single, const VolJob* jobs, int njobs, const AdjBuffers& A, float4* weights,
                          float2* cam_w, int64_t paths, uint64_t* counters, int sms, cudaStream_t st) {
   const int block = 256;
-  tape_weights_kernel<<<grid_for(A.ckpt_cap > paths ? A.ckpt_cap : paths, block), block, 0, st>>>(
+  // grid-stride: the records' number is known on the device only, and their
+  // room is many times it
+  const unsigned need = grid_for(A.ckpt_cap > paths ? A.ckpt_cap : paths, block);
+  const unsigned most = (unsigned)(sms > 0 ? sms : 1) * 16u;
+  tape_weights_kernel<<<need < most ? need : most, block, 0, st>>>(
       single, jobs, njobs, A.ckpt, A.ckpt_count, A.ckpt_cap, weights, A.path_ltot, cam_w, paths);
   int rc = launched("tape_weights launch");
   if (rc) return rc;

@@ -651,19 +651,18 @@ static int adjoint_buffers(const VolJob& J, const rcv_volpath_options* o, char* 
   A.ckpt_cap = ckpt_capacity(J.path_count);
   A.path_ltot = reinterpret_cast<float4*>(ws + L.ltot);
   const int adjoint = o == nullptr ? RCV_ADJOINT_TAPE : o->adjoint;
-  const int per_path = (o == nullptr || o->tape_events_per_path == 0) ? int(kTapeSlotsPerPath)
-                                                                    : o->tape_events_per_path;
+  const int per_path = o == nullptr ? 0 : o->tape_events_per_path;
   RCV_REQUIRE(adjoint == RCV_ADJOINT_TAPE || adjoint == RCV_ADJOINT_REPLAY, "unknown adjoint %d", adjoint);
-  RCV_REQUIRE(per_path >= 1 && per_path <= kTapeSlotsPerPath, "tape_events_per_path must be in [0, %d]",
-              int(kTapeSlotsPerPath));
+  RCV_REQUIRE(per_path >= 0 && per_path <= kTapeSlotsPerPath,
+              "tape_events_per_path must be in [0, %d]", int(kTapeSlotsPerPath));
   const bool tape = adjoint == RCV_ADJOINT_TAPE && stage != kAdjForward && J.path_count < (int64_t(1) << 28);
   if (tape) {
     A.tape = reinterpret_cast<float4*>(ws + L.tape);
     A.tape_count = qc + 2;
-    A.tape_cap = tape_capacity(J.path_count, per_path);
+    A.tape_cap = per_path > 0 ? tape_capacity(J.path_count, per_path) : tape_room(J.path_count);
     A.lost_list = reinterpret_cast<uint32_t*>(ws + L.lost);
     A.lost_count = qc + 3;
-    A.tape_f = tape_terms(ws + L.tape, J.path_count);
+    A.tape_f = tape_terms(ws + L.tape, tape_room(J.path_count));
   }
   *tape_out = tape;
   return RCV_OK;

@@ -569,11 +569,9 @@ void warm_pair_config();
 // Queries the occupancy and SM count the launchers cache, so that later
 // launches (e.g. under stream capture) make no device queries.
 void warm_launch_config();
-// The extinction terms follow the tape's slots in the tape region (16 B +
-// 4 B per slot).
-inline float* tape_terms(char* region, int64_t paths) {
-  return reinterpret_cast<float*>(region + tape_capacity(paths, kTapeSlotsPerPath) * 16);
-}
+// The extinction terms follow the `room` slots of the tape in its region
+// (16 B + 4 B per slot).
+inline float* tape_terms(char* region, int64_t room) { return reinterpret_cast<float*>(region + room * 16); }
 
 // Gradient from a kTape radiance pass (rcv_tape.cu) of one job (jobs ==
 // NULL) or of a device job table: the per-record and per-path weights

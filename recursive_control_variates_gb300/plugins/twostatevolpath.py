@@ -25,6 +25,14 @@ _SRGB_TO_XYZ = torch.tensor(
 )
 
 
+def _new_scratch(nbytes: int, film, device) -> torch.Tensor:
+    """Tracer scratch, its head (counters, pixel order, per-pixel cost) zeroed:
+    the cost that it carries from call to call starts at zero."""
+    buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    buf[: 4096 + 8 * film.width * film.height].zero_()
+    return buf
+
+
 class _VolumeIntegratorBase:
     two_state = False
 
@@ -107,8 +115,7 @@ class _VolumeIntegratorBase:
         need = int(_lib.load().rcv_render_workspace_bytes(f.width, f.height, spp, mode)) + 256
         buf = self._scratch.get(device)
         if buf is None or buf.numel() < need:
-            # zeroed once: the per-pixel cost it carries starts at zero
-            buf = torch.zeros(need, dtype=torch.uint8, device=device)
+            buf = _new_scratch(need, f, device)
             self._scratch[device] = buf
         return (buf.data_ptr() + 255) & ~255
 
@@ -122,7 +129,7 @@ class _VolumeIntegratorBase:
         buf = self._adj_scratch.get(device)
         if buf is None or buf.numel() < need:
             self._drain_ticket(device)  # the old buffer may still be in use
-            buf = torch.zeros(need, dtype=torch.uint8, device=device)
+            buf = _new_scratch(need, f, device)
             self._adj_scratch[device] = buf
         return (buf.data_ptr() + 255) & ~255
 
