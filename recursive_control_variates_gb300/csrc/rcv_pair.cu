@@ -21,7 +21,7 @@
 
 namespace rcv {
 
-template <bool kSG, bool kEnv>
+template <bool kSG, bool kEnv, bool kTable>
 __global__ void __launch_bounds__(kTraceBlock, 5)
     trace_pair_kernel(const __grid_constant__ VolJob JA, const __grid_constant__ Queue QA,
                       const __grid_constant__ VolJob JB, const __grid_constant__ Queue QB) {
@@ -39,20 +39,24 @@ __global__ void __launch_bounds__(kTraceBlock, 5)
   // each tracer returns once its queue is empty and the warp's paths ended
   // (written out rather than as a loop over the two: the loop form keeps
   // state of both bodies live and spills ~200 B a thread)
-  if (primal_first) trace_persistent<kTwoState, kSG, false, kEnv>(JA, QA, cnt);
-  trace_persistent<kTape, kSG, false, kEnv>(JB, QB, cnt);
-  if (!primal_first) trace_persistent<kTwoState, kSG, false, kEnv>(JA, QA, cnt);
+  if (primal_first) trace_persistent<kTwoState, kSG, false, kEnv, kTable>(JA, QA, cnt);
+  trace_persistent<kTape, kSG, false, kEnv, kTable>(JB, QB, cnt);
+  if (!primal_first) trace_persistent<kTwoState, kSG, false, kEnv, kTable>(JA, QA, cnt);
 }
 
 using PairKernel = void (*)(VolJob, Queue, VolJob, Queue);
-static const PairKernel kPairKernels[4] = {trace_pair_kernel<false, false>, trace_pair_kernel<true, false>,
-                                           trace_pair_kernel<false, true>, trace_pair_kernel<true, true>};
+// by supergrid + 2 * environment map (single jobs), then job tables by supergrid
+constexpr int kPairVariants = 6;
+static const PairKernel kPairKernels[kPairVariants] = {
+    trace_pair_kernel<false, false, false>, trace_pair_kernel<true, false, false>,
+    trace_pair_kernel<false, true, false>,  trace_pair_kernel<true, true, false>,
+    trace_pair_kernel<false, false, true>,  trace_pair_kernel<true, false, true>};
 
 static int pair_blocks_per_sm(int variant) {
   static std::once_flag once;
-  static int blocks[4];
+  static int blocks[kPairVariants];
   std::call_once(once, [] {
-    for (int v = 0; v < 4; ++v) {
+    for (int v = 0; v < kPairVariants; ++v) {
       blocks[v] = 1;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[v], kPairKernels[v], kTraceBlock, 0);
       if (blocks[v] < 1) blocks[v] = 1;
@@ -75,7 +79,7 @@ int launch_pair(const VolJob& JA, const Queue& QA, const VolJob& JB, const Queue
   // an environment map belongs to a single job (job tables take the constant environment)
   const bool env = single && JA.env.valid != 0;
   RCV_REQUIRE(!single || (JB.env.valid != 0) == env, "the paired jobs must share their environment");
-  const int variant = (sg ? 1 : 0) + (env ? 2 : 0);
+  const int variant = (sg ? 1 : 0) + (single ? (env ? 2 : 0) : 4);
   int per_sm = pair_blocks_per_sm(variant);
   if (o != nullptr && o->blocks_per_sm > 0 && o->blocks_per_sm < per_sm) per_sm = o->blocks_per_sm;
   const int64_t warps_needed = (QA.total + QA.batch - 1) / QA.batch + (QB.total + QB.batch - 1) / QB.batch;

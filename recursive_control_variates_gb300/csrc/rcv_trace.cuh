@@ -72,8 +72,7 @@ __device__ __forceinline__ void write_checkpoint(float4* rec, uint32_t path, int
 }
 
 // Job of a global path index: binary search in the launch's job table.
-__device__ __forceinline__ const VolJob& job_of(const VolJob& single, const Queue& Q, int64_t path) {
-  if (Q.jobs == nullptr) return single;
+__device__ __forceinline__ const VolJob& job_of(const Queue& Q, int64_t path) {
   int lo = 0, hi = Q.njobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -119,8 +118,8 @@ constexpr int kTraceBlock = 32 * kTraceWarps;
 // own no walking path).  kTape: every step taken is a gradient event, which
 // the lane that evaluated it appends to the tape with the owner's reference
 // `ref`; `lost` is set on an owner whose events did not fit.
-template <int kMode>
-__device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJob* Jp, Pcg32& rng, float mu,
+template <int kMode, bool kTable>
+__device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJob& single, const VolJob* Jp, Pcg32& rng, float mu,
                                          float inv_mu, float half_inv_mu, V3& org, const V3& dir, float& tmax,
                                          V3& c1, V3& c2, float* s_t, float* s_w1, float* s_w2, const Queue& Q,
                                          TapeCursor& tc, uint32_t ref, bool& lost) {
@@ -139,7 +138,7 @@ __device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJo
   const int owner = mm != 0u ? __ffs(mm) - 1 : (int)lane;
 
   const bool g_main = __shfl_sync(kFull, (int)main_walk, owner) != 0;
-  const VolJob* J = (const VolJob*)__shfl_sync(kFull, (unsigned long long)Jp, owner);
+  const VolJob& J = kTable ? *(const VolJob*)__shfl_sync(kFull, (unsigned long long)Jp, owner) : single;
   Pcg32 r;
   r.state = __shfl_sync(kFull, (unsigned long long)rng.state, owner);
   r.inc = __shfl_sync(kFull, (unsigned long long)rng.inc, owner);
@@ -170,14 +169,14 @@ __device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJo
   const V3 x{fmaf(t, dv.x, px), fmaf(t, dv.y, py), fmaf(t, dv.z, pz)};
   float st_o = 0.0f, st_n = 0.0f;
   if (valid) {
-    const Lookup lk = locate(*J, x);
+    const Lookup lk = locate(J, x);
     float rho_o = 0.0f, rho_n;
     if (kMode == kTwoState)
-      density2(*J, lk, rho_o, rho_n);
+      density2(J, lk, rho_o, rho_n);
     else
-      rho_n = density_new(*J, lk);
-    st_o = J->scale * rho_o;
-    st_n = J->scale * rho_n;
+      rho_n = density_new(J, lk);
+    st_o = J.scale * rho_o;
+    st_n = J.scale * rho_n;
   }
   bool term;
   float w1 = 0.0f, w2 = 0.0f;  // main: null-collision weights (two-state); shadow: transmittance factors
@@ -283,8 +282,12 @@ __device__ __forceinline__ V3 env_radiance_dir(const VolJob& J, const V3& d, flo
 // no registers).
 // kEnv: the launch's job has an environment map (else the constant white
 // environment; the two are separate kernels so that the constant one carries
-// none of the map's code).
-template <int kMode, bool kSG, bool kCount, bool kEnv>
+// none of the map's code).  kTable: the paths belong to the jobs of Q.jobs.
+// Without a table every field of the job is an operand in the kernel's
+// parameter bank; behind a pointer that may lead to a table entry, the walk
+// would load its grid size, scale, cell address and depth limits again in
+// every step (@@SINGLE@@).
+template <int kMode, bool kSG, bool kCount, bool kEnv, bool kTable>
 __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& cnt) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -419,8 +422,8 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       } else if (kRep && Q.lost_list != nullptr) {
         path = (int64_t)Q.lost_list[path];  // a path the tape could not hold
       }
-      Jp = &job_of(single, Q, path);
-      const VolJob& J = *Jp;
+      if (kTable) Jp = &job_of(Q, path);
+      const VolJob& J = kTable ? *Jp : single;
       const float mu_old = J.scale * bits_to_float(__ldg(J.maxbits + 0));
       const float mu_new = J.scale * bits_to_float(__ldg(J.maxbits + 1));
       mu = (kMode == kTwoState) ? fmaxf(mu_old, mu_new) : mu_new;
@@ -501,13 +504,13 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     }
 
     if (kMode == kReplay && run_start && iter0 == n_iter) {
-      const V3 g = pixel_dL(*Jp, pix);  // the task started in this iteration
+      const V3 g = pixel_dL(kTable ? *Jp : single, pix);  // the task started in this iteration
       s_main = (g.x * Lrem.x + g.y * Lrem.y) + g.z * Lrem.z;
     }
 
     // ------------------------------------------------- real scattering event
     if (run_scat && phase == kScatter) {
-      const VolJob& J = *Jp;
+      const VolJob& J = kTable ? *Jp : single;
       if (kRep && task == kTaskSegment) {
         finished = true;  // the event has its own checkpoint task
       } else if (kRep && task == kTaskCheckpoint && !own_event) {
@@ -636,6 +639,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
 
     // ------------------------- cooperative walk of the last paths (see above)
     if (kCoop && queue_empty) {
+      const VolJob& J = kTable ? *Jp : single;
       bool elig = false;
       if (!finished) {
         if (phase == kNee) {
@@ -643,9 +647,9 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
         } else if (phase == kMain) {
           bool alive = bn.x != 0.0f || bn.y != 0.0f || bn.z != 0.0f;
           if (kMode == kTwoState) alive = alive || (bo.x != 0.0f || bo.y != 0.0f || bo.z != 0.0f);
-          elig = alive && depth <= Jp->rr_depth;
+          elig = alive && depth <= J.rr_depth;
         }
-        if (kSG && elig && Jp->sg[0] > 0) elig = false;
+        if (kSG && elig && J.sg[0] > 0) elig = false;
       }
       const unsigned m_coop = __ballot_sync(0xffffffffu, elig);
       const int n_coop = __popc(m_coop);
@@ -657,7 +661,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
         V3 c1 = mw ? bn : V3{trn, 0.0f, 0.0f};
         V3 c2 = mw ? bo : V3{tro, 0.0f, 0.0f};
         float* s = s_coop + (threadIdx.x >> 5) * 96;
-        const int f = coop_walk<kMode>(m_coop, mw, Jp, rng, mu, inv_mu, 0.5f * inv_mu, org, dir, tmax, c1, c2, s,
+        const int f = coop_walk<kMode, kTable>(m_coop, mw, single, Jp, rng, mu, inv_mu, 0.5f * inv_mu, org, dir, tmax, c1, c2, s,
                                        s + 32, s + 64, Q, tc, tref, ck_lost);
         if (f > 0) {
           if (mw) {
@@ -680,7 +684,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
 
     // --------------------------------------------------- free-flight step
     if (phase == kMain || phase == kNee || phase == kNeeAdj) {
-      const VolJob& J = *Jp;
+      const VolJob& J = kTable ? *Jp : single;
       bool alive = true;
       V3 org, dir;
       float tmax;
@@ -863,7 +867,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
               // whole-path replay: walk the shadow ray again (saved stream) to
               // back-propagate through its transmittance
               if (kMode == kReplay) {
-                const V3 g = pixel_dL(*Jp, pix);
+                const V3 g = pixel_dL(J, pix);
                 s_nee = (g.x * cn.x + g.y * cn.y) + g.z * cn.z;
                 s_main = (g.x * Lrem.x + g.y * Lrem.y) + g.z * Lrem.z;
               } else {
@@ -913,8 +917,9 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
 
     // -------------------------------------------------------------- path end
     if (finished) {
+      const VolJob& J = kTable ? *Jp : single;
       if (kMode == kTwoState || kMode == kSingle) {
-        float4* o = Q.path_out + (Jp->path_begin + sid) * (kMode == kTwoState ? 2 : 1);
+        float4* o = Q.path_out + (J.path_begin + sid) * (kMode == kTwoState ? 2 : 1);
         __stcs(o, make_float4(Ln.x, Ln.y, Ln.z, 0.0f));
         if (kMode == kTwoState) __stcs(o + 1, make_float4(Lo.x, Lo.y, Lo.z, 0.0f));
       }
@@ -923,14 +928,14 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       if (kMode == kForward && (dL.x != 0.0f || dL.y != 0.0f || dL.z != 0.0f)) {
         // the task's share of its pixel's derivative (the pixel value is the
         // mean of its samples)
-        const float fs = (float)Jp->spp;
-        float* o = Jp->out_img + (int64_t)pix * 3;
+        const float fs = (float)J.spp;
+        float* o = J.out_img + (int64_t)pix * 3;
         atomicAdd(o + 0, dL.x / fs);
         atomicAdd(o + 1, dL.y / fs);
         atomicAdd(o + 2, dL.z / fs);
       }
       if (kCount && !kRep) ++cnt.paths;
-      if (Jp->pixel_cost != nullptr) red_add_u32(Jp->pixel_cost + pix, n_iter - iter0);
+      if (J.pixel_cost != nullptr) red_add_u32(J.pixel_cost + pix, n_iter - iter0);
       phase = kIdle;
     }
   }

@@ -1,0 +1,40 @@
+// The tracer kernel and its function-pointer tables, instantiated for single
+// jobs in rcv_volume.cu and for job tables in rcv_trace_table.cu (two files so
+// that they compile side by side).
+#pragma once
+#include "rcv_trace.cuh"
+
+namespace rcv {
+
+__device__ __forceinline__ void add_counts(unsigned long long* counters, const Counts& c) {
+  if (counters == nullptr) return;
+  const unsigned p = __reduce_add_sync(0xffffffffu, c.paths);
+  const unsigned l = __reduce_add_sync(0xffffffffu, c.lookups);
+  const unsigned n = __reduce_add_sync(0xffffffffu, c.nee_lookups);
+  const unsigned s = __reduce_add_sync(0xffffffffu, c.scatters);
+  const unsigned ge = __reduce_add_sync(0xffffffffu, c.grad_events);
+  const unsigned ae = __reduce_add_sync(0xffffffffu, c.albedo_events);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(counters + RCV_COUNTER_PATHS, (unsigned long long)p);
+    atomicAdd(counters + RCV_COUNTER_LOOKUPS, (unsigned long long)l);
+    atomicAdd(counters + RCV_COUNTER_NEE_LOOKUPS, (unsigned long long)n);
+    atomicAdd(counters + RCV_COUNTER_SCATTERS, (unsigned long long)s);
+    if (ge) atomicAdd(counters + RCV_COUNTER_GRAD_EVENTS, (unsigned long long)ge);
+    if (ae) atomicAdd(counters + RCV_COUNTER_ALBEDO_EVENTS, (unsigned long long)ae);
+  }
+}
+
+template <int kMode, bool kSG, bool kCount, bool kEnv, bool kTable>
+__global__ void __launch_bounds__(kTraceBlock, 5) trace_kernel(const __grid_constant__ VolJob J,
+                                                            const __grid_constant__ Queue Q) {
+  Counts cnt{0, 0, 0, 0, 0, 0};
+  trace_persistent<kMode, kSG, kCount, kEnv, kTable>(J, Q, cnt);
+  if (kCount) add_counts(Q.counters, cnt);
+}
+
+using TraceKernel = void (*)(VolJob, Queue);
+// Job-table tracers by supergrid + 2 * counting, then by mode (null: a mode
+// that the batched engine does not run).
+extern const TraceKernel kJobTableTracers[4][kTraceModes];
+
+}  // namespace rcv

@@ -10,7 +10,7 @@
 
 #include "rcv_common.h"
 #include "rcv_pack.cuh"
-#include "rcv_trace.cuh"
+#include "rcv_trace_kernels.cuh"
 
 namespace rcv {
 
@@ -35,51 +35,25 @@ __global__ void pack_medium_kernel(int dx, int dy, int dz, const float* __restri
 }
 
 // ----------------------------------------------------------------- tracing
-__device__ __forceinline__ void add_counts(unsigned long long* counters, const Counts& c) {
-  if (counters == nullptr) return;
-  const unsigned p = __reduce_add_sync(0xffffffffu, c.paths);
-  const unsigned l = __reduce_add_sync(0xffffffffu, c.lookups);
-  const unsigned n = __reduce_add_sync(0xffffffffu, c.nee_lookups);
-  const unsigned s = __reduce_add_sync(0xffffffffu, c.scatters);
-  const unsigned ge = __reduce_add_sync(0xffffffffu, c.grad_events);
-  const unsigned ae = __reduce_add_sync(0xffffffffu, c.albedo_events);
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(counters + RCV_COUNTER_PATHS, (unsigned long long)p);
-    atomicAdd(counters + RCV_COUNTER_LOOKUPS, (unsigned long long)l);
-    atomicAdd(counters + RCV_COUNTER_NEE_LOOKUPS, (unsigned long long)n);
-    atomicAdd(counters + RCV_COUNTER_SCATTERS, (unsigned long long)s);
-    if (ge) atomicAdd(counters + RCV_COUNTER_GRAD_EVENTS, (unsigned long long)ge);
-    if (ae) atomicAdd(counters + RCV_COUNTER_ALBEDO_EVENTS, (unsigned long long)ae);
-  }
-}
-
-template <int kMode, bool kSG, bool kCount, bool kEnv>
-__global__ void __launch_bounds__(kTraceBlock, 5) trace_kernel(const __grid_constant__ VolJob J,
-                                                            const __grid_constant__ Queue Q) {
-  Counts cnt{0, 0, 0, 0, 0, 0};
-  trace_persistent<kMode, kSG, kCount, kEnv>(J, Q, cnt);
-  if (kCount) add_counts(Q.counters, cnt);
-}
-
 // Tracer variants by index mode + kTraceModes * (supergrid + 2 * counting +
-// 4 * environment map).
-using TraceKernel = void (*)(VolJob, Queue);
+// 4 * environment map), then those of job tables (rcv_trace_table.cu).
 template <bool kSG, bool kCount, bool kEnv>
 struct TraceVariants {
   static constexpr TraceKernel k[kTraceModes] = {
-      trace_kernel<kTwoState, kSG, kCount, kEnv>, trace_kernel<kSingle, kSG, kCount, kEnv>,
-      trace_kernel<kAdjoint, kSG, kCount, kEnv>, trace_kernel<kReplay, kSG, kCount, kEnv>,
-      trace_kernel<kForward, kSG, kCount, kEnv>, trace_kernel<kTape, kSG, kCount, kEnv>};
+      trace_kernel<kTwoState, kSG, kCount, kEnv, false>, trace_kernel<kSingle, kSG, kCount, kEnv, false>,
+      trace_kernel<kAdjoint, kSG, kCount, kEnv, false>,  trace_kernel<kReplay, kSG, kCount, kEnv, false>,
+      trace_kernel<kForward, kSG, kCount, kEnv, false>,  trace_kernel<kTape, kSG, kCount, kEnv, false>};
 };
-static const TraceKernel* const kTraceTables[8] = {
+static const TraceKernel* const kTraceTables[12] = {
     TraceVariants<false, false, false>::k, TraceVariants<true, false, false>::k,
     TraceVariants<false, true, false>::k,  TraceVariants<true, true, false>::k,
     TraceVariants<false, false, true>::k,  TraceVariants<true, false, true>::k,
-    TraceVariants<false, true, true>::k,   TraceVariants<true, true, true>::k};
-constexpr int kTraceVariants = 8 * kTraceModes;
+    TraceVariants<false, true, true>::k,   TraceVariants<true, true, true>::k,
+    kJobTableTracers[0], kJobTableTracers[1], kJobTableTracers[2], kJobTableTracers[3]};
+constexpr int kTraceVariants = 12 * kTraceModes;
 
-static int trace_variant(int mode, bool sg, bool count, bool env) {
-  return mode + kTraceModes * ((sg ? 1 : 0) + (count ? 2 : 0) + (env ? 4 : 0));
+static int trace_variant(int mode, bool sg, bool count, bool env, bool table) {
+  return mode + kTraceModes * ((sg ? 1 : 0) + (count ? 2 : 0) + (table ? 8 : (env ? 4 : 0)));
 }
 static TraceKernel trace_kernel_of(int variant) { return kTraceTables[variant / kTraceModes][variant % kTraceModes]; }
 
@@ -330,6 +304,7 @@ static int resident_blocks(int variant) {
   std::call_once(once, [] {
     for (int v = 0; v < kTraceVariants; ++v) {
       blocks[v] = 1;
+      if (trace_kernel_of(v) == nullptr) continue;  // a mode that job tables do not run
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[v], trace_kernel_of(v), kTraceBlock, 0);
       if (blocks[v] < 1) blocks[v] = 1;
     }
@@ -430,7 +405,8 @@ int launch_persistent(int mode, const VolJob& J, const VolJob* jobs, int njobs, 
   if (rc) return rc;
   const bool sg = supergrid || (jobs == nullptr && J.sg[0] > 0);
   // an environment map belongs to a single job (batched tables take the constant environment)
-  const int variant = trace_variant(mode, sg, counters != nullptr, jobs == nullptr && J.env.valid != 0);
+  const int variant = trace_variant(mode, sg, counters != nullptr, jobs == nullptr && J.env.valid != 0, jobs != nullptr);
+  RCV_REQUIRE(trace_kernel_of(variant) != nullptr, "tracer mode %d does not take a job table", mode);
   int per_sm = resident_blocks(variant);
   if (o != nullptr && o->blocks_per_sm > 0 && o->blocks_per_sm < per_sm) per_sm = o->blocks_per_sm;
   // replay: the checkpoint tasks come on top of one camera task per path
