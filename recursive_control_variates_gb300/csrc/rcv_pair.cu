@@ -21,8 +21,16 @@
 
 namespace rcv {
 
-template <bool kSG, bool kEnv, bool kTable>
-__global__ void __launch_bounds__(kTraceBlock, 5)
+// kBlocks: resident blocks per SM that the registers are bounded for, 6 (80
+// registers) or 7 (72, a few spilled).  The seventh pays where a launch is
+// long against its longest paths, which it slows: job tables (24 mixed jobs
+// 19.1 -> 18.5 ms a step) and films of kManyPaths paths or more (33.6 M paths
+// on 256^3: 13.6 -> 13.3 ms; 8.4 M on 64^3: 2.71 -> 2.76 ms; 0.5 M seen by
+// five cameras: 1.66 -> 1.78 ms).
+constexpr int64_t kManyPaths = int64_t(1) << 24;
+
+template <bool kSG, bool kEnv, bool kTable, int kBlocks>
+__global__ void __launch_bounds__(kTraceBlock, kBlocks)
     trace_pair_kernel(const __grid_constant__ VolJob JA, const __grid_constant__ Queue QA,
                       const __grid_constant__ VolJob JB, const __grid_constant__ Queue QB) {
   Counts cnt{0, 0, 0, 0, 0, 0};
@@ -45,12 +53,14 @@ __global__ void __launch_bounds__(kTraceBlock, 5)
 }
 
 using PairKernel = void (*)(VolJob, Queue, VolJob, Queue);
-// by supergrid + 2 * environment map (single jobs), then job tables by supergrid
-constexpr int kPairVariants = 6;
+// by supergrid + 2 * environment map (single jobs), then job tables by
+// supergrid, then single jobs of many paths by supergrid
+constexpr int kPairVariants = 8;
 static const PairKernel kPairKernels[kPairVariants] = {
-    trace_pair_kernel<false, false, false>, trace_pair_kernel<true, false, false>,
-    trace_pair_kernel<false, true, false>,  trace_pair_kernel<true, true, false>,
-    trace_pair_kernel<false, false, true>,  trace_pair_kernel<true, false, true>};
+    trace_pair_kernel<false, false, false, 6>, trace_pair_kernel<true, false, false, 6>,
+    trace_pair_kernel<false, true, false, 6>,  trace_pair_kernel<true, true, false, 6>,
+    trace_pair_kernel<false, false, true, 7>,  trace_pair_kernel<true, false, true, 7>,
+    trace_pair_kernel<false, false, false, 7>, trace_pair_kernel<true, false, false, 7>};
 
 static int pair_blocks_per_sm(int variant) {
   static std::once_flag once;
@@ -79,7 +89,8 @@ int launch_pair(const VolJob& JA, const Queue& QA, const VolJob& JB, const Queue
   // an environment map belongs to a single job (job tables take the constant environment)
   const bool env = single && JA.env.valid != 0;
   RCV_REQUIRE(!single || (JB.env.valid != 0) == env, "the paired jobs must share their environment");
-  const int variant = (sg ? 1 : 0) + (single ? (env ? 2 : 0) : 4);
+  const bool many = single && !env && QA.total + QB.total >= kManyPaths;
+  const int variant = (sg ? 1 : 0) + (single ? (many ? 6 : (env ? 2 : 0)) : 4);
   int per_sm = pair_blocks_per_sm(variant);
   if (o != nullptr && o->blocks_per_sm > 0 && o->blocks_per_sm < per_sm) per_sm = o->blocks_per_sm;
   const int64_t warps_needed = (QA.total + QA.batch - 1) / QA.batch + (QB.total + QB.batch - 1) / QB.batch;

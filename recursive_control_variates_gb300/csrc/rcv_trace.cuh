@@ -301,25 +301,34 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
   constexpr bool kRad = kMode == kAdjoint || kMode == kTape;
   constexpr bool kCoop = kMode == kTwoState || kMode == kSingle || kRad;
   __shared__ float s_coop[kCoop ? kTraceWarps * 96 : 1];  // cooperative walk: distances, weights
-  // environment map: each lane's NEE weight e = Le / pdf * phase * MIS of its
-  // pending shadow ray, kept here from the scattering event to the end of the
-  // walk instead of in registers
-  __shared__ float s_env[kEnv ? kTraceWarps * 32 * 3 : 1];
-  float* env_e = s_env + (kEnv ? threadIdx.x * 3 : 0);
-  // replay: camera tasks [0, paths) (after a tape pass: the paths on the lost
-  // list), then the checkpoints that were written
-  const int64_t total = !kRep ? Q.total
-                              : (Q.lost_list != nullptr ? (int64_t)*Q.lost_count
-                                                        : Q.total + min((int64_t)*Q.ckpt_count, Q.ckpt_cap));
-
-  int64_t batch_next = 0, batch_end = 0;
+  // Cold state of each lane, [word][thread] (no bank conflicts): what a walk
+  // does not touch from one of its ends to the next waits here instead of in
+  // registers.  A lane walks one ray at a time, so the registers hold one
+  // position, direction and distance; during a shadow walk the vertex and the
+  // next segment are cold.
+  enum { cP = 0, cWo = 3, cT = 6, cLn = 7, cLo = 10, cSid = 13, cPix, cPath, cIter0, cScn, cSco, cBn, cBo, cPathHi, cCk, cEnv = cCk + 2,
+         cWords = cEnv + 3 };
+  constexpr int kColdWords = kEnv ? int(cWords) : (kMode == kAdjoint ? int(cEnv) : int(cCk));
+  __shared__ float s_cold[kColdWords * kTraceBlock];
+  float* const cold = s_cold + threadIdx.x;
+  const auto F = [cold](int i) -> float& { return cold[i * kTraceBlock]; };
+  const auto U = [cold](int i) -> uint32_t& { return reinterpret_cast<uint32_t*>(cold)[i * kTraceBlock]; };
+  const auto get3 = [cold](int i) {
+    return V3{cold[i * kTraceBlock], cold[(i + 1) * kTraceBlock], cold[(i + 2) * kTraceBlock]};
+  };
+  const auto put3 = [cold](int i, const V3& v) {
+    cold[i * kTraceBlock] = v.x;
+    cold[(i + 1) * kTraceBlock] = v.y;
+    cold[(i + 2) * kTraceBlock] = v.z;
+  };
+  // next path of the warp's claimed batch (its paths left are in `left`)
+  __shared__ unsigned long long s_next[kTraceWarps];
+  unsigned long long* const next = s_next + (threadIdx.x >> 5);
+  unsigned left = 0u;
   bool queue_empty = false;
-  int64_t path = 0;
   const VolJob* Jp = &single;
   int phase = kIdle;
   float mu = 0.0f, inv_mu = 0.0f;  // half of inv_mu is recomputed where needed (one register less)
-  int pix = 0;
-  uint32_t sid = 0;  // sample index within the job: pixel * spp + sample
   V3 dL{0.0f, 0.0f, 0.0f};  // kForward: the task's image derivative
   // kReplay: dL . L_rem with dL = dLoss/dL of the pixel; it changes only with
   // L_rem, and dL itself is recomputed from the image gradient at the events
@@ -330,24 +339,20 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
   // whole-path replay: state of the stream of the second shadow walk (its
   // increment is rng.inc)
   uint64_t nee_state = 0;
-  // main path state
-  V3 p, d;
-  float t_rem = 0.0f;
-  V3 bo{1, 1, 1}, bn{1, 1, 1}, Lo{0, 0, 0}, Ln{0, 0, 0};
+  // the walk: position, direction and distance left of the main path or of
+  // its shadow ray; throughputs
+  V3 x, dir;
+  float rem = 0.0f;
+  V3 bo{1, 1, 1}, bn{1, 1, 1};
   int depth = 0;
-  float sc_n = 0.0f, sc_o = 0.0f;  // sigma_t of both states at a pending scattering event
-  // NEE state
-  V3 q, w;
-  float tr_rem = 0.0f, tro = 1.0f, trn = 1.0f;
-  V3 wo_next;
-  // adjoint radiance pass: random-number state at the pending scattering event
-  uint64_t ck_state = 0;
+  // transmittances of the shadow ray (the throughputs' .x is cold meanwhile)
+  float& trn = bn.x;
+  float& tro = bo.x;
   bool ck_lost = false;  // a checkpoint (kTape: an event or event record) of this path did not fit
   // kTape: reference of the path's next events (kind << 30 | path or event
   // record), and the warp's tape chunk
   uint32_t tref = 0;
   TapeCursor tc{0u, 0u};
-  // replay
   // replay: radiance the path gathers after its current point,
   // L_rem = L - (radiance gathered so far), kept instead of L and the sum so far
   V3 Lrem{0, 0, 0}, cn_task{0, 0, 0};
@@ -355,33 +360,44 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
   float s_nee = 0.0f;
   int task = kTaskSegment;
   bool own_event = false;  // checkpoint task: its scattering event is still to be processed
-  // loop iterations: a path's length is n_iter - iter0 when it ends
-  uint32_t n_iter = 0, iter0 = 0;
+  // loop iterations: a path's length is n_iter - its cold start when it ends
+  uint32_t n_iter = 0;
 
   while (true) {
     ++n_iter;
     // ------------------------------------------- hand new paths to idle lanes
     unsigned need = __ballot_sync(0xffffffffu, phase == kIdle);
     while (need != 0u && !queue_empty) {
-      if (batch_next == batch_end) {
-        unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(Q.counter, (unsigned long long)Q.batch);
-        b = __shfl_sync(0xffffffffu, b, 0);
-        if ((int64_t)b >= total) {
+      if (left == 0u) {
+        if (lane == 0) {
+          // replay: camera tasks [0, paths) (after a tape pass: the paths on
+          // the lost list), then the checkpoints that were written
+          const int64_t total = !kRep ? Q.total
+                                      : (Q.lost_list != nullptr ? (int64_t)*Q.lost_count
+                                                                : Q.total + min((int64_t)*Q.ckpt_count, Q.ckpt_cap));
+          const int64_t b = (int64_t)atomicAdd(Q.counter, (unsigned long long)Q.batch);
+          if (b < total) {
+            *next = (unsigned long long)b;
+            left = (unsigned)min((int64_t)Q.batch, total - b);
+          }
+        }
+        left = __shfl_sync(0xffffffffu, left, 0);
+        if (left == 0u) {
           queue_empty = true;
           break;
         }
-        batch_next = (int64_t)b;
-        batch_end = min((int64_t)b + Q.batch, total);
       }
-      const unsigned avail = (unsigned)(batch_end - batch_next);
-      const unsigned take = min((unsigned)__popc(need), avail);
+      const unsigned take = min((unsigned)__popc(need), left);
       const unsigned rank = (unsigned)__popc(need & lt_mask);
       if (((need >> lane) & 1u) && rank < take) {
-        path = batch_next + rank;
+        const uint64_t path = *next + rank;
+        U(cPath) = (uint32_t)path;
+        U(cPathHi) = (uint32_t)(path >> 32);
         phase = kStart;
       }
-      batch_next += take;
+      __syncwarp();
+      if (lane == 0) *next += take;
+      left -= take;
       need = __ballot_sync(0xffffffffu, phase == kIdle);
     }
     const unsigned m_start = __ballot_sync(0xffffffffu, phase == kStart);
@@ -396,18 +412,21 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     const bool run_scat = (unsigned)__popc(m_scat) >= need_lanes || (m_walk == 0u && m_scat != 0u);
 
     bool finished = false;  // the lane's current path (or task) ends this iteration
+    // the shadow walk ends in this iteration (handled below, after the tape)
+    bool nee_done = false;
     // kTape: this iteration's events, appended where the warp has
-    // reconverged: a walk step (1: null collision at p, 2: shadow-walk step
-    // at q) with its reference and sigma_n, and the scattering event at p
+    // reconverged: a walk step at x (null collision or shadow-walk step) with
+    // its reference and sigma_n, and the scattering event at the cold vertex
     // processed in this iteration with its sigma_t
-    int ev_kind = 0;
+    bool ev_walk = false;
     uint32_t ev_ref = 0;
     float ev_f = 0.0f, ev_sf = 0.0f;
     bool ev_scat = false;
 
     // ------------------------------------------------------------ path start
     if (run_start && phase == kStart) {
-      iter0 = n_iter;
+      U(cIter0) = n_iter;
+      int64_t path = (int64_t)((uint64_t)U(cPath) | ((uint64_t)U(cPathHi) << 32));
       // replay: a checkpoint task resumes at its scattering event
       const bool resume = kRep && Q.lost_list == nullptr && path >= Q.total;
       float4 r0, r1, r2, r3;
@@ -422,6 +441,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       } else if (kRep && Q.lost_list != nullptr) {
         path = (int64_t)Q.lost_list[path];  // a path the tape could not hold
       }
+      U(cPath) = (uint32_t)path;
       if (kTable) Jp = &job_of(Q, path);
       const VolJob& J = kTable ? *Jp : single;
       const float mu_old = J.scale * bits_to_float(__ldg(J.maxbits + 0));
@@ -434,13 +454,15 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       const uint32_t uspp = (uint32_t)J.spp;
       const uint32_t k = local / uspp;
       const uint32_t smp = local - k * uspp;
-      pix = J.pixel_order != nullptr ? (int)__ldg(J.pixel_order + k) : (int)k;
-      sid = (uint32_t)pix * (uint32_t)J.spp + smp;
+      const int pix = J.pixel_order != nullptr ? (int)__ldg(J.pixel_order + k) : (int)k;
+      const uint32_t sid = (uint32_t)pix * (uint32_t)J.spp + smp;  // sample index within the job
+      U(cPix) = (uint32_t)pix;
+      U(cSid) = sid;
       seed_lane(rng, J.seed, sid);
       bo = V3{1, 1, 1};
       bn = V3{1, 1, 1};
-      Lo = V3{0, 0, 0};
-      Ln = V3{0, 0, 0};
+      put3(cLn, V3{0, 0, 0});
+      if (kMode == kTwoState) put3(cLo, V3{0, 0, 0});
       depth = 0;
       if (kRad) ck_lost = false;
       if (kMode == kTape) tref = (kEvCamera << 30) | (uint32_t)path;
@@ -456,12 +478,13 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
         } else {
           depth = __float_as_int(r0.y);
           rng.state = (uint64_t)__float_as_uint(r0.z) | ((uint64_t)__float_as_uint(r0.w) << 32);
-          p = V3{r1.x, r1.y, r1.z};
+          x = V3{r1.x, r1.y, r1.z};
           bn = V3{r1.w, r2.x, r2.y};
-          Ln = V3{r2.z, r2.w, r3.x};
+          const V3 Ln{r2.z, r2.w, r3.x};
+          put3(cLn, Ln);
           Lrem = V3{Lrem.x - Ln.x, Lrem.y - Ln.y, Lrem.z - Ln.z};
           if (kMode == kForward) cn_task = V3{r3.y, r3.z, r3.w};
-          sc_n = J.scale * density_new(J, locate(J, p));
+          F(cScn) = J.scale * density_new(J, locate(J, x));
           own_event = true;
           phase = kScatter;
         }
@@ -469,12 +492,12 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
         const float u0 = next1d(rng), u1 = next1d(rng);
         V3 o;
         const uint32_t py = (uint32_t)pix / (uint32_t)J.width;
-        camera_ray(J, (int)((uint32_t)pix - py * (uint32_t)J.width), (int)py, u0, u1, o, d);
+        camera_ray(J, (int)((uint32_t)pix - py * (uint32_t)J.width), (int)py, u0, u1, o, dir);
         (void)next1d(rng);  // colour channel for free-flight sampling (grey extinction)
         if (!roulette<kMode>(J, rng, depth, bn, bo)) {
           finished = true;
         } else {
-          const V3 inv_d = recip(d);
+          const V3 inv_d = recip(dir);
           float tn, tf;
           slab(o, inv_d, tn, tf);
           if (!(tn <= tf && tf > 0.0f)) {
@@ -482,29 +505,29 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             if (!J.hide_emitters) {
               if (kEnv) {
                 float pdf;
-                const V3 Le = env_radiance_dir(J, d, pdf);
-                Ln = V3{Ln.x + bn.x * Le.x, Ln.y + bn.y * Le.y, Ln.z + bn.z * Le.z};
-                if (kMode == kTwoState) Lo = V3{Lo.x + bo.x * Le.x, Lo.y + bo.y * Le.y, Lo.z + bo.z * Le.z};
+                const V3 Le = env_radiance_dir(J, dir, pdf);
+                put3(cLn, V3{bn.x * Le.x, bn.y * Le.y, bn.z * Le.z});
+                if (kMode == kTwoState) put3(cLo, V3{bo.x * Le.x, bo.y * Le.y, bo.z * Le.z});
               } else {
-                Ln = V3{Ln.x + bn.x, Ln.y + bn.y, Ln.z + bn.z};
-                if (kMode == kTwoState) Lo = V3{Lo.x + bo.x, Lo.y + bo.y, Lo.z + bo.z};
+                put3(cLn, bn);
+                if (kMode == kTwoState) put3(cLo, bo);
               }
             }
             finished = true;
           } else {
             // null BSDF of the cube boundary: its 1D + 2D sample is drawn and discarded
             pcg_skip3(rng);
-            p = advance(o, fmaxf(tn, 0.0f), d);
+            x = advance(o, fmaxf(tn, 0.0f), dir);
             float a;
-            slab(p, inv_d, a, t_rem);
+            slab(x, inv_d, a, rem);
             phase = kMain;
           }
         }
       }
     }
 
-    if (kMode == kReplay && run_start && iter0 == n_iter) {
-      const V3 g = pixel_dL(kTable ? *Jp : single, pix);  // the task started in this iteration
+    if (kMode == kReplay && run_start && phase != kIdle && U(cIter0) == n_iter) {
+      const V3 g = pixel_dL(kTable ? *Jp : single, (int)U(cPix));  // the task started in this iteration
       s_main = (g.x * Lrem.x + g.y * Lrem.y) + g.z * Lrem.z;
     }
 
@@ -516,9 +539,9 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       } else if (kRep && task == kTaskCheckpoint && !own_event) {
         finished = true;
       } else {
-        const Lookup lk = locate(J, p);
-        const AlbedoLookup alk = albedo_lookup(J, lk, p);
-        const float st_n = sc_n, st_o = sc_o;
+        const Lookup lk = locate(J, x);
+        const AlbedoLookup alk = albedo_lookup(J, lk, x);
+        const float st_n = F(cScn), st_o = kMode == kTwoState ? F(cSco) : 0.0f;
         const V3 an = albedo_at(J, alk, 1);
         const V3 ss_n{st_n * an.x, st_n * an.y, st_n * an.z};
         if (kMode == kTwoState) {
@@ -534,7 +557,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
           if (kMode == kReplay) {
             // d log(sigma_s) / d density and d log(albedo) / d albedo at the event
             const V3 Lr = Lrem;
-            const V3 g = pixel_dL(J, pix);
+            const V3 g = pixel_dL(J, (int)U(cPix));
             const float sd = s_main;  // (g . Lr)
             scatter_density(J, lk, (J.scale * sd) / st_n);
             if (kCount) ++cnt.grad_events;
@@ -564,7 +587,10 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             bn = V3{bn.x * (ss_n.x * k1), bn.y * (ss_n.y * k1), bn.z * (ss_n.z * k1)};
           }
         }
-        if (kMode == kAdjoint) ck_state = rng.state;
+        if (kMode == kAdjoint) {  // random-number state at the event, for its checkpoint
+          U(cCk) = (uint32_t)rng.state;
+          U(cCk + 1) = (uint32_t)(rng.state >> 32);
+        }
         if (kMode == kTape && !ck_lost) {
           // the event's record, written when its shadow walk ends; the walk's
           // steps refer to it (a path without one is replayed instead)
@@ -575,18 +601,21 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             ev_sf = st_n;
           } else {
             ck_lost = true;
-            tref = (kEvCamera << 30) | (uint32_t)path;
+            tref = (kEvCamera << 30) | U(cPath);
           }
         }
         // isotropic phase sample (1D unused + 2D), plugins/twostatevolpath.py:275
         pcg_skip1(rng);
         const float pu0 = next1d(rng), pu1 = next1d(rng);
-        wo_next = to_box(J, uniform_sphere(pu0, pu1));
+        put3(cP, x);
         {
-          // exit distance of the next segment, needed when the NEE walk
-          // ends; computed here, where many lanes run together
-          float a;
-          slab(p, recip(wo_next), a, t_rem);
+          // the next segment, needed when the NEE walk ends; its exit
+          // distance is computed here, where many lanes run together
+          const V3 wo = to_box(J, uniform_sphere(pu0, pu1));
+          float a, t_next;
+          slab(x, recip(wo), a, t_next);
+          put3(cWo, wo);
+          F(cT) = t_next;
         }
         // NEE towards the environment, then ratio tracking
         const float nu0 = next1d(rng), nu1 = next1d(rng);
@@ -596,22 +625,24 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
           // phase function's pdf
           V3 Le;
           float pdf;
-          w = to_box(J, env_sample(J.env, nu0, nu1, Le, pdf));
+          dir = to_box(J, env_sample(J.env, nu0, nu1, Le, pdf));
           float k = 0.0f;
           if (pdf > 0.0f && pdf < kInf) k = (kInvFourPi * env_mis(pdf, kInvFourPi)) / pdf;
-          env_e[0] = Le.x * k;
-          env_e[1] = Le.y * k;
-          env_e[2] = Le.z * k;
+          // NEE weight of the pending shadow ray (Le / pdf * phase * MIS)
+          put3(cEnv, V3{Le.x * k, Le.y * k, Le.z * k});
         } else {
-          w = to_box(J, uniform_sphere(nu0, nu1));
+          dir = to_box(J, uniform_sphere(nu0, nu1));
         }
-        q = p;
         {
           float a;
-          slab(q, recip(w), a, tr_rem);
+          slab(x, recip(dir), a, rem);
         }
-        tro = 1.0f;
+        F(cBn) = bn.x;
         trn = 1.0f;
+        if (kMode == kTwoState) {
+          F(cBo) = bo.x;
+          tro = 1.0f;
+        }
         phase = kNee;
         if (kRep) {
           if (task == kTaskCheckpoint) {
@@ -624,7 +655,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             }
             Lrem = V3{Lrem.x - cn.x, Lrem.y - cn.y, Lrem.z - cn.z};
             if (kMode == kReplay) {
-              const V3 g = pixel_dL(J, pix);
+              const V3 g = pixel_dL(J, (int)U(cPix));
               s_nee = (g.x * cn.x + g.y * cn.y) + g.z * cn.z;
               s_main = (g.x * Lrem.x + g.y * Lrem.y) + g.z * Lrem.z;
             }
@@ -655,29 +686,17 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       const int n_coop = __popc(m_coop);
       if (n_coop >= 1 && n_coop <= 8) {
         const bool mw = phase == kMain;
-        V3 org = mw ? p : q;
-        const V3 dir = mw ? d : w;
-        float tmax = mw ? t_rem : tr_rem;
-        V3 c1 = mw ? bn : V3{trn, 0.0f, 0.0f};
-        V3 c2 = mw ? bo : V3{tro, 0.0f, 0.0f};
         float* s = s_coop + (threadIdx.x >> 5) * 96;
-        const int f = coop_walk<kMode, kTable>(m_coop, mw, single, Jp, rng, mu, inv_mu, 0.5f * inv_mu, org, dir, tmax, c1, c2, s,
-                                       s + 32, s + 64, Q, tc, tref, ck_lost);
+        const int f = coop_walk<kMode, kTable>(m_coop, mw, single, Jp, rng, mu, inv_mu, 0.5f * inv_mu, x, dir, rem, bn,
+                                               bo, s, s + 32, s + 64, Q, tc, tref, ck_lost);
         if (f > 0) {
-          if (mw) {
-            p = org;
-            t_rem = tmax;
-            bn = c1;
-            if (kMode == kTwoState) bo = c2;
-            if (kCount) cnt.lookups += (unsigned)f;
-          } else {
-            q = org;
-            tr_rem = tmax;
-            trn = c1.x;
-            if (kMode == kTwoState) tro = c2.x;
-            if (kCount) cnt.nee_lookups += (unsigned)f;
+          if (kCount) {
+            if (mw)
+              cnt.lookups += (unsigned)f;
+            else
+              cnt.nee_lookups += (unsigned)f;
           }
-          iter0 -= (uint32_t)f;  // the path's cost counts its steps
+          U(cIter0) -= (uint32_t)f;  // the path's cost counts its steps
         }
       }
     }
@@ -685,25 +704,11 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     // --------------------------------------------------- free-flight step
     if (phase == kMain || phase == kNee || phase == kNeeAdj) {
       const VolJob& J = kTable ? *Jp : single;
-      bool alive = true;
-      V3 org, dir;
-      float tmax;
       // whole-path replay: the second shadow walk draws from the saved stream
       // (chosen by value, not through a pointer, which would put both
       // streams in local memory)
-      bool nee_stream = false;
-      if (phase == kMain) {
-        alive = roulette<kMode>(J, rng, depth, bn, bo);
-        org = p;
-        dir = d;
-        tmax = t_rem;
-      } else {
-        org = q;
-        dir = w;
-        tmax = tr_rem;
-        nee_stream = kRep && phase == kNeeAdj && task == kTaskWhole;
-      }
-      if (!alive) {
+      const bool nee_stream = kRep && phase == kNeeAdj && task == kTaskWhole;
+      if (phase == kMain && !roulette<kMode>(J, rng, depth, bn, bo)) {
         finished = true;
       } else {
         // majorant of this collision: global, or the supergrid cell it lies in
@@ -711,18 +716,17 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
         float t;
         if (kSG && J.sg[0] > 0) {
           const float tau = -log_unit(1.0f - (nee_stream ? next1d_state(nee_state, rng.inc) : next1d(rng)));
-          t = supergrid_flight(J, kMode == kTwoState ? J.sg_two : J.sg_new, org, dir, tmax, tau, mu_c);
+          t = supergrid_flight(J, kMode == kTwoState ? J.sg_two : J.sg_new, x, dir, rem, tau, mu_c);
           inv_c = 1.0f / mu_c;
           hinv_c = 0.5f * inv_c;
         } else {
           t = free_flight(nee_stream ? next1d_state(nee_state, rng.inc) : next1d(rng), mu, inv_mu);
         }
-        const bool valid = t <= tmax;
+        const bool valid = t <= rem;
         Lookup lk;
         float rho_o = 0.0f, rho_n = 0.0f;
-        V3 x;
         if (valid) {
-          x = advance(org, t, dir);
+          x = advance(x, t, dir);  // the step's end, whatever happens there
           lk = locate(J, x);
           if (kMode == kTwoState)
             density2(J, lk, rho_o, rho_n);
@@ -768,10 +772,9 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
                 dL = V3{dL.x + Lr.x * f, dL.y + Lr.y * f, dL.z + Lr.z * f};
                 if (kCount) ++cnt.grad_events;
               }
-              p = x;
-              t_rem = t_rem - t;
+              rem = rem - t;
               if (kMode == kTape) {
-                ev_kind = 1;
+                ev_walk = true;
                 ev_ref = tref;
                 ev_f = mu_c - st_n;
               }
@@ -782,9 +785,8 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
                 finished = true;
               } else {
                 if (kCount) ++cnt.scatters;
-                p = x;
-                sc_n = st_n;
-                sc_o = st_o;
+                F(cScn) = st_n;
+                if (kMode == kTwoState) F(cSco) = st_o;
                 phase = kScatter;
               }
             }
@@ -792,11 +794,13 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             // leaves the cube: null BSDF sample, outside iteration RR, environment
             pcg_skip3(rng);
             if (roulette<kMode>(J, rng, depth, bn, bo) && !(J.hide_emitters && depth == 0)) {
+              V3 Ln = get3(cLn), Lo{0, 0, 0};
+              if (kMode == kTwoState) Lo = get3(cLo);
               if (kEnv) {
                 // environment map hit after a phase sample: power heuristic
                 // against NEE (plugins/twostatevolpath.py:288-308)
                 float pdf;
-                const V3 Le = env_radiance_dir(J, d, pdf);
+                const V3 Le = env_radiance_dir(J, dir, pdf);
                 const float k = depth == 0 ? 1.0f : env_mis(kInvFourPi, pdf);
                 Ln = V3{Ln.x + (bn.x * Le.x) * k, Ln.y + (bn.y * Le.y) * k, Ln.z + (bn.z * Le.z) * k};
                 if (kMode == kTwoState)
@@ -806,82 +810,24 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
                 Ln = V3{Ln.x + bn.x * k, Ln.y + bn.y * k, Ln.z + bn.z * k};
                 if (kMode == kTwoState) Lo = V3{Lo.x + bo.x * k, Lo.y + bo.y * k, Lo.z + bo.z * k};
               }
+              put3(cLn, Ln);
+              if (kMode == kTwoState) put3(cLo, Lo);
             }
             finished = true;
           }
         } else if (phase == kNee) {
-          bool done = !valid;
+          nee_done = !valid;
           if (valid) {
             // ratio tracking (plugins/twostatevolpath.py:443-452)
             trn = trn * ((mu_c - st_n) * inv_c);
             if (kMode == kTwoState) tro = tro * ((mu_c - st_o) * inv_c);
-            q = x;
-            tr_rem = tr_rem - t;
+            rem = rem - t;
             if (kMode == kTape) {
-              ev_kind = 2;
+              ev_walk = true;
               ev_ref = tref;
               ev_f = mu_c - st_n;
             }
-            done = (kMode == kTwoState) ? (trn == 0.0f && tro == 0.0f) : (trn == 0.0f);
-          }
-          if (done) {
-            V3 cn;
-            if (kEnv) {
-              cn = V3{(bn.x * env_e[0]) * trn, (bn.y * env_e[1]) * trn, (bn.z * env_e[2]) * trn};
-            } else {
-              const float en = emit_weight * trn;
-              cn = V3{((bn.x * kInvFourPi) * mis) * en, ((bn.y * kInvFourPi) * mis) * en,
-                      ((bn.z * kInvFourPi) * mis) * en};
-            }
-            if (kMode == kAdjoint && !ck_lost) {
-              const unsigned long long slot = atomicAdd(Q.ckpt_count, 1ull);
-              if ((int64_t)slot < Q.ckpt_cap)
-                write_checkpoint(Q.ckpt + slot * 4, (uint32_t)path, depth, ck_state, p, bn, Ln, cn);
-              else
-                ck_lost = true;
-            }
-            if (kMode == kTape && (tref >> 30) == kEvShadow) {
-              // the scattering event's record: its path, the radiance gathered
-              // before its NEE contribution, and that contribution; the event
-              // itself goes on the tape, and the next segment's null
-              // collisions refer to the record too
-              const uint32_t k = tref & kTapeIndexMask;
-              float4* rec = Q.ckpt + (int64_t)k * 2;
-              __stcs(rec, make_float4(__uint_as_float((uint32_t)path), Ln.x, Ln.y, Ln.z));
-              __stcs(rec + 1, make_float4(cn.x, cn.y, cn.z, 0.0f));
-              tref = (kEvSegment << 30) | k;
-            }
-            Ln = V3{Ln.x + cn.x, Ln.y + cn.y, Ln.z + cn.z};
-            if (kRep) Lrem = V3{Lrem.x - cn.x, Lrem.y - cn.y, Lrem.z - cn.z};
-            if (kMode == kTwoState) {
-              if (kEnv) {
-                Lo = V3{Lo.x + (bo.x * env_e[0]) * tro, Lo.y + (bo.y * env_e[1]) * tro,
-                        Lo.z + (bo.z * env_e[2]) * tro};
-              } else {
-                const float eo = emit_weight * tro;
-                Lo = V3{Lo.x + ((bo.x * kInvFourPi) * mis) * eo, Lo.y + ((bo.y * kInvFourPi) * mis) * eo,
-                        Lo.z + ((bo.z * kInvFourPi) * mis) * eo};
-              }
-            }
-            if (kRep) {
-              // whole-path replay: walk the shadow ray again (saved stream) to
-              // back-propagate through its transmittance
-              if (kMode == kReplay) {
-                const V3 g = pixel_dL(J, pix);
-                s_nee = (g.x * cn.x + g.y * cn.y) + g.z * cn.z;
-                s_main = (g.x * Lrem.x + g.y * Lrem.y) + g.z * Lrem.z;
-              } else {
-                cn_task = cn;
-              }
-              q = p;
-              float a;
-              slab(q, recip(w), a, tr_rem);
-              trn = 1.0f;
-              phase = kNeeAdj;
-            } else {
-              d = wo_next;  // t_rem was set at the scattering event
-              phase = kMain;
-            }
+            nee_done = (kMode == kTwoState) ? (trn == 0.0f && tro == 0.0f) : (trn == 0.0f);
           }
         } else {  // kNeeAdj: the shadow walk with gradients
           bool done = !valid;
@@ -897,12 +843,14 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
               if (kCount) ++cnt.grad_events;
             }
             trn = trn * (sn * inv_c);
-            q = x;
-            tr_rem = tr_rem - t;
+            rem = rem - t;
             done = trn == 0.0f;
           }
           if (done) {
-            d = wo_next;  // t_rem was set at the scattering event
+            bn.x = F(cBn);
+            x = get3(cP);
+            dir = get3(cWo);
+            rem = F(cT);
             phase = kMain;
           }
         }
@@ -910,32 +858,106 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     }
 
     if (kMode == kTape) {
-      if (!tape_append(Q, tc, ev_kind != 0 && !ck_lost, ev_kind == 2 ? q : p, ev_ref, ev_f)) ck_lost = true;
-      if (!tape_append(Q, tc, ev_scat && !ck_lost, p, (kEvScatter << 30) | (tref & kTapeIndexMask), ev_sf))
+      if (!tape_append(Q, tc, ev_walk && !ck_lost, x, ev_ref, ev_f)) ck_lost = true;
+      if (!tape_append(Q, tc, ev_scat && !ck_lost, get3(cP), (kEvScatter << 30) | (tref & kTapeIndexMask), ev_sf))
         ck_lost = true;
+    }
+
+    // -------------------------------------------------- end of the shadow walk
+    if (nee_done) {
+      const VolJob& J = kTable ? *Jp : single;
+      const V3 p = get3(cP);
+      const float tn = trn, to = tro;
+      bn.x = F(cBn);
+      if (kMode == kTwoState) bo.x = F(cBo);
+      V3 Ln = get3(cLn);
+      V3 cn;
+      if (kEnv) {
+        const V3 e = get3(cEnv);
+        cn = V3{(bn.x * e.x) * tn, (bn.y * e.y) * tn, (bn.z * e.z) * tn};
+      } else {
+        const float en = emit_weight * tn;
+        cn = V3{((bn.x * kInvFourPi) * mis) * en, ((bn.y * kInvFourPi) * mis) * en,
+                ((bn.z * kInvFourPi) * mis) * en};
+      }
+      if (kMode == kAdjoint && !ck_lost) {
+        const unsigned long long slot = atomicAdd(Q.ckpt_count, 1ull);
+        if ((int64_t)slot < Q.ckpt_cap)
+          write_checkpoint(Q.ckpt + slot * 4, U(cPath), depth, (uint64_t)U(cCk) | ((uint64_t)U(cCk + 1) << 32), p, bn,
+                           Ln, cn);
+        else
+          ck_lost = true;
+      }
+      if (kMode == kTape && (tref >> 30) == kEvShadow) {
+        // the scattering event's record: its path, the radiance gathered
+        // before its NEE contribution, and that contribution; the event
+        // itself goes on the tape, and the next segment's null
+        // collisions refer to the record too
+        const uint32_t k = tref & kTapeIndexMask;
+        float4* rec = Q.ckpt + (int64_t)k * 2;
+        __stcs(rec, make_float4(__uint_as_float(U(cPath)), Ln.x, Ln.y, Ln.z));
+        __stcs(rec + 1, make_float4(cn.x, cn.y, cn.z, 0.0f));
+        tref = (kEvSegment << 30) | k;
+      }
+      Ln = V3{Ln.x + cn.x, Ln.y + cn.y, Ln.z + cn.z};
+      put3(cLn, Ln);
+      if (kRep) Lrem = V3{Lrem.x - cn.x, Lrem.y - cn.y, Lrem.z - cn.z};
+      if (kMode == kTwoState) {
+        V3 Lo = get3(cLo);
+        if (kEnv) {
+          const V3 e = get3(cEnv);
+          Lo = V3{Lo.x + (bo.x * e.x) * to, Lo.y + (bo.y * e.y) * to, Lo.z + (bo.z * e.z) * to};
+        } else {
+          const float eo = emit_weight * to;
+          Lo = V3{Lo.x + ((bo.x * kInvFourPi) * mis) * eo, Lo.y + ((bo.y * kInvFourPi) * mis) * eo,
+                  Lo.z + ((bo.z * kInvFourPi) * mis) * eo};
+        }
+        put3(cLo, Lo);
+      }
+      x = p;
+      if (kRep) {
+        // whole-path replay: walk the shadow ray again (saved stream) to
+        // back-propagate through its transmittance
+        if (kMode == kReplay) {
+          const V3 g = pixel_dL(J, (int)U(cPix));
+          s_nee = (g.x * cn.x + g.y * cn.y) + g.z * cn.z;
+          s_main = (g.x * Lrem.x + g.y * Lrem.y) + g.z * Lrem.z;
+        } else {
+          cn_task = cn;
+        }
+        float a;
+        slab(x, recip(dir), a, rem);
+        trn = 1.0f;  // bn.x is still cold
+        phase = kNeeAdj;
+      } else {
+        dir = get3(cWo);
+        rem = F(cT);
+        phase = kMain;
+      }
     }
 
     // -------------------------------------------------------------- path end
     if (finished) {
       const VolJob& J = kTable ? *Jp : single;
       if (kMode == kTwoState || kMode == kSingle) {
-        float4* o = Q.path_out + (J.path_begin + sid) * (kMode == kTwoState ? 2 : 1);
-        __stcs(o, make_float4(Ln.x, Ln.y, Ln.z, 0.0f));
-        if (kMode == kTwoState) __stcs(o + 1, make_float4(Lo.x, Lo.y, Lo.z, 0.0f));
+        float4* o = Q.path_out + (J.path_begin + U(cSid)) * (kMode == kTwoState ? 2 : 1);
+        __stcs(o, make_float4(F(cLn), F(cLn + 1), F(cLn + 2), 0.0f));
+        if (kMode == kTwoState) __stcs(o + 1, make_float4(F(cLo), F(cLo + 1), F(cLo + 2), 0.0f));
       }
-      if (kRad) __stcs(Q.path_ltot + path, make_float4(Ln.x, Ln.y, Ln.z, ck_lost ? 1.0f : 0.0f));
-      if (kMode == kTape && ck_lost) Q.lost_list[atomicAdd(Q.lost_count, 1ull)] = (uint32_t)path;
+      if (kRad)
+        __stcs(Q.path_ltot + U(cPath), make_float4(F(cLn), F(cLn + 1), F(cLn + 2), ck_lost ? 1.0f : 0.0f));
+      if (kMode == kTape && ck_lost) Q.lost_list[atomicAdd(Q.lost_count, 1ull)] = U(cPath);
       if (kMode == kForward && (dL.x != 0.0f || dL.y != 0.0f || dL.z != 0.0f)) {
         // the task's share of its pixel's derivative (the pixel value is the
         // mean of its samples)
         const float fs = (float)J.spp;
-        float* o = J.out_img + (int64_t)pix * 3;
+        float* o = J.out_img + (int64_t)U(cPix) * 3;
         atomicAdd(o + 0, dL.x / fs);
         atomicAdd(o + 1, dL.y / fs);
         atomicAdd(o + 2, dL.z / fs);
       }
       if (kCount && !kRep) ++cnt.paths;
-      if (J.pixel_cost != nullptr) red_add_u32(J.pixel_cost + pix, n_iter - iter0);
+      if (J.pixel_cost != nullptr) red_add_u32(J.pixel_cost + U(cPix), n_iter - U(cIter0));
       phase = kIdle;
     }
   }

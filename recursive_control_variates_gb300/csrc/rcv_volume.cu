@@ -270,6 +270,10 @@ int make_volume_job(const rcv_medium* m, const rcv_sensor* s, const rcv_volpath_
   J->dy = m->dims[1];
   J->dz = m->dims[2];
   J->scale = m->scale;
+  J->fdx = (float)m->dims[0];
+  J->fdy = (float)m->dims[1];
+  J->fdz = (float)m->dims[2];
+  J->long_axis = (m->dims[0] | m->dims[1] | m->dims[2]) >= (1 << 21) ? 1 : 0;
   const MediumLayout L = medium_layout(m);
   char* ws = static_cast<char*>(m->workspace);
   J->cells = reinterpret_cast<const float4*>(ws + L.cells);

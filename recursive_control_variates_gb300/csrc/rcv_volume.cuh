@@ -62,6 +62,8 @@ struct VolJob {
   // medium
   int32_t dx, dy, dz;
   float scale;
+  float fdx, fdy, fdz;  // dx, dy, dz
+  int32_t long_axis;    // an axis has 2^21 voxels or more
   const float4* __restrict__ cells;   // (dz+1)(dy+1)(dx+1) * 4
   const float4* __restrict__ albedo;  // adz*ady*adx * 2 (old, new) or null
   int32_t adx, ady, adz;              // albedo grid resolution
@@ -277,9 +279,15 @@ struct Lookup {
 
 __device__ __forceinline__ Lookup locate(const VolJob& J, const V3& x) {
   Lookup l;
-  l.ax = axis_coord(x.x, J.dx);
-  l.ay = axis_coord(x.y, J.dy);
-  l.az = axis_coord(x.z, J.dz);
+  if (J.long_axis) {
+    l.ax = axis_coord(x.x, J.dx);
+    l.ay = axis_coord(x.y, J.dy);
+    l.az = axis_coord(x.z, J.dz);
+  } else {
+    l.ax = axis_coord_magic(x.x, J.dx, J.fdx);
+    l.ay = axis_coord_magic(x.y, J.dy, J.fdy);
+    l.az = axis_coord_magic(x.z, J.dz, J.fdz);
+  }
   l.cell = ((uint32_t)l.az.cell * (uint32_t)(J.dy + 1) + (uint32_t)l.ay.cell) * (uint32_t)(J.dx + 1) +
            (uint32_t)l.ax.cell;
   return l;

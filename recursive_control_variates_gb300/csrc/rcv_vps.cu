@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(128) vps_kernel(const __grid_constant__ VolJob
 }
 
 template <int kMode, bool kSG, bool kEnv>
-__global__ void __launch_bounds__(kVpsBlock, 5) vps_trace_kernel(const __grid_constant__ VolJob J,
+__global__ void __launch_bounds__(kVpsBlock, 6) vps_trace_kernel(const __grid_constant__ VolJob J,
                                                                  const __grid_constant__ VpsParams P,
                                                                  const __grid_constant__ Queue Q) {
   trace_vps<kMode, kSG, kEnv>(J, P, Q);

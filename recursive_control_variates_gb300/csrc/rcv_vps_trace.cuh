@@ -93,13 +93,14 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
 
   const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
   const unsigned defer = (unsigned)Q.defer;
-  const int64_t total = kDrt ? (int64_t)*P.task_count : Q.total;
   const float mu = J.scale * bits_to_float(__ldg(J.maxbits + 1)), inv_mu = 1.0f / mu;
 
-  int64_t batch_next = 0, batch_end = 0;
+  __shared__ unsigned s_next[kVpsWarps];  // next path of the warp's claimed batch
+  unsigned* const next = s_next + (threadIdx.x >> 5);
+  unsigned left = 0u;  // paths left in it
   bool queue_empty = false;
   uint32_t path = 0;
-  int phase = kVIdle, pix = 0, depth = 0;
+  int phase = kVIdle, depth = 0;
   int stage = 0;  // kVpsDrt: 0 distance on the kept segment, 1 NEE there, 2 the path from there
   Pcg32 rng;
   V3 xo, sd, p, w;          // segment origin and direction; walk position and direction
@@ -108,31 +109,34 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
   bool lost = false;
   uint32_t rec = 0, nseg = 0;
   TapeCursor tc{0u, 0u};
-  uint32_t n_iter = 0, iter0 = 0;
 
   while (true) {
-    ++n_iter;
     unsigned need = __ballot_sync(0xffffffffu, phase == kVIdle);
     while (need != 0u && !queue_empty) {
-      if (batch_next == batch_end) {
-        unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(Q.counter, (unsigned long long)Q.batch);
-        b = __shfl_sync(0xffffffffu, b, 0);
-        if ((int64_t)b >= total) {
+      if (left == 0u) {
+        if (lane == 0) {
+          const int64_t total = kDrt ? (int64_t)*P.task_count : Q.total;
+          const int64_t b = (int64_t)atomicAdd(Q.counter, (unsigned long long)Q.batch);
+          if (b < total) {
+            *next = (unsigned)b;
+            left = (unsigned)min((int64_t)Q.batch, total - b);
+          }
+        }
+        left = __shfl_sync(0xffffffffu, left, 0);
+        if (left == 0u) {
           queue_empty = true;
           break;
         }
-        batch_next = (int64_t)b;
-        batch_end = min((int64_t)b + Q.batch, total);
       }
-      const unsigned avail = (unsigned)(batch_end - batch_next);
-      const unsigned take = min((unsigned)__popc(need), avail);
+      const unsigned take = min((unsigned)__popc(need), left);
       const unsigned rank = (unsigned)__popc(need & lt_mask);
       if (((need >> lane) & 1u) && rank < take) {
-        path = (uint32_t)(batch_next + rank);
+        path = *next + rank;
         phase = kVStart;
       }
-      batch_next += take;
+      __syncwarp();
+      if (lane == 0) *next += take;
+      left -= take;
       need = __ballot_sync(0xffffffffu, phase == kVIdle);
     }
     const unsigned m_start = __ballot_sync(0xffffffffu, phase == kVStart);
@@ -148,7 +152,7 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
 
     // ------------------------------------------------------------ path start
     if (run_start && phase == kVStart) {
-      iter0 = n_iter;
+      int pix;
       thr = V3{1, 1, 1};
       L = V3{0, 0, 0};
       if (kDrt) {
@@ -194,9 +198,7 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
         float tn, tf;
         slab(o, inv_d, tn, tf);
         if (!(tn <= tf && tf > 0.0f)) {
-          // misses the medium: no gradient, nothing to record
-          if (J.pixel_cost != nullptr) red_add_u32(J.pixel_cost + pix, 1u);
-          phase = kVIdle;
+          phase = kVIdle;  // misses the medium: no gradient, nothing to record
         } else {
           pcg_skip1(rng);  // the draw that seeds the second stream
           xo = advance(o, fmaxf(tn, 0.0f), d);
@@ -469,7 +471,6 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
             t[1] = make_float4((wmean * cur.x) / dmean, (wmean * cur.y) / dmean, (wmean * cur.z) / dmean, 0.0f);
           }
         }
-        if (J.pixel_cost != nullptr) red_add_u32(J.pixel_cost + pix, n_iter - iter0);
       }
       phase = kVIdle;
     }
