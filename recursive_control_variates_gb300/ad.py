@@ -88,7 +88,7 @@ class Adam:
             lr = self.lr_per_key.get(key, self.lr)
             _lib.check(
                 lib.rcv_adam_step(
-                    p.data.data_ptr(), g.data_ptr(), st[1].data_ptr(), st[2].data_ptr(), p.numel(), st[0], lr,
+                    p.data_ptr(), g.data_ptr(), st[1].data_ptr(), st[2].data_ptr(), p.numel(), st[0], lr,
                     self.beta_1, self.beta_2, self.epsilon, float(lo), float(hi), 1, stream_handle(p.device),
                 ),
                 "rcv_adam_step",

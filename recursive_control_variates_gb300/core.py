@@ -233,11 +233,15 @@ class PerspectiveSensor:
 
     def c_struct(self) -> _lib.Sensor:
         w, h = self.film_.width, self.film_.height
-        s = _lib.Sensor()
-        s.width, s.height = w, h
-        s.origin[:], s.forward[:], s.right[:], s.up[:] = self.frame(w, h)
-        s.count = 1
-        return s
+        frame = self.frame(w, h)
+        made = self.__dict__.get("_struct")
+        if made is None or made[0] is not frame:  # frames are memoised: the same one, the same struct
+            s = _lib.Sensor()
+            s.width, s.height = w, h
+            s.origin[:], s.forward[:], s.right[:], s.up[:] = frame
+            s.count = 1
+            made = self.__dict__["_struct"] = (frame, bytes(s))
+        return _lib.Sensor.from_buffer_copy(made[1])
 
 
 class BatchSensor:
@@ -267,14 +271,18 @@ class BatchSensor:
         n = len(self.sensors)
         w, h = self.film_.width, self.film_.height
         sub_w = w // n
-        s = _lib.Sensor()
-        s.width, s.height = w, h
-        s.origin[:], s.forward[:], s.right[:], s.up[:] = self.sensors[0].frame(sub_w, h)
-        s.count = n
-        for k, sub in enumerate(self.sensors[1:]):
-            f = s.more[k]
-            f.origin[:], f.forward[:], f.right[:], f.up[:] = sub.frame(sub_w, h)
-        return s
+        frames = [sub.frame(sub_w, h) for sub in self.sensors]
+        made = self.__dict__.get("_struct")
+        if made is None or made[0] != (w, h) or len(made[1]) != n or any(a is not b for a, b in zip(made[1], frames)):
+            s = _lib.Sensor()
+            s.width, s.height = w, h
+            s.origin[:], s.forward[:], s.right[:], s.up[:] = frames[0]
+            s.count = n
+            for k, frame in enumerate(frames[1:]):
+                f = s.more[k]
+                f.origin[:], f.forward[:], f.right[:], f.up[:] = frame
+            made = self.__dict__["_struct"] = ((w, h), frames, bytes(s))
+        return _lib.Sensor.from_buffer_copy(made[2])
 
 
 # ----------------------------------------------------------------- emitters
@@ -480,21 +488,30 @@ class _PackedMedium:
 
     def _describe(self, aligned: int) -> _lib.Medium:
         old, new = self._states()
-        m = _lib.Medium()
-        m.dims[:] = list(self.dims)
-        m.scale = new.scale
+        grid = new.albedo_grid
+        # what does not change from step to step, as bytes; a step fills in
+        # the addresses of its states
+        key = (new.density.shape, None if grid is None else grid.shape, new.scale, new.albedo_value, self._factor(),
+               new.box)
+        made = self.__dict__.get("_fixed")
+        if made is None or made[0] != key:
+            m = _lib.Medium()
+            m.dims[:] = list(self.dims)
+            m.scale = new.scale
+            m.albedo_value[:] = list(new.albedo_value)
+            m.majorant_factor = self._factor()
+            m.box_min[:] = [float(np.float32(v)) for v in new.box.box_min]
+            m.box_size[:] = [float(np.float32(v)) for v in new.box.box_size]
+            if grid is not None and tuple(self.albedo_dims) != tuple(self.dims):
+                m.albedo_dims[:] = list(self.albedo_dims)
+            made = self.__dict__["_fixed"] = (key, bytes(m))
+        m = _lib.Medium.from_buffer_copy(made[1])
         m.density_old = old.density.data_ptr()
         m.density_new = new.density.data_ptr()
-        if self.has_albedo_grid:
+        if grid is not None:
             m.albedo_old = old.albedo_grid.data_ptr()
-            m.albedo_new = new.albedo_grid.data_ptr()
-        m.albedo_value[:] = list(new.albedo_value)
-        m.majorant_factor = self._factor()
+            m.albedo_new = grid.data_ptr()
         m.workspace = aligned
-        m.box_min[:] = [float(np.float32(v)) for v in new.box.box_min]
-        m.box_size[:] = [float(np.float32(v)) for v in new.box.box_size]
-        if self.has_albedo_grid and tuple(self.albedo_dims) != tuple(self.dims):
-            m.albedo_dims[:] = list(self.albedo_dims)
         return m
 
     def prepare(self, stream) -> _lib.Medium:
@@ -788,7 +805,7 @@ class SceneParameters:
         owner, sub = self._owners[key]
         cur = owner.traverse()[sub] if hasattr(owner, "traverse") else None
         v = value if isinstance(value, torch.Tensor) else torch.as_tensor(np.asarray(value, np.float32))
-        if cur is not None and tuple(v.shape) != tuple(cur.shape):
+        if cur is not None and v.shape != cur.shape:
             if v.numel() == 1:
                 v = v.reshape(()).expand(cur.shape)
             elif not (hasattr(owner, "set_grid") and v.dim() == cur.dim() == 4 and v.shape[-1] == cur.shape[-1]):
@@ -802,16 +819,18 @@ class SceneParameters:
                 if key in self._owners:
                     self[key] = opt[key]
         owners = {}
-        for key in self._pending:
-            owner, sub = self._owners[key]
-            dst = owner.traverse()[sub]
-            val = self._values[key].detach()
-            with torch.no_grad():
-                if tuple(val.shape) != tuple(dst.shape) and val.numel() != dst.numel():
+        with torch.no_grad():
+            for key in self._pending:
+                owner, sub = self._owners[key]
+                dst = owner.traverse()[sub]
+                val = self._values[key].detach()
+                if val.shape != dst.shape and val.numel() != dst.numel():
                     owner.set_grid(sub, val)  # a new resolution
+                elif val.shape == dst.shape and val.dtype == torch.float32 and val.device == dst.device:
+                    dst.copy_(val)
                 else:
                     dst.copy_(val.to(dst.device, torch.float32).reshape(dst.shape))
-            owners[id(owner)] = owner
+                owners[id(owner)] = owner
         self._pending.clear()
         for owner in owners.values():
             owner.parameters_changed()

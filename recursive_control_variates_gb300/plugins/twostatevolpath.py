@@ -138,10 +138,10 @@ class _VolumeIntegratorBase:
         if t is not None:
             torch.cuda.current_stream(device).wait_event(t[1])
 
-    def _adjoint_key(self, scene, medium, sensor, seed: int, spp: int):
-        o = self.options(scene)
-        return (id(medium), medium.version, id(sensor), seed & 0xFFFFFFFF, int(spp),
-                tuple(getattr(o, f) for f, _ in o._fields_))
+    @staticmethod
+    def _adjoint_key(o, medium, sensor, seed: int, spp: int):
+        """What an adjoint radiance pass depends on (o: the call's options)."""
+        return (id(medium), medium.version, id(sensor), seed & 0xFFFFFFFF, int(spp), bytes(o))
 
     def prefetch_adjoint(self, scene, sensor=0, seed: int = 0, spp: int = 0):
         """Prepares the adjoint's first launch (each path's radiance and its
@@ -164,15 +164,17 @@ class _VolumeIntegratorBase:
         s = sensor.c_struct()
         o = self.options(scene)
         ws = self.adjoint_scratch(dev, sensor, spp)
-        packed = torch.cuda.Event()
-        packed.record(main)
-        key = self._adjoint_key(scene, medium, sensor, seed, spp)
-        side = self._side.get(dev)
-        if side is None:
-            side = self._side[dev] = torch.cuda.Stream(dev)
+        key = self._adjoint_key(o, medium, sensor, seed, spp)
         counters = self.counters_ptr(dev)
         pending = {"key": key, "seed": seed, "spp": spp, "ws": ws, "used": False}
         self._pending = pending if self.pair_adjoint else None
+        # where a render_twostates will most likely take the pass, the point
+        # that a pass on the side stream has to wait for is not recorded now:
+        # should it go there after all, it waits for the launches up to then
+        packed = None
+        if not (self.pair_adjoint and self.two_state):
+            packed = torch.cuda.Event()
+            packed.record(main)
 
         def launch():
             if self._pending is pending:
@@ -180,7 +182,13 @@ class _VolumeIntegratorBase:
             if pending["used"]:
                 return  # it ran in the launch of the two-state render
             self._drain_ticket(dev)
-            side.wait_event(packed)
+            side = self._side.get(dev)
+            if side is None:
+                side = self._side[dev] = torch.cuda.Stream(dev)
+            if packed is None:
+                side.wait_stream(main)
+            else:
+                side.wait_event(packed)
             with torch.cuda.stream(side), profiling.region("trace_adjoint_radiance", dev):
                 _lib.check(
                     _lib.load().rcv_render_adjoint_radiance(
@@ -265,14 +273,14 @@ class _VolumeIntegratorBase:
         if tuple(g.shape) != (f.height, f.width, 3):
             raise ValueError(f"grad_in has shape {tuple(g.shape)}, expected {(f.height, f.width, 3)}")
         dev = medium.device
+        o = self.options(scene)
         ticket, key = self._ticket, None
         if ticket is not None:
-            key = self._adjoint_key(scene, medium, sensor, seed, spp)
+            key = self._adjoint_key(o, medium, sensor, seed, spp)
         self._drain_ticket(dev)  # orders this stream after a radiance pass started ahead
         st = stream_handle(dev)
         m = medium.prepare(st)
         s = sensor.c_struct()
-        o = self.options(scene)
         dx, dy, dz = medium.dims
         gd = torch.zeros((dz, dy, dx, 1), dtype=torch.float32, device=dev)
         ga = medium.albedo_grad_buffer()
@@ -392,9 +400,10 @@ class TwoStatePRBVolpathIntegrator(_VolumeIntegratorBase):
         # an adjoint radiance pass prepared for this medium state, sensor and
         # options runs in the same launch
         pend, self._pending = self._pending, None
-        key = self._adjoint_key(scene, medium, sensor, 0, 0)
-        if pend is not None and (pend["key"][:3] != key[:3] or pend["key"][5:] != key[5:]):
-            pend = None
+        if pend is not None:
+            key = self._adjoint_key(o, medium, sensor, 0, 0)
+            if pend["key"][:3] != key[:3] or pend["key"][5] != key[5]:
+                pend = None
         with profiling.region("trace_twostate", medium.device):
             if pend is None:
                 fn = "rcv_render_twostates_volume"

@@ -40,12 +40,17 @@ class KernelTimer:
         return out
 
 
-@contextlib.contextmanager
+_OFF = contextlib.nullcontext()
+
+
 def region(name: str, device=None):
+    """Context of a launch: timed while a ``KernelTimer`` is active."""
     t = _active
-    if t is None:
-        yield
-        return
+    return _OFF if t is None else _timed(t, name, device)
+
+
+@contextlib.contextmanager
+def _timed(t: KernelTimer, name: str, device):
     s = torch.cuda.current_stream(device)
     a = torch.cuda.Event(enable_timing=True)
     b = torch.cuda.Event(enable_timing=True)

@@ -9,10 +9,19 @@ import torch
 from . import _lib
 
 
+# torch's current stream as a bare handle: asking for the Stream object costs
+# ten times as much host time, and a step asks nine times
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_handle(device: torch.device | None = None) -> int:
     """cudaStream_t of torch's current stream on `device` (0 = legacy default)."""
-    if device is not None and device.type != "cuda":
-        raise RuntimeError("librcv kernels need CUDA tensors")
+    if device is not None:
+        if device.type != "cuda":
+            raise RuntimeError("librcv kernels need CUDA tensors")
+        if _raw_stream is not None and torch.cuda.is_initialized():
+            index = device.index
+            return _raw_stream(torch.cuda.current_device() if index is None else index)
     return torch.cuda.current_stream(device).cuda_stream
 
 
@@ -28,7 +37,10 @@ class _LossOp(torch.autograd.Function):
     @staticmethod
     def forward(ctx, img, ref, kind):
         img_c = img.detach().contiguous()
-        ref_c = ref.detach().to(img.device, torch.float32).contiguous()
+        ref_c = ref.detach()
+        if ref_c.dtype != torch.float32 or ref_c.device != img_c.device:
+            ref_c = ref_c.to(img_c.device, torch.float32)
+        ref_c = ref_c.contiguous()
         require_cuda(img_c, ref_c)
         if img_c.shape != ref_c.shape:
             raise ValueError(f"image shape {tuple(img_c.shape)} != reference shape {tuple(ref_c.shape)}")
