@@ -76,7 +76,7 @@ static JobLayout job_layout(const rcv_batch_job& j) {
   L.medium = off;
   off = align256(off + medium_layout(j.dims, j.albedo[0] != nullptr ? j.dims : nullptr, j.majorant_factor).total);
   L.buckets = off;
-  off = align256(off + kRenderOrderBuckets * sizeof(uint32_t));
+  off = align256(off + 2 * kRenderOrderBuckets * sizeof(uint32_t));
   L.order = off;
   off = align256(off + npix * sizeof(uint32_t));
   L.cost = off;
@@ -510,8 +510,14 @@ extern "C" int rcv_batch_job_init(const rcv_batch_job* job, void* stream) {
   VolJob J;
   rc = make_volume_job(&m, &job->sensor, &o, 0u, job->spp, &J);
   if (rc) return rc;
-  rc = order_pixels(J, reinterpret_cast<uint32_t*>(ws + L.buckets), reinterpret_cast<uint32_t*>(ws + L.order),
-                    nullptr, st);
+  OrderJob O;
+  O.J = J;
+  O.npix = J.width * J.height;
+  O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
+  O.order = reinterpret_cast<uint32_t*>(ws + L.order);
+  O.cost = nullptr;
+  RCV_TRY_CUDA(cudaMemsetAsync(O.buckets, 0, 2 * kRenderOrderBuckets * sizeof(uint32_t), st), "order reset");
+  rc = order_pixels(&O, 1, st);
   if (rc) return rc;
   const int npix = J.width * J.height;
   cost_from_chord_kernel<<<grid_for(npix, kBatchBlock), kBatchBlock, 0, st>>>(
@@ -780,11 +786,11 @@ static int enqueue_step(rcv_batch* b, cudaStream_t st) {
   if (b->tape) {
     // the gradient from the tape; the replay then takes only the lost paths
     rc = launch_tape_gradient(none, b->adj, n, b->adjbuf, b->tape_weights, b->cam_w, b->total_adj,
-                              cnt ? cnt + RCV_COUNTER_COUNT : nullptr, tracer_sm_count(), st);
+                              b->queue + 2, cnt ? cnt + RCV_COUNTER_COUNT : nullptr, tracer_sm_count(), st);
     if (rc) return rc;
   }
   rc = launch_persistent(kReplay, none, b->adj, n, b->total_adj, &b->opt, b->queue + 2, nullptr, &b->adjbuf,
-                         cnt ? cnt + RCV_COUNTER_COUNT : nullptr, st, sg);
+                         cnt ? cnt + RCV_COUNTER_COUNT : nullptr, st, sg, b->tape);
   if (rc) return rc;
   batch_update_kernel<<<(unsigned)b->vox_blocks, kBatchBlock, 0, st>>>(b->entries, pv, n);
   return launched("batch update launch");

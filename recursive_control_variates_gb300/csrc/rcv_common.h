@@ -115,12 +115,15 @@ inline MediumLayout medium_layout(const rcv_medium* m) {
 }
 
 // Scratch layout of one tracer call (all offsets 256-byte aligned):
-// counters (queue, checkpoints / event records, tape slots, lost paths) |
-// order bucket counts | pixel order | per-pixel cost | per-path radiance (32 B
+// counters (queue, checkpoints / event records, tape slots, lost paths, replay
+// queue) | order bucket counts | slots handed out per bucket | pixel order | per-pixel cost | per-path radiance (32 B
 // per path for two-state, 16 B single-state) | adjoint: per-path total
 // radiance | scatter checkpoints (tape: event records, then their weights) |
 // event tape | per-path camera-segment weight | lost-path list.
 constexpr int kRenderOrderBuckets = 256;
+// counters, bucket counts and hand-outs: one clear of the workspace's head
+// before a call (offset 0)
+constexpr uint64_t kRenderHeadBytes = 256 + 2 * kRenderOrderBuckets * sizeof(uint32_t);
 
 struct RenderLayout {
   uint64_t counter, buckets, order, cost, path_out, ltot, ckpt, tape, cam_w, lost, total;
@@ -169,7 +172,7 @@ inline RenderLayout render_layout(int64_t npix, int64_t paths, int mode) {
   RenderLayout L;
   L.counter = 0;
   L.buckets = 256;
-  L.order = align256(L.buckets + kRenderOrderBuckets * sizeof(uint32_t));
+  L.order = align256(kRenderHeadBytes);
   L.cost = align256(L.order + uint64_t(npix) * sizeof(uint32_t));
   L.path_out = align256(L.cost + uint64_t(npix) * sizeof(uint32_t));
   const bool adj = mode == RCV_MODE_ADJOINT;

@@ -68,7 +68,8 @@ __global__ void tape_weights_kernel(const __grid_constant__ VolJob single, const
                                     int njobs, const float4* __restrict__ rec,
                                     const unsigned long long* __restrict__ rec_count, int64_t rec_cap,
                                     float4* __restrict__ w, const float4* __restrict__ ltot,
-                                    float2* __restrict__ cam_w, int64_t paths) {
+                                    float2* __restrict__ cam_w, int64_t paths, unsigned long long* replay_counter) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *replay_counter = 0ull;
   const int64_t nrec = min((int64_t)*rec_count, rec_cap);
   const int64_t n = max(nrec, paths);
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
@@ -167,14 +168,16 @@ __global__ void __launch_bounds__(256) tape_scatter_kernel(const __grid_constant
 }
 
 int launch_tape_gradient(const VolJob& single, const VolJob* jobs, int njobs, const AdjBuffers& A, float4* weights,
-                         float2* cam_w, int64_t paths, uint64_t* counters, int sms, cudaStream_t st) {
+                         float2* cam_w, int64_t paths, unsigned long long* replay_counter, uint64_t* counters,
+                         int sms, cudaStream_t st) {
   const int block = 256;
   // grid-stride: the records' number is known on the device only, and their
   // room is many times it
   const unsigned need = grid_for(A.ckpt_cap > paths ? A.ckpt_cap : paths, block);
   const unsigned most = (unsigned)(sms > 0 ? sms : 1) * 16u;
   tape_weights_kernel<<<need < most ? need : most, block, 0, st>>>(
-      single, jobs, njobs, A.ckpt, A.ckpt_count, A.ckpt_cap, weights, A.path_ltot, cam_w, paths);
+      single, jobs, njobs, A.ckpt, A.ckpt_count, A.ckpt_cap, weights, A.path_ltot, cam_w, paths,
+      replay_counter);
   int rc = launched("tape_weights launch");
   if (rc) return rc;
   const unsigned grid = (unsigned)(sms > 0 ? sms : 1) * 8u;

@@ -79,39 +79,41 @@ __device__ __forceinline__ int order_key(const VolJob& J, int pix, const uint32_
   return cost != nullptr ? cost_bucket(cost[pix]) : chord_key(J, pix);
 }
 
-__global__ void order_count_kernel(const __grid_constant__ VolJob J, int npix, uint32_t* counts,
-                                   const uint32_t* cost) {
+__global__ void order_count_kernel(const __grid_constant__ OrderJob A, const __grid_constant__ OrderJob B) {
+  const OrderJob& O = blockIdx.y == 0 ? A : B;
   __shared__ uint32_t hist[kOrderBuckets];
   for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x) hist[k] = 0;
   __syncthreads();
   const int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix < npix) atomicAdd(&hist[order_key(J, pix, cost)], 1u);
+  if (pix < O.npix) atomicAdd(&hist[order_key(O.J, pix, O.cost)], 1u);
   __syncthreads();
   for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x)
-    if (hist[k]) atomicAdd(counts + k, hist[k]);
+    if (hist[k]) atomicAdd(O.buckets + k, hist[k]);
 }
 
-__global__ void order_scan_kernel(uint32_t* counts) {
-  // exclusive prefix sum of the 256 bucket counts, in place (one block)
-  __shared__ uint32_t s[kOrderBuckets];
+// Every block derives the buckets' first slots from the counts itself (256
+// values; a launch of its own for the scan cost more than that).
+__global__ void __launch_bounds__(kOrderBuckets) order_place_kernel(const __grid_constant__ OrderJob A,
+                                                                    const __grid_constant__ OrderJob B) {
+  const OrderJob& O = blockIdx.y == 0 ? A : B;
+  if (int(blockIdx.x * blockDim.x) >= O.npix) return;  // the other job's film is larger
+  __shared__ uint32_t first[kOrderBuckets], warp_sum[kOrderBuckets / 32];
   const int t = threadIdx.x;
-  s[t] = counts[t];
-  __syncthreads();
-  for (int off = 1; off < kOrderBuckets; off <<= 1) {
-    const uint32_t v = t >= off ? s[t - off] : 0u;
-    __syncthreads();
-    s[t] += v;
-    __syncthreads();
+  const uint32_t n = __ldcg(O.buckets + t);
+  uint32_t sum = n;  // inclusive in the warp
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, sum, off);
+    if ((t & 31) >= off) sum += v;
   }
-  counts[t] = t == 0 ? 0u : s[t - 1];
-}
-
-__global__ void order_place_kernel(const __grid_constant__ VolJob J, int npix, uint32_t* starts,
-                                   uint32_t* order, uint32_t* cost) {
-  const int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = pix < npix;
-  place_block(valid ? order_key(J, pix, cost) : 0, valid, (uint32_t)pix, starts, order);
-  if (valid && cost != nullptr) cost[pix] = 0u;  // the next tracer call accumulates afresh
+  if ((t & 31) == 31) warp_sum[t >> 5] = sum;
+  __syncthreads();
+  for (int w = 0; w < (t >> 5); ++w) sum += warp_sum[w];
+  first[t] = sum - n;
+  __syncthreads();
+  const int pix = blockIdx.x * blockDim.x + t;
+  const bool valid = pix < O.npix;
+  place_block(valid ? order_key(O.J, pix, O.cost) : 0, valid, (uint32_t)pix, O.buckets + kOrderBuckets, O.order, first);
+  if (valid && O.cost != nullptr) O.cost[pix] = 0u;  // the next tracer call accumulates afresh
 }
 
 // Sum of a pixel's samples in sample order, divided by spp (the box-filter
@@ -339,18 +341,14 @@ void warm_launch_config() {
 static_assert(kOrderBuckets == kRenderOrderBuckets, "order bucket count mismatch");
 static_assert(int64_t(kTapeChunk) == kTapeChunkSlots, "tape chunk mismatch");
 
-// Fills `order` with the job's pixels, longest expected path first.
-int order_pixels(const VolJob& J, uint32_t* buckets, uint32_t* order, uint32_t* cost, cudaStream_t st) {
-  const int npix = J.width * J.height;
-  RCV_TRY_CUDA(cudaMemsetAsync(buckets, 0, kOrderBuckets * sizeof(uint32_t), st), "order reset");
-  const int block = 256;
-  order_count_kernel<<<grid_for(npix, block), block, 0, st>>>(J, npix, buckets, cost);
+int order_pixels(const OrderJob* jobs, int n, cudaStream_t st) {
+  const OrderJob& A = jobs[0];
+  const OrderJob& B = jobs[n - 1];
+  const dim3 grid(grid_for(A.npix > B.npix ? A.npix : B.npix, kOrderBuckets), (unsigned)n);
+  order_count_kernel<<<grid, kOrderBuckets, 0, st>>>(A, B);
   int rc = launched("order_count launch");
   if (rc) return rc;
-  order_scan_kernel<<<1, kOrderBuckets, 0, st>>>(buckets);
-  rc = launched("order_scan launch");
-  if (rc) return rc;
-  order_place_kernel<<<grid_for(npix, block), block, 0, st>>>(J, npix, buckets, order, cost);
+  order_place_kernel<<<grid, kOrderBuckets, 0, st>>>(A, B);
   return launched("order_place launch");
 }
 
@@ -358,7 +356,7 @@ int order_pixels(const VolJob& J, uint32_t* buckets, uint32_t* order, uint32_t* 
 // null) or of a device job table; zeroes its hand-out counter on `st`.
 int make_queue(int mode, const VolJob* jobs, int njobs, int64_t total, const rcv_volpath_options* o,
                unsigned long long* queue_counter, float4* path_out, const AdjBuffers* adj, uint64_t* counters,
-               cudaStream_t st, Queue* out) {
+               cudaStream_t st, Queue* out, bool zeroed) {
   Queue& Q = *out;
   std::memset(&Q, 0, sizeof(Q));
   Q.counter = queue_counter;
@@ -394,7 +392,7 @@ int make_queue(int mode, const VolJob* jobs, int njobs, int64_t total, const rcv
   RCV_REQUIRE(Q.batch <= (1 << 20), "batch must be <= 2^20");
   Q.defer = (o != nullptr && o->defer > 0) ? o->defer : 8;
   RCV_REQUIRE(Q.defer <= 32, "defer must be in [1, 32]");
-  RCV_TRY_CUDA(cudaMemsetAsync(Q.counter, 0, sizeof(unsigned long long), st), "queue reset");
+  if (!zeroed) RCV_TRY_CUDA(cudaMemsetAsync(Q.counter, 0, sizeof(unsigned long long), st), "queue reset");
   return RCV_OK;
 }
 
@@ -403,9 +401,9 @@ int make_queue(int mode, const VolJob* jobs, int njobs, int64_t total, const rcv
 int launch_persistent(int mode, const VolJob& J, const VolJob* jobs, int njobs, int64_t total,
                       const rcv_volpath_options* o, unsigned long long* queue_counter,
                       float4* path_out, const AdjBuffers* adj, uint64_t* counters, cudaStream_t st,
-                      bool supergrid) {
+                      bool supergrid, bool zeroed) {
   Queue Q;
-  int rc = make_queue(mode, jobs, njobs, total, o, queue_counter, path_out, adj, counters, st, &Q);
+  int rc = make_queue(mode, jobs, njobs, total, o, queue_counter, path_out, adj, counters, st, &Q, zeroed);
   if (rc) return rc;
   const bool sg = supergrid || (jobs == nullptr && J.sg[0] > 0);
   // an environment map belongs to a single job (batched tables take the constant environment)
@@ -597,21 +595,27 @@ static int check_workspace(const void* workspace) {
   return RCV_OK;
 }
 
-// Pixel hand-out order of a job (RCV_ORDER_*), in its workspace; `sort`
-// false reuses the order an earlier stage left there.
-static int order_job(VolJob& J, const rcv_volpath_options* o, char* ws, const RenderLayout& L, bool sort,
-                     cudaStream_t st) {
+// Head of a job's workspace cleared (queue counters, order buckets) and its
+// pixel hand-out order (RCV_ORDER_*) chosen; jobs that sort their pixels are
+// added to `sort` for order_pixels.  `keep`: the order and the counters are
+// those that an earlier stage left there.
+static int order_job(VolJob& J, const rcv_volpath_options* o, char* ws, const RenderLayout& L, bool keep,
+                     OrderJob* sort, int* nsort, cudaStream_t st) {
   J.pixel_order = nullptr;
   J.pixel_cost = nullptr;
   const int order = o == nullptr ? RCV_ORDER_COST : o->order;
   RCV_REQUIRE(order == RCV_ORDER_COST || order == RCV_ORDER_ROW_MAJOR || order == RCV_ORDER_LONGEST_FIRST,
               "unknown pixel order %d", order);
+  if (!keep) RCV_TRY_CUDA(cudaMemsetAsync(ws, 0, kRenderHeadBytes, st), "counters reset");
   if (order == RCV_ORDER_ROW_MAJOR) return RCV_OK;
   uint32_t* cost = order == RCV_ORDER_COST ? reinterpret_cast<uint32_t*>(ws + L.cost) : nullptr;
-  if (sort) {
-    const int rc = order_pixels(J, reinterpret_cast<uint32_t*>(ws + L.buckets),
-                                reinterpret_cast<uint32_t*>(ws + L.order), cost, st);
-    if (rc) return rc;
+  if (!keep) {
+    OrderJob& O = sort[(*nsort)++];
+    O.J = J;
+    O.npix = J.width * J.height;
+    O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
+    O.order = reinterpret_cast<uint32_t*>(ws + L.order);
+    O.cost = cost;
   }
   J.pixel_order = reinterpret_cast<const uint32_t*>(ws + L.order);
   J.pixel_cost = cost;
@@ -658,7 +662,10 @@ static int run_single_job(int mode, VolJob& J, const rcv_volpath_options* o, voi
   const int64_t npix = int64_t(J.width) * J.height;
   const RenderLayout L = render_layout(npix, J.path_count, mode);
   char* ws = static_cast<char*>(workspace);
-  rc = order_job(J, o, ws, L, stage != kAdjReplay, st);
+  OrderJob sort[1];
+  int nsort = 0;
+  rc = order_job(J, o, ws, L, stage == kAdjReplay, sort, &nsort, st);
+  if (rc == RCV_OK && nsort > 0) rc = order_pixels(sort, nsort, st);
   if (rc) return rc;
   float4* po = reinterpret_cast<float4*>(ws + L.path_out);
   unsigned long long* qc = reinterpret_cast<unsigned long long*>(ws + L.counter);
@@ -668,23 +675,22 @@ static int run_single_job(int mode, VolJob& J, const rcv_volpath_options* o, voi
     rc = adjoint_buffers(J, o, ws, L, qc, stage, &A, &tape);
     if (rc) return rc;
     if (stage != kAdjReplay) {
-      RCV_TRY_CUDA(cudaMemsetAsync(A.ckpt_count, 0, 3 * sizeof(unsigned long long), st), "adjoint counters reset");
       rc = launch_persistent(tape ? kTape : kAdjoint, J, nullptr, 0, J.path_count, o, qc, nullptr, &A, counters,
-                             st, false);
+                             st, false, true);
       if (rc || stage == kAdjRadiance) return rc;
     }
     if (tape) {
       // weights of the event records: the second half of the checkpoint buffer
       float4* weights = reinterpret_cast<float4*>(ws + L.ckpt + uint64_t(A.ckpt_cap) * 32u);
       rc = launch_tape_gradient(J, nullptr, 0, A, weights, reinterpret_cast<float2*>(ws + L.cam_w), J.path_count,
-                                counters, sm_count(), st);
+                                qc + 4, counters, sm_count(), st);
       if (rc) return rc;
       // the paths whose events did not fit, replayed whole
     }
-    return launch_persistent(stage == kAdjForward ? kForward : kReplay, J, nullptr, 0, J.path_count, o, qc,
-                             nullptr, &A, counters, st, false);
+    return launch_persistent(stage == kAdjForward ? kForward : kReplay, J, nullptr, 0, J.path_count, o, qc + 4,
+                             nullptr, &A, counters, st, false, tape);
   }
-  rc = launch_persistent(mode, J, nullptr, 0, J.path_count, o, qc, po, nullptr, counters, st, false);
+  rc = launch_persistent(mode, J, nullptr, 0, J.path_count, o, qc, po, nullptr, counters, st, false, true);
   if (rc) return rc;
   return launch_reduce(mode == kTwoState, po, 0, npix, J.spp, img_new, img_old, st);
 }
@@ -749,14 +755,16 @@ extern "C" int rcv_render_twostates_volume_and_adjoint_radiance(
     if (rc) return rc;
     return run_single_job(kAdjoint, JB, o, adjoint_workspace, counters, nullptr, nullptr, st, kAdjRadiance);
   }
-  rc = order_job(JA, o, wa, LA, true, st);
-  if (rc == RCV_OK) rc = order_job(JB, o, wb, LB, true, st);
+  OrderJob sort[2];
+  int nsort = 0;
+  rc = order_job(JA, o, wa, LA, false, sort, &nsort, st);
+  if (rc == RCV_OK) rc = order_job(JB, o, wb, LB, false, sort, &nsort, st);
+  if (rc == RCV_OK && nsort > 0) rc = order_pixels(sort, nsort, st);
   if (rc) return rc;
-  RCV_TRY_CUDA(cudaMemsetAsync(A.ckpt_count, 0, 3 * sizeof(unsigned long long), st), "adjoint counters reset");
   float4* po = reinterpret_cast<float4*>(wa + LA.path_out);
   Queue QA, QB;
-  rc = make_queue(kTwoState, nullptr, 0, JA.path_count, o, qa, po, nullptr, nullptr, st, &QA);
-  if (rc == RCV_OK) rc = make_queue(kTape, nullptr, 0, JB.path_count, o, qb, nullptr, &A, nullptr, st, &QB);
+  rc = make_queue(kTwoState, nullptr, 0, JA.path_count, o, qa, po, nullptr, nullptr, st, &QA, true);
+  if (rc == RCV_OK) rc = make_queue(kTape, nullptr, 0, JB.path_count, o, qb, nullptr, &A, nullptr, st, &QB, true);
   if (rc == RCV_OK) rc = launch_pair(JA, QA, JB, QB, o, st, false);
   if (rc) return rc;
   return launch_reduce(true, po, 0, npix, JA.spp, img_new, img_old, st);

@@ -510,11 +510,19 @@ __device__ __forceinline__ bool roulette(const VolJob& J, Pcg32& rng, int depth,
 // Validates a medium + sensor + options and fills a job for one launch.
 int make_volume_job(const rcv_medium* m, const rcv_sensor* s, const rcv_volpath_options* o, uint32_t seed,
                     int spp, VolJob* J);
-// Writes the job's pixels into `order`, most expensive first: by `cost` (the
-// per-pixel path lengths of the previous call, cleared here) or, when cost is
-// null, by the chord length of the pixel's centre ray through the medium
-// (buckets: 256 uint32 of scratch).
-int order_pixels(const VolJob& J, uint32_t* buckets, uint32_t* order, uint32_t* cost, cudaStream_t st);
+// Pixel hand-out of one job: `order` receives its pixels, most expensive
+// first, by `cost` (the per-pixel path lengths of the previous call, cleared
+// here) or, when cost is null, by the chord length of the pixel's centre ray
+// through the medium.  buckets: 2 x 256 zeroed uint32 of scratch.
+struct OrderJob {
+  VolJob J;
+  int32_t npix;
+  uint32_t* buckets;
+  uint32_t* order;
+  uint32_t* cost;
+};
+// Orders the pixels of one job or of two, in the same two launches.
+int order_pixels(const OrderJob* jobs, int n, cudaStream_t st);
 // Clears the medium workspace's cell (and albedo) gradient accumulators.
 int reset_gradients(const rcv_medium* m, bool albedo, cudaStream_t st);
 // Adds the folded voxel gradients of the medium workspace to grad_density
@@ -536,15 +544,18 @@ __device__ __forceinline__ int chord_key(const VolJob& J, int pix) {
 // Places the pixels of one block in their buckets: block-local ranks from a
 // shared histogram, one global reservation per (block, bucket), so a popular
 // bucket costs one global atomic per block instead of one per pixel.  Order
-// within a bucket is arbitrary (it never changes results).
+// within a bucket is arbitrary (it never changes results).  `starts` holds
+// each bucket's next slot; with `first` (shared, 256) a bucket's slots begin
+// there and `starts` counts those handed out.
 __device__ __forceinline__ void place_block(int key, bool valid, uint32_t pix, uint32_t* starts,
-                                            uint32_t* order) {
+                                            uint32_t* order, const uint32_t* first = nullptr) {
   __shared__ uint32_t cnt[256], base[256];
   for (int k = threadIdx.x; k < 256; k += blockDim.x) cnt[k] = 0u;
   __syncthreads();
   const uint32_t rank = valid ? atomicAdd(&cnt[key], 1u) : 0u;
   __syncthreads();
-  for (int k = threadIdx.x; k < 256; k += blockDim.x) base[k] = cnt[k] ? atomicAdd(starts + k, cnt[k]) : 0u;
+  for (int k = threadIdx.x; k < 256; k += blockDim.x) 
+    base[k] = cnt[k] ? (first != nullptr ? first[k] : 0u) + atomicAdd(starts + k, cnt[k]) : 0u;
   __syncthreads();
   if (valid) order[base[key] + rank] = pix;
 }
@@ -561,12 +572,14 @@ __device__ __forceinline__ int cost_bucket(uint32_t c) {
 // variant that can traverse one is launched; single jobs decide from J.sg).
 int launch_persistent(int mode, const VolJob& J, const VolJob* jobs, int njobs, int64_t total,
                       const rcv_volpath_options* o, unsigned long long* queue_counter, float4* path_out,
-                      const AdjBuffers* adj, uint64_t* counters, cudaStream_t st, bool supergrid);
+                      const AdjBuffers* adj, uint64_t* counters, cudaStream_t st, bool supergrid,
+                      bool zeroed = false);
 // Work queue of a persistent tracer launch (the arguments of
-// launch_persistent); zeroes its hand-out counter on `st`.
+// launch_persistent); zeroes its hand-out counter on `st` unless that is
+// known to be zero.
 int make_queue(int mode, const VolJob* jobs, int njobs, int64_t total, const rcv_volpath_options* o,
                unsigned long long* queue_counter, float4* path_out, const AdjBuffers* adj, uint64_t* counters,
-               cudaStream_t st, Queue* out);
+               cudaStream_t st, Queue* out, bool zeroed = false);
 // One persistent launch of two tracers (rcv_pair.cu): the two-state primal
 // over QA and the tape radiance pass over QB, each of a single job (JA, JB:
 // the same medium and environment) or both of job tables (supergrid: some
@@ -584,9 +597,11 @@ inline float* tape_terms(char* region, int64_t room) { return reinterpret_cast<f
 // Gradient from a kTape radiance pass (rcv_tape.cu) of one job (jobs ==
 // NULL) or of a device job table: the per-record and per-path weights
 // (`weights`: 2 float4 per record, `cam_w`: one float2 per path) and the
-// scatter of every tape event into its job's gradient records.
+// scatter of every tape event into its job's gradient records.  Zeroes
+// *replay_counter, the hand-out counter of the replay that follows.
 int launch_tape_gradient(const VolJob& single, const VolJob* jobs, int njobs, const AdjBuffers& A, float4* weights,
-                         float2* cam_w, int64_t paths, uint64_t* counters, int sms, cudaStream_t st);
+                         float2* cam_w, int64_t paths, unsigned long long* replay_counter, uint64_t* counters,
+                         int sms, cudaStream_t st);
 int tracer_sm_count();
 
 }  // namespace rcv

@@ -526,7 +526,7 @@ static VpsLayout vps_layout(int64_t npix, int64_t paths) {
   const uint64_t n = (uint64_t)paths;
   L.counters = 0;
   L.buckets = 256;
-  L.order = align256(L.buckets + kRenderOrderBuckets * sizeof(uint32_t));
+  L.order = align256(kRenderHeadBytes);
   L.ltot = align256(L.order + uint64_t(npix) * sizeof(uint32_t));
   L.rec = align256(L.ltot + n * 16u);
   L.wn = align256(L.rec + n * kVpsRecsPerPath * 64u);
@@ -630,10 +630,16 @@ static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, cha
   if (o->order != RCV_ORDER_ROW_MAJOR) {
     // longest chord through the medium first: the path lengths of an earlier
     // call would order a little better but would tie the scratch to the caller
-    uint32_t* order = reinterpret_cast<uint32_t*>(ws + L.order);
-    rc = order_pixels(J, reinterpret_cast<uint32_t*>(ws + L.buckets), order, nullptr, st);
+    OrderJob O;
+    O.J = J;
+    O.npix = (int32_t)npix;
+    O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
+    O.order = reinterpret_cast<uint32_t*>(ws + L.order);
+    O.cost = nullptr;
+    RCV_TRY_CUDA(cudaMemsetAsync(ws, 0, kRenderHeadBytes, st), "counters reset");
+    rc = order_pixels(&O, 1, st);
     if (rc) return rc;
-    J.pixel_order = order;
+    J.pixel_order = O.order;
   }
   P.draws = P.use_drt ? 5 : 4;
   P.task = reinterpret_cast<float4*>(ws + L.task);
@@ -660,7 +666,8 @@ static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, cha
   for (int64_t base = 0; base < J.path_count; base += chunk) {
     const int64_t n = J.path_count - base < chunk ? J.path_count - base : chunk;
     J.path_begin = -base;  // path p of the pass is path base + p of the film
-    RCV_TRY_CUDA(cudaMemsetAsync(qc, 0, 8 * sizeof(unsigned long long), st), "counters reset");
+    if (base > 0 || J.pixel_order == nullptr)
+      RCV_TRY_CUDA(cudaMemsetAsync(qc, 0, 8 * sizeof(unsigned long long), st), "counters reset");
     for (int mode = kVpsTape; mode <= (P.use_drt ? kVpsDrt : kVpsTape); ++mode) {
       Q.counter = qc + mode;
       Q.total = n;
