@@ -332,6 +332,11 @@ static int sm_count() {
 
 int tracer_sm_count() { return sm_count(); }
 
+int paths_per_fetch(int64_t total) {
+  const int64_t share = total / (int64_t(sm_count()) * 24 * 8);
+  return (int)(share < 2 ? 2 : (share > 64 ? 64 : share));
+}
+
 void warm_launch_config() {
   (void)resident_blocks(0);
   (void)sm_count();
@@ -388,7 +393,7 @@ int make_queue(int mode, const VolJob* jobs, int njobs, int64_t total, const rcv
   Q.jobs = jobs;
   Q.njobs = njobs;
   Q.total = total;
-  Q.batch = (o != nullptr && o->batch > 0) ? o->batch : 64;
+  Q.batch = (o != nullptr && o->batch > 0) ? o->batch : paths_per_fetch(total);
   RCV_REQUIRE(Q.batch <= (1 << 20), "batch must be <= 2^20");
   Q.defer = (o != nullptr && o->defer > 0) ? o->defer : 8;
   RCV_REQUIRE(Q.defer <= 32, "defer must be in [1, 32]");

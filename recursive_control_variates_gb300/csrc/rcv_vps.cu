@@ -672,9 +672,7 @@ static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, cha
       Q.counter = qc + mode;
       Q.total = n;
       const int64_t cap = int64_t(sms) * vps_resident(mode, variant);
-      // paths per fetch: 64, or fewer so that a small film reaches every warp
-      int64_t batch = n / (cap * kVpsWarps * 2);
-      batch = batch < 1 ? 1 : (batch > 64 ? 64 : batch);
+      const int64_t batch = paths_per_fetch(n);
       Q.batch = (int32_t)batch;
       int64_t blocks = (n + batch * kVpsWarps - 1) / (batch * kVpsWarps);
       if (blocks > cap) blocks = cap;
