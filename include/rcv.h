@@ -229,7 +229,7 @@ int rcv_medium_prepare(const rcv_medium* medium, void* stream);
  * cost and, for the primal tracers, one radiance slot per path; for the
  * adjoint 476 B per path: total radiance, 2 scatter checkpoints or event
  * records with their weights, 16 tape slots of 16 B each with a 4-B
- * extinction term, camera-segment weight, lost-path list): 256-B aligned device memory of this size, passed as
+ * extinction term, camera-segment weight, entered- and lost-path lists): 256-B aligned device memory of this size, passed as
  * `workspace`.  The per-pixel cost persists from call to call
  * (RCV_ORDER_COST); pass the same workspace to the calls of one image size.
  * mode = RCV_MODE_*. */

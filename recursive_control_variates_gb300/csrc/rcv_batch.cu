@@ -248,7 +248,7 @@ __global__ void batch_supergrid_kernel(const BatchEntry* __restrict__ E, const V
   const int j = job_of_block(bp, n, blockIdx.x);
   const BatchEntry& B = E[j];
   const VolJob& J = two[j];
-  const int64_t i = int64_t(blockIdx.x - __ldg(bp + j)) * blockDim.x + threadIdx.x;
+  const int64_t i = (int64_t(blockIdx.x - __ldg(bp + j)) * blockDim.x + threadIdx.x) >> 5;  // one warp per cell
   if (J.sg[0] == 0 || i >= int64_t(J.sg[0]) * J.sg[1] * J.sg[2]) return;
   const int cur = B.hdr->step.cur;
   supergrid_cell(i, J.sg, B.d.dims[0], B.d.dims[1], B.d.dims[2], B.d.scale, B.d.density[cur ^ 1],
@@ -267,10 +267,11 @@ __global__ void batch_image_kernel(const BatchEntry* __restrict__ E, const int32
   const BatchEntry& B = E[j];
   const int64_t pix = int64_t(blockIdx.x - __ldg(bp + j)) * blockDim.x + threadIdx.x;
   double acc = 0.0;
+  __shared__ float4 tile[kReduceTile];
+  V3 F, H;
+  reduce_pixel<true>(path_out, B.two_begin, pix, B.npix, B.d.spp, tile, F, H);
   if (pix < B.npix) {
     const CvScalars S = B.hdr->step.S;
-    V3 F, H;
-    reduce_pixel<true>(path_out, B.two_begin, pix, B.d.spp, F, H);
     if (B.d.img_new != nullptr) {
       B.d.img_new[pix * 3 + 0] = F.x;
       B.d.img_new[pix * 3 + 1] = F.y;
@@ -382,17 +383,20 @@ static int validate_job(const rcv_batch_job* j, int idx) {
 
 // Plan workspace: entries | two-state jobs | adjoint jobs | block prefixes |
 // queue counters (two-state, adjoint radiance, replay, checkpoints / event
-// records, tape slots, lost paths) | tracer counters | per-path radiance |
+// records, tape slots, lost paths, entered paths) | tracer counters | per-path radiance |
 // adjoint per-path total radiance | scatter checkpoints (tape: event records
-// and their weights) | event tape | per-path camera-segment weights |
-// lost-path list.
+// and their weights) | event tape | camera-segment weights and paths
+// of those that entered the medium | lost-path list.
 struct PlanLayout {
-  uint64_t entries, two, adj, prefix, queue, counters, path_out, ltot, ckpt, tape, cam_w, lost, total;
+  uint64_t entries, two, adj, prefix, queue, counters, path_out, ltot, ckpt, tape, cam_w, entered, lost, total;
 };
 
 // A plan's scratch grows with its paths alone (the serving budget adds its
-// jobs' shares up): 2 checkpoints and kTapeSlotsPerPath tape slots per path.
-static int64_t batch_ckpt_capacity(int64_t paths) { return kTapeSlotsPerPath / 8 * paths + kCkptMargin; }
+// jobs' shares up): 2 checkpoints of 64 bytes per path, less the 4 bytes of the
+// entered paths' list, and kTapeSlotsPerPath tape slots.
+static int64_t batch_ckpt_capacity(int64_t paths) {
+  return kTapeSlotsPerPath / 8 * paths - paths / 16 + kCkptMargin;
+}
 
 static PlanLayout plan_layout(int n, int64_t total_two_paths, int64_t total_adj_paths) {
   PlanLayout L;
@@ -419,6 +423,8 @@ static PlanLayout plan_layout(int n, int64_t total_two_paths, int64_t total_adj_
   off = align256(off + uint64_t(tape_capacity(total_adj_paths, kTapeSlotsPerPath)) * 20u);
   L.cam_w = off;
   off = align256(off + uint64_t(total_adj_paths) * 8u);
+  L.entered = off;
+  off = align256(off + uint64_t(total_adj_paths) * 4u);
   L.lost = off;
   off = align256(off + uint64_t(total_adj_paths) * 4u);
   L.total = off;
@@ -476,7 +482,6 @@ struct rcv_batch {
   // two launches on two streams
   bool paired = false;
   float4* tape_weights = nullptr;
-  float2* cam_w = nullptr;
   int64_t total_two = 0, total_adj = 0;
   int32_t pack_blocks = 0, pix_blocks = 0, vox_blocks = 0, sg_blocks = 0;
   // host copies of the tables (kept until destroy: the upload reads them)
@@ -642,7 +647,7 @@ extern "C" int rcv_batch_create(const rcv_batch_job* jobs, int32_t n, const rcv_
     pack_blocks += grid_for(e.nc, kBatchBlock);
     pix_blocks += grid_for(e.npix, kBatchBlock);
     vox_blocks += grid_for(e.nv, kBatchBlock);
-    if (T.sg[0] > 0) sg_blocks += grid_for(int64_t(T.sg[0]) * T.sg[1] * T.sg[2], kBatchBlock);
+    if (T.sg[0] > 0) sg_blocks += grid_for(int64_t(T.sg[0]) * T.sg[1] * T.sg[2] * 32, kBatchBlock);
     two_total += T.path_count;
     adj_total += A.path_count;
     if (pack_blocks >= INT32_MAX || pix_blocks >= INT32_MAX || vox_blocks >= INT32_MAX) {
@@ -688,7 +693,9 @@ extern "C" int rcv_batch_create(const rcv_batch_job* jobs, int32_t n, const rcv_
     b->adjbuf.lost_count = b->queue + 5;
     b->adjbuf.tape_f = tape_terms(w + P.tape, tape_capacity(adj_total, kTapeSlotsPerPath));
     b->tape_weights = reinterpret_cast<float4*>(w + P.ckpt + uint64_t(b->adjbuf.ckpt_cap) * 32u);
-    b->cam_w = reinterpret_cast<float2*>(w + P.cam_w);
+    b->adjbuf.cam_w = reinterpret_cast<float2*>(w + P.cam_w);
+    b->adjbuf.entered = reinterpret_cast<uint32_t*>(w + P.entered);
+    b->adjbuf.entered_count = b->queue + 6;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemcpyAsync(b->entries, b->h_entries.data(), sizeof(BatchEntry) * n, cudaMemcpyHostToDevice, st);
@@ -752,7 +759,7 @@ static int enqueue_step(rcv_batch* b, cudaStream_t st) {
   if (b->paired) {
     // the adjoint radiance pass needs no image gradient: it runs in the
     // launch of the two-state pass
-    RCV_TRY_CUDA(cudaMemsetAsync(b->adjbuf.ckpt_count, 0, 3 * sizeof(unsigned long long), st),
+    RCV_TRY_CUDA(cudaMemsetAsync(b->adjbuf.ckpt_count, 0, 4 * sizeof(unsigned long long), st),
                  "adjoint counters reset");
     Queue QA, QB;
     rc = make_queue(kTwoState, b->two, n, b->total_two, &b->opt, b->queue + 0, b->path_out, nullptr, nullptr, st,
@@ -768,8 +775,8 @@ static int enqueue_step(rcv_batch* b, cudaStream_t st) {
     // ... or on the side stream beside the two-state pass and the image kernel
     RCV_TRY_CUDA(cudaEventRecord(b->fork, st), "fork record");
     RCV_TRY_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0), "fork wait");
-    // checkpoint / event-record, tape-slot and lost-path counters
-    RCV_TRY_CUDA(cudaMemsetAsync(b->adjbuf.ckpt_count, 0, 3 * sizeof(unsigned long long), b->side),
+    // checkpoint / event-record, tape-slot, lost-path and entered-path counters
+    RCV_TRY_CUDA(cudaMemsetAsync(b->adjbuf.ckpt_count, 0, 4 * sizeof(unsigned long long), b->side),
                  "adjoint counters reset");
     rc = launch_persistent(b->tape ? kTape : kAdjoint, none, b->adj, n, b->total_adj, &b->opt, b->queue + 1,
                            nullptr, &b->adjbuf, cnt ? cnt + RCV_COUNTER_COUNT : nullptr, b->side, sg);
@@ -785,8 +792,8 @@ static int enqueue_step(rcv_batch* b, cudaStream_t st) {
   }
   if (b->tape) {
     // the gradient from the tape; the replay then takes only the lost paths
-    rc = launch_tape_gradient(none, b->adj, n, b->adjbuf, b->tape_weights, b->cam_w, b->total_adj,
-                              b->queue + 2, cnt ? cnt + RCV_COUNTER_COUNT : nullptr, tracer_sm_count(), st);
+    rc = launch_tape_gradient(none, b->adj, n, b->adjbuf, b->tape_weights, b->queue + 2,
+                              cnt ? cnt + RCV_COUNTER_COUNT : nullptr, tracer_sm_count(), st);
     if (rc) return rc;
   }
   rc = launch_persistent(kReplay, none, b->adj, n, b->total_adj, &b->opt, b->queue + 2, nullptr, &b->adjbuf,

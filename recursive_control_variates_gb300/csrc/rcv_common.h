@@ -119,14 +119,15 @@ inline MediumLayout medium_layout(const rcv_medium* m) {
 // queue) | order bucket counts | slots handed out per bucket | pixel order | per-pixel cost | per-path radiance (32 B
 // per path for two-state, 16 B single-state) | adjoint: per-path total
 // radiance | scatter checkpoints (tape: event records, then their weights) |
-// event tape | per-path camera-segment weight | lost-path list.
+// event tape | camera-segment weight and path of those that entered the
+// medium | lost-path list.
 constexpr int kRenderOrderBuckets = 256;
 // counters, bucket counts and hand-outs: one clear of the workspace's head
 // before a call (offset 0)
 constexpr uint64_t kRenderHeadBytes = 256 + 2 * kRenderOrderBuckets * sizeof(uint32_t);
 
 struct RenderLayout {
-  uint64_t counter, buckets, order, cost, path_out, ltot, ckpt, tape, cam_w, lost, total;
+  uint64_t counter, buckets, order, cost, path_out, ltot, ckpt, tape, cam_w, entered, lost, total;
 };
 
 // Event tape of the adjoint: 16 bytes per event (whole chunks of
@@ -180,7 +181,8 @@ inline RenderLayout render_layout(int64_t npix, int64_t paths, int mode) {
   L.ckpt = align256(L.ltot + (adj ? uint64_t(paths) * 16u : 0u));
   L.tape = align256(L.ckpt + (adj ? uint64_t(ckpt_capacity(paths)) * 64u : 0u));
   L.cam_w = align256(L.tape + (adj ? uint64_t(tape_room(paths)) * 20u : 0u));
-  L.lost = align256(L.cam_w + (adj ? uint64_t(paths) * 8u : 0u));
+  L.entered = align256(L.cam_w + (adj ? uint64_t(paths) * 8u : 0u));
+  L.lost = align256(L.entered + (adj ? uint64_t(paths) * 4u : 0u));
   L.total = align256(L.lost + (adj ? uint64_t(paths) * 4u : 0u));
   return L;
 }

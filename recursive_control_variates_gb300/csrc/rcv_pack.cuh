@@ -44,6 +44,10 @@ __device__ __forceinline__ void supergrid_span(int c, int S, int D, int& lo, int
 
 // Majorants of supergrid cell i (x fastest): scale * the largest old / new
 // density (non-negative part) over its voxel span; two = max of both states.
+// Called by a whole warp, 8 lanes along x and 4 rows at a time: a cell of
+// factor 8 spans up to 1000 voxels of each state, which one thread took one
+// after the other (128^3: 82 us, too few threads to hide the loads; a warp
+// per cell 24 us).
 __device__ __forceinline__ void supergrid_cell(int64_t i, const int sg[3], int dx, int dy, int dz, float scale,
                                                const float* __restrict__ old_d, const float* __restrict__ new_d,
                                                float* __restrict__ sg_two, float* __restrict__ sg_new) {
@@ -52,16 +56,22 @@ __device__ __forceinline__ void supergrid_cell(int64_t i, const int sg[3], int d
   supergrid_span(cx, sg[0], dx, x0, x1);
   supergrid_span(cy, sg[1], dy, y0, y1);
   supergrid_span(cz, sg[2], dz, z0, z1);
+  const int lane = threadIdx.x & 31;
   float mo = 0.0f, mn = 0.0f;
   for (int z = z0; z <= z1; ++z)
-    for (int y = y0; y <= y1; ++y)
-      for (int x = x0; x <= x1; ++x) {
+    for (int y = y0 + (lane >> 3); y <= y1; y += 4)
+      for (int x = x0 + (lane & 7); x <= x1; x += 8) {
         const int64_t v = (int64_t(z) * dy + y) * dx + x;
         mo = fmaxf(mo, old_d[v]);
         mn = fmaxf(mn, new_d[v]);
       }
-  sg_two[i] = scale * fmaxf(mo, mn);
-  sg_new[i] = scale * mn;
+  // non-negative floats order like their bits
+  mo = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mo)));
+  mn = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mn)));
+  if (lane == 0) {
+    sg_two[i] = scale * fmaxf(mo, mn);
+    sg_new[i] = scale * mn;
+  }
 }
 
 // Voxel i of the old and the new RGB albedo as one 32-byte pair.
@@ -73,23 +83,57 @@ __device__ __forceinline__ void pack_albedo(int64_t i, const float* __restrict__
 
 // Sum of a pixel's per-path radiance slots in sample order, divided by spp
 // (the box-filter film develop of plugins/twostatevolpath.py:80-89).  Slots
-// are [path][new, old] for two-state launches and [path] otherwise.
+// are [path][new, old] for two-state launches and [path] otherwise.  Called by
+// whole blocks of kReduceBlock threads, one pixel per thread (`pix` of
+// consecutive threads consecutive, none from npix on).  The slots of a warp's
+// 32 pixels are one stretch of memory; a thread that reads its own pixel's
+// slots touches another 128-byte line than its neighbours with every load
+// (3.4 TB/s).  So the warp loads 8 slots of each of its pixels at a time, 128
+// consecutive bytes per 8 lanes, into shared memory, where each thread adds up
+// its row (stride 9: no bank conflicts): 512^2 x
+// 16 spp of both states 41 -> 26 us (5.2 TB/s), 512^2 x 256 spp of one 305 -> 192
+// us (5.6 TB/s of 6.8).
+constexpr int kReduceBlock = 256;
+constexpr int kReduceChunk = 8;
+constexpr int kReduceTile = kReduceBlock * (kReduceChunk + 1);
+
 template <bool kTwo>
 __device__ __forceinline__ void reduce_pixel(const float4* __restrict__ path_out, int64_t path_begin, int64_t pix,
-                                             int spp, V3& out_new, V3& out_old) {
+                                             int64_t npix, int spp, float4* tile, V3& out_new, V3& out_old) {
   constexpr int K = kTwo ? 2 : 1;
-  const float4* src = path_out + (path_begin + pix * spp) * K;
   float nx = 0.0f, ny = 0.0f, nz = 0.0f, ox = 0.0f, oy = 0.0f, oz = 0.0f;
-  for (int s = 0; s < spp; ++s) {
-    const float4 a = __ldcs(src + s * K);
-    nx += a.x;
-    ny += a.y;
-    nz += a.z;
-    if (kTwo) {
-      const float4 b = __ldcs(src + s * K + 1);
-      ox += b.x;
-      oy += b.y;
-      oz += b.z;
+  const int64_t row = int64_t(spp) * K;  // slots of a pixel
+  const int lane = threadIdx.x & 31;
+  const int64_t pix0 = pix - lane;
+  const float4* src = path_out + path_begin * K + pix0 * row;
+  float4* rows = tile + (threadIdx.x & ~31u) * (kReduceChunk + 1);
+  const float4* mine = rows + lane * (kReduceChunk + 1);
+  const int here = npix - pix0 < 32 ? int(npix - pix0 < 0 ? 0 : npix - pix0) : 32;  // pixels of this warp
+  const int col = lane & (kReduceChunk - 1), first = lane / kReduceChunk;
+  for (int64_t s = 0; s < row; s += kReduceChunk) {
+    const int n = row - s < kReduceChunk ? int(row - s) : kReduceChunk;
+    float4 v[kReduceChunk];
+#pragma unroll
+    for (int r = 0; r < kReduceChunk; ++r) {
+      const int p = first + r * (32 / kReduceChunk);
+      v[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (col < n && p < here) v[r] = __ldcs(src + p * row + s + col);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kReduceChunk; ++r) rows[(first + r * (32 / kReduceChunk)) * (kReduceChunk + 1) + col] = v[r];
+    __syncwarp();
+    for (int k = 0; k < n; k += K) {
+      const float4 a = mine[k];
+      nx += a.x;
+      ny += a.y;
+      nz += a.z;
+      if (kTwo) {
+        const float4 b = mine[k + 1];
+        ox += b.x;
+        oy += b.y;
+        oz += b.z;
+      }
     }
   }
   const float fs = (float)spp;

@@ -9,8 +9,9 @@
 // launches, the same arithmetic as the replay event by event
 // (plugins/twostatevolpath.py:141-479 for the events; the adjoint
 // semantics of Mitsuba's prb_volpath):
-//   tape_weights_kernel  per event record and per path, dL . L_rem of every
-//                        kind of event that refers to it, once dL is known;
+//   tape_weights_kernel  per event record and per path that entered the
+//                        medium, dL . L_rem of every kind of event that
+//                        refers to it, once dL is known;
 //   tape_scatter_kernel  per tape slot: the event's extinction term that
 //                        the radiance pass kept beside it (and at
 //                        scattering events the albedo from the medium),
@@ -61,15 +62,21 @@ __device__ __forceinline__ V3 tape_dL(const VolJob& J, int pix) {
 // Record k (2 float4: [path, radiance gathered before the event's NEE
 // contribution] [NEE contribution]) -> weights [dL . L_rem after the NEE
 // contribution (the next segment), dL . c_nee (the shadow walk), dL . L_rem
-// (the event), job] [dL * L_rem per channel (the event's albedo)].  Path p ->
-// [dL . L (its camera segment), job].  Job -1: the path is replayed instead
-// and its events are skipped.
+// (the event), job] [dL * L_rem per channel (the event's albedo)].  Entered
+// path -> [dL . L (its camera segment), job].  Job -1: the path is
+// replayed instead and its events are skipped.  Bound by the gathers of
+// radiance and image gradient; taking every path of the film instead of those
+// that entered the medium (a fifth of them) was 51 instead of 28 us at
+// 512^2 x 16 spp.
 __global__ void tape_weights_kernel(const __grid_constant__ VolJob single, const VolJob* __restrict__ jobs,
                                     int njobs, const float4* __restrict__ rec,
                                     const unsigned long long* __restrict__ rec_count, int64_t rec_cap,
                                     float4* __restrict__ w, const float4* __restrict__ ltot,
-                                    float2* __restrict__ cam_w, int64_t paths, unsigned long long* replay_counter) {
+                                    const uint32_t* __restrict__ entered, float2* __restrict__ cam_w,
+                                    const unsigned long long* __restrict__ entered_count,
+                                    unsigned long long* replay_counter) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *replay_counter = 0ull;
+  const int64_t paths = (int64_t)*entered_count;
   const int64_t nrec = min((int64_t)*rec_count, rec_cap);
   const int64_t n = max(nrec, paths);
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
@@ -93,12 +100,13 @@ __global__ void tape_weights_kernel(const __grid_constant__ VolJob single, const
       }
     }
     if (i < paths) {
-      const float4 lt = ltot[i];
+      const uint32_t path = entered[i];
+      const float4 lt = ltot[path];
       float2 c = make_float2(0.0f, __int_as_float(-1));
       if (lt.w == 0.0f) {
-        const int j = tape_job(jobs, njobs, (uint32_t)i);
+        const int j = tape_job(jobs, njobs, path);
         const VolJob& J = jobs != nullptr ? jobs[j] : single;
-        const V3 g = tape_dL(J, tape_pixel(J, (uint32_t)i));
+        const V3 g = tape_dL(J, tape_pixel(J, path));
         c = make_float2((g.x * lt.x + g.y * lt.y) + g.z * lt.z, __int_as_float(j));
       }
       cam_w[i] = c;
@@ -168,26 +176,23 @@ __global__ void __launch_bounds__(256) tape_scatter_kernel(const __grid_constant
 }
 
 int launch_tape_gradient(const VolJob& single, const VolJob* jobs, int njobs, const AdjBuffers& A, float4* weights,
-                         float2* cam_w, int64_t paths, unsigned long long* replay_counter, uint64_t* counters,
-                         int sms, cudaStream_t st) {
+                         unsigned long long* replay_counter, uint64_t* counters, int sms, cudaStream_t st) {
   const int block = 256;
-  // grid-stride: the records' number is known on the device only, and their
-  // room is many times it
-  const unsigned need = grid_for(A.ckpt_cap > paths ? A.ckpt_cap : paths, block);
-  const unsigned most = (unsigned)(sms > 0 ? sms : 1) * 16u;
-  tape_weights_kernel<<<need < most ? need : most, block, 0, st>>>(
-      single, jobs, njobs, A.ckpt, A.ckpt_count, A.ckpt_cap, weights, A.path_ltot, cam_w, paths,
-      replay_counter);
+  // grid-stride: the numbers of records and paths are known on the device only
+  const unsigned need = grid_for(A.ckpt_cap, block), most = (unsigned)(sms > 0 ? sms : 1) * 16u;
+  tape_weights_kernel<<<need < most ? need : most, block, 0, st>>>(single, jobs, njobs, A.ckpt, A.ckpt_count,
+                                                                   A.ckpt_cap, weights, A.path_ltot, A.entered,
+                                                                   A.cam_w, A.entered_count, replay_counter);
   int rc = launched("tape_weights launch");
   if (rc) return rc;
   const unsigned grid = (unsigned)(sms > 0 ? sms : 1) * 8u;
   unsigned long long* c = reinterpret_cast<unsigned long long*>(counters);
   if (counters != nullptr)
     tape_scatter_kernel<true><<<grid, block, 0, st>>>(single, jobs, A.tape, A.tape_count, A.tape_cap, weights,
-                                                       cam_w, A.tape_f, c);
+                                                       A.cam_w, A.tape_f, c);
   else
     tape_scatter_kernel<false><<<grid, block, 0, st>>>(single, jobs, A.tape, A.tape_count, A.tape_cap, weights,
-                                                        cam_w, A.tape_f, c);
+                                                        A.cam_w, A.tape_f, c);
   return launched("tape_scatter launch");
 }
 

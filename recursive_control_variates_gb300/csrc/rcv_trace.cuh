@@ -349,8 +349,8 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
   float& trn = bn.x;
   float& tro = bo.x;
   bool ck_lost = false;  // a checkpoint (kTape: an event or event record) of this path did not fit
-  // kTape: reference of the path's next events (kind << 30 | path or event
-  // record), and the warp's tape chunk
+  // kTape: reference of the path's next events (kind << 30 | entered path or
+  // event record), and the warp's tape chunk
   uint32_t tref = 0;
   TapeCursor tc{0u, 0u};
   // replay: radiance the path gathers after its current point,
@@ -465,7 +465,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       if (kMode == kTwoState) put3(cLo, V3{0, 0, 0});
       depth = 0;
       if (kRad) ck_lost = false;
-      if (kMode == kTape) tref = (kEvCamera << 30) | (uint32_t)path;
+      if (kMode == kTape) tref = kTapeEmpty;  // until the path enters the medium
       if (kRep) {
         if (kMode == kForward) dL = V3{0.0f, 0.0f, 0.0f};
         const float4 lt = Q.path_ltot[path];
@@ -521,6 +521,11 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             float a;
             slab(x, inv_d, a, rem);
             phase = kMain;
+            if (kMode == kTape) {
+              const uint32_t k = (uint32_t)atomicAdd(Q.entered_count, 1ull);
+              __stcs(Q.entered + k, (uint32_t)path);
+              tref = (kEvCamera << 30) | k;
+            }
           }
         }
       }
@@ -600,8 +605,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             ev_scat = true;  // the event itself
             ev_sf = st_n;
           } else {
-            ck_lost = true;
-            tref = (kEvCamera << 30) | U(cPath);
+            ck_lost = true;  // its events are not recorded any more
           }
         }
         // isotropic phase sample (1D unused + 2D), plugins/twostatevolpath.py:275
@@ -944,7 +948,8 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
         __stcs(o, make_float4(F(cLn), F(cLn + 1), F(cLn + 2), 0.0f));
         if (kMode == kTwoState) __stcs(o + 1, make_float4(F(cLo), F(cLo + 1), F(cLo + 2), 0.0f));
       }
-      if (kRad)
+      // (no event refers to a path that did not enter the medium)
+      if (kRad && (kMode != kTape || tref != kTapeEmpty))
         __stcs(Q.path_ltot + U(cPath), make_float4(F(cLn), F(cLn + 1), F(cLn + 2), ck_lost ? 1.0f : 0.0f));
       if (kMode == kTape && ck_lost) Q.lost_list[atomicAdd(Q.lost_count, 1ull)] = U(cPath);
       if (kMode == kForward && (dL.x != 0.0f || dL.y != 0.0f || dL.z != 0.0f)) {

@@ -61,7 +61,7 @@ static TraceKernel trace_kernel_of(int variant) { return kTraceTables[variant / 
 __global__ void supergrid_kernel(int sx, int sy, int sz, int dx, int dy, int dz, float scale,
                                  const float* __restrict__ old_d, const float* __restrict__ new_d,
                                  float* __restrict__ sg_two, float* __restrict__ sg_new) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;  // one warp per cell
   if (i >= int64_t(sx) * sy * sz) return;
   const int sg[3] = {sx, sy, sz};
   supergrid_cell(i, sg, dx, dy, dz, scale, old_d, new_d, sg_two, sg_new);
@@ -119,13 +119,15 @@ __global__ void __launch_bounds__(kOrderBuckets) order_place_kernel(const __grid
 // Sum of a pixel's samples in sample order, divided by spp (the box-filter
 // film develop of plugins/twostatevolpath.py:80-89).
 template <bool kTwo>
-__global__ void reduce_paths_kernel(const float4* __restrict__ path_out, int64_t path_begin,
-                                    int64_t npix, int spp, float* __restrict__ out_new,
-                                    float* __restrict__ out_old) {
+__global__ void __launch_bounds__(kReduceBlock) reduce_paths_kernel(const float4* __restrict__ path_out,
+                                                                    int64_t path_begin, int64_t npix, int spp,
+                                                                    float* __restrict__ out_new,
+                                                                    float* __restrict__ out_old) {
+  __shared__ float4 tile[kReduceTile];
   const int64_t pix = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (pix >= npix) return;
   V3 n, o;
-  reduce_pixel<kTwo>(path_out, path_begin, pix, spp, n, o);
+  reduce_pixel<kTwo>(path_out, path_begin, pix, npix, spp, tile, n, o);
+  if (pix >= npix) return;
   out_new[pix * 3 + 0] = n.x;
   out_new[pix * 3 + 1] = n.y;
   out_new[pix * 3 + 2] = n.z;
@@ -379,9 +381,13 @@ int make_queue(int mode, const VolJob* jobs, int njobs, int64_t total, const rcv
       RCV_REQUIRE(total < (int64_t(1) << 30) && adj->ckpt_cap < (int64_t(1) << 30) &&
                       adj->tape_cap <= (int64_t(1) << 32) - int64_t(kTapeChunk),
                   "too many paths for the tape adjoint");
-      RCV_REQUIRE(adj->tape_f != nullptr, "the tape needs its extinction terms");
+      RCV_REQUIRE(adj->tape_f != nullptr && adj->entered != nullptr && adj->entered_count != nullptr &&
+                      adj->cam_w != nullptr,
+                  "the tape needs its extinction terms and the list of entered paths");
       Q.tape = adj->tape;
       Q.tape_f = adj->tape_f;
+      Q.entered = adj->entered;
+      Q.entered_count = adj->entered_count;
       Q.tape_count = adj->tape_count;
       Q.tape_cap = adj->tape_cap;
       Q.lost_list = adj->lost_list;
@@ -430,7 +436,7 @@ int launch_persistent(int mode, const VolJob& J, const VolJob* jobs, int njobs, 
 
 int launch_reduce(bool two, const float4* po, int64_t path_begin, int64_t npix, int spp,
                   float* out_new, float* out_old, cudaStream_t st) {
-  const int block = 256;
+  const int block = kReduceBlock;
   if (two)
     reduce_paths_kernel<true><<<grid_for(npix, block), block, 0, st>>>(po, path_begin, npix, spp,
                                                                      out_new, out_old);
@@ -583,7 +589,7 @@ extern "C" int rcv_medium_prepare(const rcv_medium* m, void* stream) {
   const int sx = supergrid_cells(m->dims[0], m->majorant_factor);
   const int sy = supergrid_cells(m->dims[1], m->majorant_factor);
   const int sz = supergrid_cells(m->dims[2], m->majorant_factor);
-  supergrid_kernel<<<grid_for(int64_t(sx) * sy * sz, 128), 128, 0, st>>>(
+  supergrid_kernel<<<grid_for(int64_t(sx) * sy * sz * 32, 128), 128, 0, st>>>(
       sx, sy, sz, m->dims[0], m->dims[1], m->dims[2], m->scale, m->density_old, m->density_new,
       reinterpret_cast<float*>(ws + L.sg_two), reinterpret_cast<float*>(ws + L.sg_new));
   return launched("supergrid launch");
@@ -652,6 +658,9 @@ static int adjoint_buffers(const VolJob& J, const rcv_volpath_options* o, char* 
     A.lost_list = reinterpret_cast<uint32_t*>(ws + L.lost);
     A.lost_count = qc + 3;
     A.tape_f = tape_terms(ws + L.tape, tape_room(J.path_count));
+    A.cam_w = reinterpret_cast<float2*>(ws + L.cam_w);
+    A.entered = reinterpret_cast<uint32_t*>(ws + L.entered);
+    A.entered_count = qc + 5;
   }
   *tape_out = tape;
   return RCV_OK;
@@ -687,8 +696,7 @@ static int run_single_job(int mode, VolJob& J, const rcv_volpath_options* o, voi
     if (tape) {
       // weights of the event records: the second half of the checkpoint buffer
       float4* weights = reinterpret_cast<float4*>(ws + L.ckpt + uint64_t(A.ckpt_cap) * 32u);
-      rc = launch_tape_gradient(J, nullptr, 0, A, weights, reinterpret_cast<float2*>(ws + L.cam_w), J.path_count,
-                                qc + 4, counters, sm_count(), st);
+      rc = launch_tape_gradient(J, nullptr, 0, A, weights, qc + 4, counters, sm_count(), st);
       if (rc) return rc;
       // the paths whose events did not fit, replayed whole
     }

@@ -126,6 +126,10 @@ struct Queue {
   // the new state (null collisions, shadow-walk steps) or sigma_t
   // (scattering events), so that the gradient pass needs no grid lookup
   float* tape_f;
+  // paths that entered the medium, and how many there are; the others have no
+  // events, and their total radiance is not kept either
+  uint32_t* entered;
+  unsigned long long* entered_count;
 };
 
 // kForward: the replay tasks of kReplay, gathering a tangent field at every
@@ -139,8 +143,8 @@ enum TraceMode { kTwoState = 0, kSingle = 1, kAdjoint = 2, kReplay = 3, kForward
 constexpr int kTraceModes = 6;
 
 // Tape events: float4 (x, y, z, ref) with ref = kind << 30 | index.  The
-// index is the path (kEvCamera: null collisions before the first scattering
-// event) or the event record of the last scattering event (kEvSegment: null
+// index is that of the path among those that entered the medium (kEvCamera:
+// null collisions before the first scattering event) or the event record of the last scattering event (kEvSegment: null
 // collisions after its shadow walk; kEvScatter: the event itself; kEvShadow:
 // steps of its shadow walk).  Event record (2 float4): [path, radiance
 // gathered before the event's NEE contribution] [NEE contribution, 0].
@@ -229,6 +233,9 @@ struct AdjBuffers {
   uint32_t* lost_list;
   unsigned long long* lost_count;
   float* tape_f;  // each event's sigma_n (sigma_t at scattering events)
+  uint32_t* entered;  // paths that entered the medium
+  unsigned long long* entered_count;
+  float2* cam_w;  // their camera segments' weights
 };
 
 struct Counts {
@@ -605,12 +612,11 @@ inline float* tape_terms(char* region, int64_t room) { return reinterpret_cast<f
 
 // Gradient from a kTape radiance pass (rcv_tape.cu) of one job (jobs ==
 // NULL) or of a device job table: the per-record and per-path weights
-// (`weights`: 2 float4 per record, `cam_w`: one float2 per path) and the
+// (`weights`: 2 float4 per record) and the
 // scatter of every tape event into its job's gradient records.  Zeroes
 // *replay_counter, the hand-out counter of the replay that follows.
 int launch_tape_gradient(const VolJob& single, const VolJob* jobs, int njobs, const AdjBuffers& A, float4* weights,
-                         float2* cam_w, int64_t paths, unsigned long long* replay_counter, uint64_t* counters,
-                         int sms, cudaStream_t st);
+                         unsigned long long* replay_counter, uint64_t* counters, int sms, cudaStream_t st);
 int tracer_sm_count();
 
 }  // namespace rcv
