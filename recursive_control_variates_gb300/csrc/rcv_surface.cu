@@ -12,6 +12,10 @@
 namespace rcv {
 
 constexpr int kSurfBlock = 128;
+// Resident blocks per SM that the registers are bounded for: 7 (72 registers,
+// a few spilled) 316 us for the two-state pass of 1024^2 x 8 spp, 6 324, 5
+// (94, none spilled) 341; the replays spill more and stay at 5.
+constexpr int surf_blocks(int mode) { return mode == kAdjoint || mode == kForward ? 5 : 7; }
 
 __global__ void pack_texture_kernel(int64_t n, const float* __restrict__ old_t,
                                     const float* __restrict__ new_t, float4* __restrict__ pairs) {
@@ -21,17 +25,23 @@ __global__ void pack_texture_kernel(int64_t n, const float* __restrict__ old_t,
   pairs[i * 2 + 1] = make_float4(new_t[i * 3 + 0], new_t[i * 3 + 1], new_t[i * 3 + 2], 0.0f);
 }
 
-__global__ void fold_texture_kernel(int64_t n, const float4* __restrict__ g, float* __restrict__ out) {
+// Texel (x, y) is corner 00 of its own cell, 10 of its left neighbour's, 01 of
+// the one above and 11 of the one above to the left (repeat wrap).
+__global__ void fold_texture_kernel(int tw, int th, const float* __restrict__ g, float* __restrict__ out) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 v = g[i];
-  out[i * 3 + 0] += v.x;
-  out[i * 3 + 1] += v.y;
-  out[i * 3 + 2] += v.z;
+  if (i >= int64_t(tw) * th) return;
+  const int y = (int)((uint32_t)i / (uint32_t)tw), x = (int)((uint32_t)i - (uint32_t)y * (uint32_t)tw);
+  const int xl = x == 0 ? tw - 1 : x - 1, yl = y == 0 ? th - 1 : y - 1;
+  const float* c00 = g + i * 12;
+  const float* c10 = g + (int64_t(y) * tw + xl) * 12 + 3;
+  const float* c01 = g + (int64_t(yl) * tw + x) * 12 + 6;
+  const float* c11 = g + (int64_t(yl) * tw + xl) * 12 + 9;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) out[i * 3 + k] += (c00[k] + c10[k]) + (c01[k] + c11[k]);
 }
 
 template <int kMode>
-__global__ void __launch_bounds__(kSurfBlock) trace_surface_kernel(const __grid_constant__ SurfJob S,
+__global__ void __launch_bounds__(kSurfBlock, surf_blocks(kMode)) trace_surface_kernel(const __grid_constant__ SurfJob S,
                                                                    const __grid_constant__ Queue Q) {
   SurfCounts cnt{0, 0, 0, 0, 0};
   trace_surface<kMode>(S, Q, cnt);
@@ -59,7 +69,7 @@ static SurfLayout surf_layout(int tw, int th) {
   SurfLayout L;
   L.pairs = 0;
   L.grad = align256(n * 32u);
-  L.total = align256(L.grad + n * 16u);
+  L.total = align256(L.grad + n * 48u);
   return L;
 }
 
@@ -299,14 +309,14 @@ extern "C" int rcv_render_backward_surface(const rcv_surface_scene* sc, const rc
   const SurfLayout L = surf_layout(sc->tex_width, sc->tex_height);
   char* ws = static_cast<char*>(sc->workspace);
   const int64_t n = int64_t(sc->tex_width) * sc->tex_height;
-  RCV_TRY_CUDA(cudaMemsetAsync(ws + L.grad, 0, n * 16, st), "texture gradient reset");
+  RCV_TRY_CUDA(cudaMemsetAsync(ws + L.grad, 0, n * 48, st), "texture gradient reset");
   S.grad_img = grad_img;
   S.grad_tex = reinterpret_cast<float4*>(ws + L.grad);
   rc = run_surface(kAdjoint, S, o, workspace, counters, nullptr, nullptr, st);
   if (rc) return rc;
   const int block = 256;
-  fold_texture_kernel<<<grid_for(n, block), block, 0, st>>>(n, reinterpret_cast<const float4*>(ws + L.grad),
-                                                           grad_texture);
+  fold_texture_kernel<<<grid_for(n, block), block, 0, st>>>(sc->tex_width, sc->tex_height,
+                                                           reinterpret_cast<const float*>(ws + L.grad), grad_texture);
   return launched("fold_texture launch");
 }
 

@@ -49,7 +49,9 @@ struct SurfJob {
   float light_hx, light_hz, light_area;
   V3 light_le;
   const float* grad_img;
-  float4* grad_tex;  // [tex_h * tex_w] rgb + pad (forward mode: the texture tangent)
+  // gradient records, 3 float4 per texel cell (4 corners x RGB); forward mode:
+  // the texture tangent, one float4 (rgb + pad) per texel
+  float4* grad_tex;
   float* out_img;    // forward mode: image derivative
   int64_t path_count;
 };
@@ -66,7 +68,8 @@ __device__ __forceinline__ int intersect(const SurfJob& S, const V3& o, const V3
   int id = kMiss;
   t_hit = tmax;
   if (d.y != 0.0f) {
-    const float t = (0.0f - o.y) / d.y;
+    const float inv_y = 1.0f / d.y;
+    const float t = div_by(0.0f - o.y, d.y, inv_y);
     if (t > 1e-6f && t < t_hit) {
       const float x = fmaf(t, d.x, o.x), z = fmaf(t, d.z, o.z);
       if (fabsf(x) <= S.plane_half && fabsf(z) <= S.plane_half) {
@@ -74,7 +77,7 @@ __device__ __forceinline__ int intersect(const SurfJob& S, const V3& o, const V3
         id = kPlane;
       }
     }
-    const float tl = (S.light_c.y - o.y) / d.y;
+    const float tl = div_by(S.light_c.y - o.y, d.y, inv_y);
     if (tl > 1e-6f && tl < t_hit) {
       const float x = fmaf(tl, d.x, o.x) - S.light_c.x, z = fmaf(tl, d.z, o.z) - S.light_c.z;
       if (fabsf(x) <= S.light_hx && fabsf(z) <= S.light_hz) {
@@ -100,11 +103,37 @@ __device__ __forceinline__ int intersect(const SurfJob& S, const V3& o, const V3
   return id;
 }
 
-// Shadow test: is anything but the light between o and o + dist * d?
+// Shadow test: is anything but the light between o and o + dist * d?  The
+// closest hit's test without the hit: a sphere counts up to the plane's or the
+// light's distance, and the first one ends the search.  Shadow rays rise (d.y >
+// 0), so the ground is behind them unless they start below it.
 __device__ __forceinline__ bool occluded(const SurfJob& S, const V3& o, const V3& d, float dist) {
-  float t;
-  const int id = intersect(S, o, d, dist * (1.0f - kShadowEps), t);
-  return id != kMiss && id != kLight;
+  float t_hit = dist * (1.0f - kShadowEps);
+  if (o.y < 0.0f) {
+    float t;
+    const int id = intersect(S, o, d, t_hit, t);
+    return id != kMiss && id != kLight;
+  }
+  const float dy = S.light_c.y - o.y;
+  if (dy <= t_hit * d.y) {  // the light's plane comes (nearly) before: the exact distance decides
+    const float tl = dy / d.y;
+    if (tl > 1e-6f && tl < t_hit) {
+      const float x = fmaf(tl, d.x, o.x) - S.light_c.x, z = fmaf(tl, d.z, o.z) - S.light_c.z;
+      if (fabsf(x) <= S.light_hx && fabsf(z) <= S.light_hz) t_hit = tl;
+    }
+  }
+  for (int k = 0; k < S.nspheres; ++k) {
+    const V3 oc{o.x - S.sph[k].c.x, o.y - S.sph[k].c.y, o.z - S.sph[k].c.z};
+    const float b = dot3(oc, d);
+    const float c = fmaf(-S.sph[k].r, S.sph[k].r, dot3(oc, oc));
+    const float disc = fmaf(b, b, -c);
+    if (disc < 0.0f) continue;
+    const float sq = sqrtf(disc);
+    float t = -b - sq;
+    if (!(t > 1e-6f)) t = -b + sq;
+    if (t > 1e-6f && t < t_hit) return true;
+  }
+  return false;
 }
 
 __device__ __forceinline__ V3 shape_normal(const SurfJob& S, int id, const V3& p) {
@@ -167,13 +196,17 @@ __device__ __forceinline__ V3 tex_eval(const SurfJob& S, const TexLookup& l, int
   return V3{lerpf(lo.x, hi.x, l.fy), lerpf(lo.y, hi.y, l.fy), lerpf(lo.z, hi.z, l.fy)};
 }
 
+// Scatters g * (bilinear weight of each corner) into the record of the lookup's
+// cell (its corner 00: 12 floats, corners 00 10 01 11 by RGB): three vector
+// reductions, none of them padding, where the four texels took four.  The
+// fold adds up the records that hold a texel.
 __device__ __forceinline__ void tex_scatter(const SurfJob& S, const TexLookup& l, const V3& g) {
   const float gx = 1.0f - l.fx, gy = 1.0f - l.fy;
   const float w00 = gx * gy, w10 = l.fx * gy, w01 = gx * l.fy, w11 = l.fx * l.fy;
-  red_add_v4(S.grad_tex + l.i00, g.x * w00, g.y * w00, g.z * w00, 0.0f);
-  red_add_v4(S.grad_tex + l.i10, g.x * w10, g.y * w10, g.z * w10, 0.0f);
-  red_add_v4(S.grad_tex + l.i01, g.x * w01, g.y * w01, g.z * w01, 0.0f);
-  red_add_v4(S.grad_tex + l.i11, g.x * w11, g.y * w11, g.z * w11, 0.0f);
+  float4* r = S.grad_tex + (int64_t)l.i00 * 3;
+  red_add_v4(r + 0, g.x * w00, g.y * w00, g.z * w00, g.x * w10);
+  red_add_v4(r + 1, g.y * w10, g.z * w10, g.x * w01, g.y * w01);
+  red_add_v4(r + 2, g.z * w01, g.x * w11, g.y * w11, g.z * w11);
 }
 
 // Forward mode: bilinear tangent of the texture (grad_tex holds it).
@@ -206,7 +239,16 @@ struct SurfCounts {
   uint32_t paths, bounces, shadow_rays, tex_vertices, grad_events;
 };
 
-enum SurfPhase { kSIdle = 0, kSStart = 1, kSBounce = 2 };
+// A lane starts a path, traces its ray, and shades the hit.  Half of the
+// camera rays and most bounced rays miss everything, while shading (light
+// sample with its shadow ray, reflectances, next direction) costs three times
+// a ray; so hits wait until kShadeLanes lanes of the warp have one, and the
+// lanes that missed start and trace new paths meanwhile.  Shading with
+// whatever hits each round of rays gave ran with a third of the lanes
+// (1024^2 x 8 spp, two-state pass: 393 us; 12 / 16 / 20 / 24 / 28 lanes 363 / 328
+// / 324 / 325 / 331).
+enum SurfPhase { kSIdle = 0, kSStart = 1, kSTrace = 2, kSHit = 3 };
+constexpr unsigned kShadeLanes = 20;
 
 template <int kMode>
 __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt) {
@@ -219,7 +261,7 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
   bool lost = false;      // kTape: a vertex of this path did not fit
   int64_t batch_next = 0, batch_end = 0;
   bool queue_empty = false;
-  int64_t path = 0;
+  uint32_t path = 0;  // a film has fewer than 2^32 paths
   int phase = kSIdle, pass = 0;
   Pcg32 rng;
   V3 o, d;
@@ -227,6 +269,36 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
   float prev_pdf = 1.0f;
   bool prev_delta = true;
   int depth = 0;
+  float t = 0.0f;  // the hit that waits for shading
+  int id = kMiss;
+
+  // end of the lane's path (or of its first pass)
+  const auto end_path = [&]() {
+    if (kMode == kTape) {
+      Q.path_ltot[path] = make_float4(Ln.x, Ln.y, Ln.z, lost ? 1.0f : 0.0f);
+      if (lost) Q.lost_list[atomicAdd(Q.lost_count, 1ull)] = path;
+    }
+    if ((kMode == kAdjoint || kMode == kForward) && pass == 0) {
+      Ltot = Ln;
+      pass = 1;
+      phase = kSStart;
+    } else {
+      if (kMode == kForward && (dL.x != 0.0f || dL.y != 0.0f || dL.z != 0.0f)) {
+        const float fs = (float)S.spp;
+        float* o = S.out_img + (int64_t)(path / (uint32_t)S.spp) * 3;
+        atomicAdd(o + 0, dL.x / fs);
+        atomicAdd(o + 1, dL.y / fs);
+        atomicAdd(o + 2, dL.z / fs);
+      }
+      if (kMode == kTwoState || kMode == kSingle) {
+        float4* out = Q.path_out + (int64_t)path * (kMode == kTwoState ? 2 : 1);
+        __stcs(out, make_float4(Ln.x, Ln.y, Ln.z, 0.0f));
+        if (kMode == kTwoState) __stcs(out + 1, make_float4(Lo.x, Lo.y, Lo.z, 0.0f));
+      }
+      ++cnt.paths;
+      phase = kSIdle;
+    }
+  };
 
   while (true) {
     unsigned need = __ballot_sync(0xffffffffu, phase == kSIdle);
@@ -246,7 +318,7 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
       const unsigned take = min((unsigned)__popc(need), avail);
       const unsigned rank = (unsigned)__popc(need & lt_mask);
       if (((need >> lane) & 1u) && rank < take) {
-        path = lost_only ? (int64_t)Q.lost_list[batch_next + rank] : batch_next + rank;
+        path = lost_only ? Q.lost_list[batch_next + rank] : (uint32_t)(batch_next + rank);
         phase = kSStart;
         pass = 0;
       }
@@ -254,17 +326,11 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
       need = __ballot_sync(0xffffffffu, phase == kSIdle);
     }
     if (queue_empty && __all_sync(0xffffffffu, phase == kSIdle)) break;
-    // kTape: idle lanes stay for the warp-wide tape append below
-    if (kMode != kTape && phase == kSIdle) continue;
-
-    const int pix = (int)(path / S.spp);
-    bool finished = false;
-    bool ev = false;  // kTape: this bounce's texture vertex, recorded below
-    V3 ev_p{0.0f, 0.0f, 0.0f}, ev_l{0.0f, 0.0f, 0.0f};
     if (phase == kSStart) {
-      seed_lane(rng, S.seed, (uint32_t)path);
+      seed_lane(rng, S.seed, path);
       const float u0 = next1d(rng), u1 = next1d(rng);
-      surf_camera(S, pix % S.width, pix / S.width, u0, u1, d);
+      const uint32_t pix = path / (uint32_t)S.spp, py = pix / (uint32_t)S.width;
+      surf_camera(S, (int)(pix - py * (uint32_t)S.width), (int)py, u0, u1, d);
       o = S.cam_o;
       bo = V3{1, 1, 1};
       bn = V3{1, 1, 1};
@@ -286,17 +352,29 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
         }
         Lrem = Ltot;
       }
-      phase = kSBounce;
+      phase = kSTrace;
     }
 
-    // ------------------------------------------------------------ one bounce
-    if (kMode != kTape || phase == kSBounce) {
+    // ------------------------------------------------------------ trace a ray
+    if (phase == kSTrace) {
       ++cnt.bounces;
-      float t;
-      const int id = intersect(S, o, d, kInf, t);
-      if (id == kMiss) {
-        finished = true;  // no environment light
-      } else {
+      id = intersect(S, o, d, kInf, t);
+      if (id == kMiss)
+        end_path();  // no environment light
+      else
+        phase = kSHit;
+    }
+
+    // -------------------------------------------------------------- shade hits
+    // (while paths are left to hand out, lanes that ended theirs come first)
+    const unsigned m_hit = __ballot_sync(0xffffffffu, phase == kSHit);
+    if (m_hit == 0u || (!queue_empty && (unsigned)__popc(m_hit) < kShadeLanes)) continue;
+    bool finished = false;
+    bool ev = false;  // kTape: this bounce's texture vertex, recorded below
+    V3 ev_p{0.0f, 0.0f, 0.0f}, ev_l{0.0f, 0.0f, 0.0f};
+    {
+      if (phase == kSHit) {
+        phase = kSTrace;
         const V3 p = advance(o, t, d);
         const V3 n = shape_normal(S, id, p);
         const V3 wi{-d.x, -d.y, -d.z};
@@ -371,7 +449,14 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
             if (!occluded(S, org, wl, dist)) {
               const float pdf_b = kInvPi * cos_o;
               const float mis = mis_power(pdf_l, pdf_b);
-              const V3 ew{S.light_le.x / pdf_l, S.light_le.y / pdf_l, S.light_le.z / pdf_l};
+              V3 ew;
+              if (pdf_l > 1e-30f && pdf_l < 1e30f) {
+                const float inv_l = 1.0f / pdf_l;
+                ew = V3{div_by(S.light_le.x, pdf_l, inv_l), div_by(S.light_le.y, pdf_l, inv_l),
+                        div_by(S.light_le.z, pdf_l, inv_l)};
+              } else {
+                ew = V3{S.light_le.x / pdf_l, S.light_le.y / pdf_l, S.light_le.z / pdf_l};
+              }
               const V3 vn{(an.x * kInvPi) * cos_o, (an.y * kInvPi) * cos_o, (an.z * kInvPi) * cos_o};
               const V3 cn{((bn.x * mis) * vn.x) * ew.x, ((bn.y * mis) * vn.y) * ew.y,
                           ((bn.z * mis) * vn.z) * ew.z};
@@ -404,7 +489,10 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
           if (pdf > 0.0f) {
             if (kMode == kTwoState) {
               const V3 vold{(ao.x * kInvPi) * lz, (ao.y * kInvPi) * lz, (ao.z * kInvPi) * lz};
-              bo = V3{bo.x * (vold.x / pdf), bo.y * (vold.y / pdf), bo.z * (vold.z / pdf)};
+              // pdf is between 1e-4 and 1/pi (s0 <= 1 - 2^-23)
+              const float inv_pdf = 1.0f / pdf;
+              bo = V3{bo.x * div_by(vold.x, pdf, inv_pdf), bo.y * div_by(vold.y, pdf, inv_pdf),
+                      bo.z * div_by(vold.z, pdf, inv_pdf)};
             }
             bn = V3{bn.x * an.x, bn.y * an.y, bn.z * an.z};  // diffuse sample weight = reflectance
             prev_pdf = pdf;
@@ -436,37 +524,12 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
     }
 
     if (kMode == kTape) {
-      const float4 a = make_float4(ev_p.x, ev_p.z, __uint_as_float((uint32_t)path), 0.0f);
+      const float4 a = make_float4(ev_p.x, ev_p.z, __uint_as_float(path), 0.0f);
       const float4 b = make_float4(ev_l.x, ev_l.y, ev_l.z, 0.0f);
       if (!tape_append_n<2>(Q, tc, ev && !lost, a, b)) lost = true;
     }
 
-    if (finished) {
-      if (kMode == kTape) {
-        Q.path_ltot[path] = make_float4(Ln.x, Ln.y, Ln.z, lost ? 1.0f : 0.0f);
-        if (lost) Q.lost_list[atomicAdd(Q.lost_count, 1ull)] = (uint32_t)path;
-      }
-      if ((kMode == kAdjoint || kMode == kForward) && pass == 0) {
-        Ltot = Ln;
-        pass = 1;
-        phase = kSStart;
-      } else {
-        if (kMode == kForward && (dL.x != 0.0f || dL.y != 0.0f || dL.z != 0.0f)) {
-          const float fs = (float)S.spp;
-          float* o = S.out_img + (int64_t)pix * 3;
-          atomicAdd(o + 0, dL.x / fs);
-          atomicAdd(o + 1, dL.y / fs);
-          atomicAdd(o + 2, dL.z / fs);
-        }
-        if (kMode == kTwoState || kMode == kSingle) {
-          float4* out = Q.path_out + path * (kMode == kTwoState ? 2 : 1);
-          out[0] = make_float4(Ln.x, Ln.y, Ln.z, 0.0f);
-          if (kMode == kTwoState) out[1] = make_float4(Lo.x, Lo.y, Lo.z, 0.0f);
-        }
-        ++cnt.paths;
-        phase = kSIdle;
-      }
-    }
+    if (finished) end_path();
   }
   if (kMode == kTape) tape_close(Q, tc);  // the unused slots of the warp's last chunk
 }

@@ -55,15 +55,6 @@ struct VpsParams {
   const unsigned long long* lost_count;
 };
 
-// a / b for 0 <= a <= b given inv = 1 / b rounded: a quotient estimate and one
-// correction by its exact residual, which rounds correctly (Markstein 1990,
-// "Computation of elementary functions on the IBM RISC System/6000
-// processor"); three operations instead of a division per free-flight step.
-__device__ __forceinline__ float div_by(float a, float b, float inv) {
-  const float q = a * inv;
-  return fmaf(fmaf(-q, b, a), inv, q);
-}
-
 __device__ __forceinline__ uint64_t pack64(uint32_t lo, uint32_t hi) { return (uint64_t)lo | ((uint64_t)hi << 32); }
 
 // Pixel of a path in the launch's hand-out order, and its random stream.
