@@ -8,7 +8,7 @@
 namespace rcv {
 
 // Cell i of a (dx+1)(dy+1)(dz+1) lattice: the 8 clamped corner voxels of the
-// old and the new density.
+// old and the new density, x pairs as value and difference (trilerp_diff).
 // 32-bit index arithmetic: 4 (dx+1)(dy+1)(dz+1) < 2^32 is enforced on the host.
 __device__ __forceinline__ void pack_cell(int64_t i, int dx, int dy, int dz, const float* __restrict__ old_d,
                                           const float* __restrict__ new_d, float4* __restrict__ cells) {
@@ -25,10 +25,11 @@ __device__ __forceinline__ void pack_cell(int64_t i, int dx, int dy, int dz, con
   const int64_t i000 = idx(x0, y0, z0), i100 = idx(x1, y0, z0), i010 = idx(x0, y1, z0), i110 = idx(x1, y1, z0),
                 i001 = idx(x0, y0, z1), i101 = idx(x1, y0, z1), i011 = idx(x0, y1, z1), i111 = idx(x1, y1, z1);
   float4* c = cells + i * 4;
-  c[0] = make_float4(old_d[i000], old_d[i100], old_d[i010], old_d[i110]);
-  c[1] = make_float4(old_d[i001], old_d[i101], old_d[i011], old_d[i111]);
-  c[2] = make_float4(new_d[i000], new_d[i100], new_d[i010], new_d[i110]);
-  c[3] = make_float4(new_d[i001], new_d[i101], new_d[i011], new_d[i111]);
+  const auto pairs = [](float a0, float a1, float b0, float b1) { return make_float4(a0, a1 - a0, b0, b1 - b0); };
+  c[0] = pairs(old_d[i000], old_d[i100], old_d[i010], old_d[i110]);
+  c[1] = pairs(old_d[i001], old_d[i101], old_d[i011], old_d[i111]);
+  c[2] = pairs(new_d[i000], new_d[i100], new_d[i010], new_d[i110]);
+  c[3] = pairs(new_d[i001], new_d[i101], new_d[i011], new_d[i111]);
 }
 
 // Voxels whose trilinear weight can be non-zero inside supergrid cell c of

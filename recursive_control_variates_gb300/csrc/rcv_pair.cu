@@ -21,14 +21,11 @@
 
 namespace rcv {
 
-// kBlocks: resident blocks per SM that the registers are bounded for, 6 (80
-// registers) or 7 (72, a few spilled).  The seventh pays where a launch is
-// long against its longest paths, which it slows: job tables (24 mixed jobs
-// 19.1 -> 18.5 ms a step) and films of kManyPaths paths or more (33.6 M paths
-// on 256^3: 13.6 -> 13.3 ms; 8.4 M on 64^3: 2.71 -> 2.76 ms; 0.5 M seen by
-// five cameras: 1.66 -> 1.78 ms).
-constexpr int64_t kManyPaths = int64_t(1) << 24;
-
+// kBlocks: resident blocks per SM that the registers are bounded for: 7 (72
+// registers, none spilled) but under an environment map, whose launches end on
+// longer paths, 6.  Paired launch at 6 / 7 / 8 blocks: 512^2 x (16 + 16) spp on
+// 64^3 1477 / 1430 / 1466 us, 1024^2 on 256^3 5.79 / 5.25 / 5.62 ms, 24 mixed
+// jobs 12.8 / 12.5 / 13.5 ms, five map-lit 107 x 83 views 791 / 817 / 846 us.
 template <bool kSG, bool kEnv, bool kTable, int kBlocks>
 __global__ void __launch_bounds__(kTraceBlock, kBlocks)
     trace_pair_kernel(const __grid_constant__ VolJob JA, const __grid_constant__ Queue QA,
@@ -53,14 +50,12 @@ __global__ void __launch_bounds__(kTraceBlock, kBlocks)
 }
 
 using PairKernel = void (*)(VolJob, Queue, VolJob, Queue);
-// by supergrid + 2 * environment map (single jobs), then job tables by
-// supergrid, then single jobs of many paths by supergrid
-constexpr int kPairVariants = 8;
+// by supergrid + 2 * environment map (single jobs), then job tables by supergrid
+constexpr int kPairVariants = 6;
 static const PairKernel kPairKernels[kPairVariants] = {
-    trace_pair_kernel<false, false, false, 6>, trace_pair_kernel<true, false, false, 6>,
+    trace_pair_kernel<false, false, false, 7>, trace_pair_kernel<true, false, false, 7>,
     trace_pair_kernel<false, true, false, 6>,  trace_pair_kernel<true, true, false, 6>,
-    trace_pair_kernel<false, false, true, 7>,  trace_pair_kernel<true, false, true, 7>,
-    trace_pair_kernel<false, false, false, 7>, trace_pair_kernel<true, false, false, 7>};
+    trace_pair_kernel<false, false, true, 7>,  trace_pair_kernel<true, false, true, 7>};
 
 static int pair_blocks_per_sm(int variant) {
   static std::once_flag once;
@@ -89,8 +84,7 @@ int launch_pair(const VolJob& JA, const Queue& QA, const VolJob& JB, const Queue
   // an environment map belongs to a single job (job tables take the constant environment)
   const bool env = single && JA.env.valid != 0;
   RCV_REQUIRE(!single || (JB.env.valid != 0) == env, "the paired jobs must share their environment");
-  const bool many = single && !env && QA.total + QB.total >= kManyPaths;
-  const int variant = (sg ? 1 : 0) + (single ? (many ? 6 : (env ? 2 : 0)) : 4);
+  const int variant = (sg ? 1 : 0) + (single ? (env ? 2 : 0) : 4);
   int per_sm = pair_blocks_per_sm(variant);
   if (o != nullptr && o->blocks_per_sm > 0 && o->blocks_per_sm < per_sm) per_sm = o->blocks_per_sm;
   const int64_t warps_needed = (QA.total + QA.batch - 1) / QA.batch + (QB.total + QB.batch - 1) / QB.batch;

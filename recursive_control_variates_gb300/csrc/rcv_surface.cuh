@@ -263,8 +263,8 @@ __device__ void trace_surface(const SurfJob& S, const Queue& Q, SurfCounts& cnt)
   bool queue_empty = false;
   uint32_t path = 0;  // a film has fewer than 2^32 paths
   int phase = kSIdle, pass = 0;
-  Pcg32 rng;
-  V3 o, d;
+  Pcg32 rng{0ull, 0ull};
+  V3 o{0, 0, 0}, d{0, 0, 0};
   V3 bo{1, 1, 1}, bn{1, 1, 1}, Lo{0, 0, 0}, Ln{0, 0, 0}, Lrem{0, 0, 0}, Ltot{0, 0, 0}, dL{0, 0, 0};
   float prev_pdf = 1.0f;
   bool prev_delta = true;

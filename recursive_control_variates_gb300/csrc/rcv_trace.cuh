@@ -326,22 +326,31 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
   unsigned long long* const next = s_next + (threadIdx.x >> 5);
   unsigned left = 0u;
   bool queue_empty = false;
-  const VolJob* Jp = &single;
+  const VolJob* Jp = kTable ? Q.jobs : nullptr;
   int phase = kIdle;
   float mu = 0.0f, inv_mu = 0.0f;  // half of inv_mu is recomputed where needed (one register less)
+  const auto job_majorant = [&](const VolJob& J) {
+    const float mu_old = J.scale * bits_to_float(__ldg(J.maxbits + 0));
+    const float mu_new = J.scale * bits_to_float(__ldg(J.maxbits + 1));
+    mu = (kMode == kTwoState) ? fmaxf(mu_old, mu_new) : mu_new;
+    inv_mu = 1.0f / mu;
+  };
+  if (!kTable) job_majorant(single);  // the same for every path
   V3 dL{0.0f, 0.0f, 0.0f};  // kForward: the task's image derivative
   // kReplay: dL . L_rem with dL = dLoss/dL of the pixel; it changes only with
   // L_rem, and dL itself is recomputed from the image gradient at the events
   // that need it per channel (fewer registers live through the walk)
   float s_main = 0.0f;
 
-  Pcg32 rng;
+  // (defined from the start: left undefined, a state would carry from one
+  // tracer of a paired launch into the next and cost registers there)
+  Pcg32 rng{0ull, 0ull};
   // whole-path replay: state of the stream of the second shadow walk (its
   // increment is rng.inc)
   uint64_t nee_state = 0;
   // the walk: position, direction and distance left of the main path or of
   // its shadow ray; throughputs
-  V3 x, dir;
+  V3 x{0, 0, 0}, dir{0, 0, 0};
   float rem = 0.0f;
   V3 bo{1, 1, 1}, bn{1, 1, 1};
   int depth = 0;
@@ -402,7 +411,8 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     }
     const unsigned m_start = __ballot_sync(0xffffffffu, phase == kStart);
     const unsigned m_scat = __ballot_sync(0xffffffffu, phase == kScatter);
-    const unsigned m_walk = __ballot_sync(0xffffffffu, phase >= kMain && phase != kScatter);
+    // (`need` holds the idle lanes: every other lane walks)
+    const unsigned m_walk = ~(need | m_start | m_scat);
     if (queue_empty && (m_start | m_scat | m_walk) == 0u) break;
     // Once the queue is empty no new lanes arrive to fill a deferred branch;
     // waiting would only make the warp's last paths take turns.
@@ -444,10 +454,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       U(cPath) = (uint32_t)path;
       if (kTable) Jp = &job_of(Q, path);
       const VolJob& J = kTable ? *Jp : single;
-      const float mu_old = J.scale * bits_to_float(__ldg(J.maxbits + 0));
-      const float mu_new = J.scale * bits_to_float(__ldg(J.maxbits + 1));
-      mu = (kMode == kTwoState) ? fmaxf(mu_old, mu_new) : mu_new;
-      inv_mu = 1.0f / mu;
+      if (kTable) job_majorant(J);
       // k-th pixel of the job's hand-out order, sample s of that pixel
       // 32-bit index arithmetic: a job has fewer than 2^32 paths
       const uint32_t local = (uint32_t)(path - J.path_begin);
@@ -745,8 +752,16 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
         }
         const float st_o = J.scale * rho_o, st_n = J.scale * rho_n;
 
-        if (phase == kMain) {
-          if (valid) {
+        bool walk_done = false;  // the shadow walk ends
+        if (valid) {
+          // factors of the step if it is not a scattering event: ratio
+          // tracking of a shadow ray (plugins/twostatevolpath.py:443-452), or
+          // the weights of a null collision (:227-231, 256-257; they sum to 2,
+          // equal states give exactly 1)
+          const float sn_n = mu_c - st_n;
+          float fn = sn_n * inv_c, fo = kMode == kTwoState ? (mu_c - st_o) * inv_c : 1.0f;
+          bool null = true;
+          if (phase == kMain) {
             const float ur = next1d(rng);
             // real-collision probability: mean of both states' sigma_t / mu
             // (plugins/twostatevolpath.py:222-225); equal states give exactly
@@ -756,107 +771,89 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
               prob = (st_n + st_o) * hinv_c;
             else
               prob = st_n * inv_c;
-            if (ur >= prob) {
-              // null collision (plugins/twostatevolpath.py:227-231, 256-257);
-              // the two weights sum to 2, equal states give exactly 1
-              if (kMode == kTwoState) {
-                const float sn_o = mu_c - st_o, sn_n = mu_c - st_n;
-                const float den = sn_n + sn_o;
-                const float wn = (2.0f * sn_n) / den, wo = 2.0f - wn;
-                bn = V3{bn.x * wn, bn.y * wn, bn.z * wn};
-                bo = V3{bo.x * wo, bo.y * wo, bo.z * wo};
-              } else if (kMode == kReplay) {
-                const float sn = mu_c - st_n;
-                scatter_density(J, lk, -(J.scale * s_main) / sn);
-                if (kCount) ++cnt.grad_events;
-              } else if (kMode == kForward) {
-                const float sn = mu_c - st_n;
-                const V3 Lr = Lrem;
-                const float f = -(J.scale * tangent_density(J, lk)) / sn;
-                dL = V3{dL.x + Lr.x * f, dL.y + Lr.y * f, dL.z + Lr.z * f};
-                if (kCount) ++cnt.grad_events;
-              }
-              rem = rem - t;
-              if (kMode == kTape) {
-                ev_walk = true;
-                ev_ref = tref;
-                ev_f = mu_c - st_n;
-              }
-            } else {
-              // real scattering event (plugins/twostatevolpath.py:249-253)
-              depth += 1;
-              if (depth >= J.max_depth) {
-                finished = true;
-              } else {
-                if (kCount) ++cnt.scatters;
-                F(cScn) = st_n;
-                if (kMode == kTwoState) F(cSco) = st_o;
-                phase = kScatter;
-              }
+            null = ur >= prob;
+            fn = 1.0f;
+            if (kMode == kTwoState) {
+              const float den = sn_n + (mu_c - st_o);
+              fn = (2.0f * sn_n) / den;
+              fo = 2.0f - fn;
             }
-          } else {
-            // leaves the cube: null BSDF sample, outside iteration RR, environment
-            pcg_skip3(rng);
-            if (roulette<kMode>(J, rng, depth, bn, bo) && !(J.hide_emitters && depth == 0)) {
-              V3 Ln = get3(cLn), Lo{0, 0, 0};
-              if (kMode == kTwoState) Lo = get3(cLo);
-              if (kEnv) {
-                // environment map hit after a phase sample: power heuristic
-                // against NEE (plugins/twostatevolpath.py:288-308)
-                float pdf;
-                const V3 Le = env_radiance_dir(J, dir, pdf);
-                const float k = depth == 0 ? 1.0f : env_mis(kInvFourPi, pdf);
-                Ln = V3{Ln.x + (bn.x * Le.x) * k, Ln.y + (bn.y * Le.y) * k, Ln.z + (bn.z * Le.z) * k};
-                if (kMode == kTwoState)
-                  Lo = V3{Lo.x + (bo.x * Le.x) * k, Lo.y + (bo.y * Le.y) * k, Lo.z + (bo.z * Le.z) * k};
-              } else {
-                const float k = depth == 0 ? 1.0f : mis;
-                Ln = V3{Ln.x + bn.x * k, Ln.y + bn.y * k, Ln.z + bn.z * k};
-                if (kMode == kTwoState) Lo = V3{Lo.x + bo.x * k, Lo.y + bo.y * k, Lo.z + bo.z * k};
-              }
-              put3(cLn, Ln);
-              if (kMode == kTwoState) put3(cLo, Lo);
-            }
-            finished = true;
           }
-        } else if (phase == kNee) {
-          nee_done = !valid;
-          if (valid) {
-            // ratio tracking (plugins/twostatevolpath.py:443-452)
-            trn = trn * ((mu_c - st_n) * inv_c);
-            if (kMode == kTwoState) tro = tro * ((mu_c - st_o) * inv_c);
+          if (null) {
+            bn.x *= fn;  // (of a shadow ray: its transmittance)
+            if (kMode == kTwoState) {
+              bo.x *= fo;
+              const float gn = phase == kMain ? fn : 1.0f, go = phase == kMain ? fo : 1.0f;
+              bn.y *= gn;
+              bn.z *= gn;
+              bo.y *= go;
+              bo.z *= go;
+            }
+            if (kRep && phase != kNee && (phase == kMain || sn_n > 0.0f)) {
+              if (kMode == kForward) {
+                const V3 Lr = phase == kMain ? Lrem : cn_task;
+                const float f = -(J.scale * tangent_density(J, lk)) / sn_n;
+                dL = V3{dL.x + Lr.x * f, dL.y + Lr.y * f, dL.z + Lr.z * f};
+              } else {
+                scatter_density(J, lk, -(J.scale * (phase == kMain ? s_main : s_nee)) / sn_n);
+              }
+              if (kCount) ++cnt.grad_events;
+            }
             rem = rem - t;
             if (kMode == kTape) {
               ev_walk = true;
               ev_ref = tref;
-              ev_f = mu_c - st_n;
+              ev_f = sn_n;
             }
-            nee_done = (kMode == kTwoState) ? (trn == 0.0f && tro == 0.0f) : (trn == 0.0f);
-          }
-        } else {  // kNeeAdj: the shadow walk with gradients
-          bool done = !valid;
-          if (valid) {
-            const float sn = mu_c - st_n;
-            if (sn > 0.0f) {
-              if (kMode == kForward) {
-                const float f = -(J.scale * tangent_density(J, lk)) / sn;
-                dL = V3{dL.x + cn_task.x * f, dL.y + cn_task.y * f, dL.z + cn_task.z * f};
-              } else {
-                scatter_density(J, lk, -(J.scale * s_nee) / sn);
-              }
-              if (kCount) ++cnt.grad_events;
+            walk_done = phase != kMain && ((kMode == kTwoState) ? (trn == 0.0f && tro == 0.0f) : (trn == 0.0f));
+          } else {
+            // real scattering event (plugins/twostatevolpath.py:249-253)
+            depth += 1;
+            if (depth >= J.max_depth) {
+              finished = true;
+            } else {
+              if (kCount) ++cnt.scatters;
+              F(cScn) = st_n;
+              if (kMode == kTwoState) F(cSco) = st_o;
+              phase = kScatter;
             }
-            trn = trn * (sn * inv_c);
-            rem = rem - t;
-            done = trn == 0.0f;
           }
-          if (done) {
-            bn.x = F(cBn);
-            x = get3(cP);
-            dir = get3(cWo);
-            rem = F(cT);
-            phase = kMain;
+        } else if (phase == kMain) {
+          // leaves the cube: null BSDF sample, outside iteration RR, environment
+          pcg_skip3(rng);
+          if (roulette<kMode>(J, rng, depth, bn, bo) && !(J.hide_emitters && depth == 0)) {
+            V3 Ln = get3(cLn), Lo{0, 0, 0};
+            if (kMode == kTwoState) Lo = get3(cLo);
+            if (kEnv) {
+              // environment map hit after a phase sample: power heuristic
+              // against NEE (plugins/twostatevolpath.py:288-308)
+              float pdf;
+              const V3 Le = env_radiance_dir(J, dir, pdf);
+              const float k = depth == 0 ? 1.0f : env_mis(kInvFourPi, pdf);
+              Ln = V3{Ln.x + (bn.x * Le.x) * k, Ln.y + (bn.y * Le.y) * k, Ln.z + (bn.z * Le.z) * k};
+              if (kMode == kTwoState)
+                Lo = V3{Lo.x + (bo.x * Le.x) * k, Lo.y + (bo.y * Le.y) * k, Lo.z + (bo.z * Le.z) * k};
+            } else {
+              const float k = depth == 0 ? 1.0f : mis;
+              Ln = V3{Ln.x + bn.x * k, Ln.y + bn.y * k, Ln.z + bn.z * k};
+              if (kMode == kTwoState) Lo = V3{Lo.x + bo.x * k, Lo.y + bo.y * k, Lo.z + bo.z * k};
+            }
+            put3(cLn, Ln);
+            if (kMode == kTwoState) put3(cLo, Lo);
           }
+          finished = true;
+        } else {
+          walk_done = true;
+        }
+        if (!kRep || phase == kNee) {
+          nee_done = walk_done;
+        } else if (walk_done) {
+          // kNeeAdj: the shadow walk with gradients ends
+          bn.x = F(cBn);
+          x = get3(cP);
+          dir = get3(cWo);
+          rem = F(cT);
+          phase = kMain;
         }
       }
     }

@@ -25,13 +25,13 @@ __device__ __forceinline__ void add_counts(unsigned long long* counters, const C
 }
 
 // Resident blocks per SM that a tracer's registers are bounded for.  More
-// warps hide more of the walk's latency but slow each of the longest paths,
-// on which a launch ends: the single-state tracer of target renders (64
-// registers suffice) 5 / 6 / 7 / 8 blocks 17.3 / 16.6 / 15.5 / 14.8 ms at
-// 512^2 x 256 spp; the two-state and radiance passes end on their tails from
-// 7 on; the replays spill below 96 registers.
+// warps hide more of the walk's latency but slow each of the longest paths, on
+// which a launch ends: the single-state tracer of target renders (56 registers
+// suffice) 5 / 6 / 7 / 8 / 9 blocks 17.3 / 16.6 / 15.5 / 14.8 / 14.5 ms at 512^2
+// x 256 spp; the other primal passes alone end on their tails from 7 on; the
+// replays spill below 96 registers.
 constexpr int tracer_blocks(int mode) {
-  return mode == kSingle ? 8 : (mode == kReplay || mode == kForward ? 5 : 6);
+  return mode == kSingle ? 9 : (mode == kReplay || mode == kForward ? 5 : 6);
 }
 
 template <int kMode, bool kSG, bool kCount, bool kEnv, bool kTable>

@@ -44,10 +44,23 @@ struct CamFrame {
   V3 o, f, r, u;
 };
 
-// Packed lookup cell: 8 corners of the old and the new density, 64 bytes.
-//   [0] old v000 v100 v010 v110   [1] old v001 v101 v011 v111
-//   [2] new v000 ...              [3] new v001 ...
-struct VolJob {
+// Packed lookup cell: 8 corners of the old and the new density, 64 bytes, the
+// second of each x pair as its difference to the first (d = v1 - v0, which a
+// lookup would subtract first).
+//   [0] old v000 d00 v010 d10   [1] old v001 d01 v011 d11
+//   [2] new v000 ...            [3] new v001 ...
+struct alignas(16) VolJob {
+  // medium: what every step of a walk reads comes first, in 16-byte groups
+  // that job tables load as vectors
+  int32_t dx, dy, dz;
+  int32_t long_axis;    // an axis has 2^21 voxels or more
+  float fdx, fdy, fdz;  // dx, dy, dz
+  float scale;
+  const float4* __restrict__ cells;   // (dz+1)(dy+1)(dx+1) * 4
+  const float4* __restrict__ albedo;  // adz*ady*adx * 2 (old, new) or null
+  // integrator
+  int32_t max_depth, rr_depth, hide_emitters;
+  uint32_t seed;
   // film / camera
   int32_t width, height, spp;
   int32_t n_cams;      // sub-sensors of a batch film (1 = a single sensor)
@@ -56,16 +69,7 @@ struct VolJob {
   // coordinates, so distances along a ray stay world distances
   V3 inv_box;
   CamFrame cam[RCV_MAX_SENSORS];
-  // integrator
-  int32_t max_depth, rr_depth, hide_emitters;
-  uint32_t seed;
-  // medium
-  int32_t dx, dy, dz;
-  float scale;
-  float fdx, fdy, fdz;  // dx, dy, dz
-  int32_t long_axis;    // an axis has 2^21 voxels or more
-  const float4* __restrict__ cells;   // (dz+1)(dy+1)(dx+1) * 4
-  const float4* __restrict__ albedo;  // adz*ady*adx * 2 (old, new) or null
+  // albedo
   int32_t adx, ady, adz;              // albedo grid resolution
   int32_t albedo_own_res;             // 1: differs from the density's
   float albedo_const[3];
@@ -304,14 +308,14 @@ __device__ __forceinline__ void density2(const VolJob& J, const Lookup& l, float
                                          float& rho_new) {
   const float4* c = J.cells + l.cell * 4;
   const float4 o0 = __ldg(c + 0), o1 = __ldg(c + 1), n0 = __ldg(c + 2), n1 = __ldg(c + 3);
-  rho_old = trilerp(o0, o1, l.ax.f, l.ay.f, l.az.f);
-  rho_new = trilerp(n0, n1, l.ax.f, l.ay.f, l.az.f);
+  rho_old = trilerp_diff(o0, o1, l.ax.f, l.ay.f, l.az.f);
+  rho_new = trilerp_diff(n0, n1, l.ax.f, l.ay.f, l.az.f);
 }
 
 __device__ __forceinline__ float density_new(const VolJob& J, const Lookup& l) {
   const float4* c = J.cells + l.cell * 4;
   const float4 n0 = __ldg(c + 2), n1 = __ldg(c + 3);
-  return trilerp(n0, n1, l.ax.f, l.ay.f, l.az.f);
+  return trilerp_diff(n0, n1, l.ax.f, l.ay.f, l.az.f);
 }
 
 __device__ __forceinline__ int clampi(int v, int hi) { return v < 0 ? 0 : (v > hi ? hi : v); }
@@ -491,17 +495,23 @@ __device__ __forceinline__ V3 tangent_albedo(const VolJob& J, const AlbedoLookup
             tri(a000.z, a100.z, a010.z, a110.z, a001.z, a101.z, a011.z, a111.z)};
 }
 
+// Whether a throughput component is not zero (any bit but the sign set).
+template <int kMode>
+__device__ __forceinline__ bool nonzero(const V3& bn, const V3& bo) {
+  uint32_t b = __float_as_uint(bn.x) | __float_as_uint(bn.y) | __float_as_uint(bn.z);
+  if (kMode == kTwoState) b |= __float_as_uint(bo.x) | __float_as_uint(bo.y) | __float_as_uint(bo.z);
+  return (b & 0x7fffffffu) != 0u;
+}
+
 // Russian roulette at the top of an iteration (plugins/twostatevolpath.py:182-188).
 // Returns false when the path terminates.
 template <int kMode>
 __device__ __forceinline__ bool roulette(const VolJob& J, Pcg32& rng, int depth, V3& bn, V3& bo) {
-  bool alive = (bn.x != 0.0f || bn.y != 0.0f || bn.z != 0.0f);
-  if (kMode == kTwoState) alive = alive || (bo.x != 0.0f || bo.y != 0.0f || bo.z != 0.0f);
-  if (!alive) return false;
-  float m = fmaxf(fmaxf(bn.x, bn.y), bn.z);
-  if (kMode == kTwoState) m = fmaxf(fmaxf(fmaxf(bn.x, bo.x), fmaxf(bn.y, bo.y)), fmaxf(bn.z, bo.z));
-  const float q = fminf(m, 0.99f);
+  if (!nonzero<kMode>(bn, bo)) return false;
   if (depth > J.rr_depth) {
+    float m = fmaxf(fmaxf(bn.x, bn.y), bn.z);
+    if (kMode == kTwoState) m = fmaxf(fmaxf(fmaxf(bn.x, bo.x), fmaxf(bn.y, bo.y)), fmaxf(bn.z, bo.z));
+    const float q = fminf(m, 0.99f);
     const float u = next1d(rng);
     if (!(u < q)) return false;
     const float inv = 1.0f / q;

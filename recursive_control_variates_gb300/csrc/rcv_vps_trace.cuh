@@ -93,8 +93,8 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
   uint32_t path = 0;
   int phase = kVIdle, depth = 0;
   int stage = 0;  // kVpsDrt: 0 distance on the kept segment, 1 NEE there, 2 the path from there
-  Pcg32 rng;
-  V3 xo, sd, p, w;          // segment origin and direction; walk position and direction
+  Pcg32 rng{0ull, 0ull};
+  V3 xo{0, 0, 0}, sd{0, 0, 0}, p{0, 0, 0}, w{0, 0, 0};          // segment origin and direction; walk position and direction
   float rem = 0.0f, acc = 0.0f;  // distance left; distance walked (segment) or transmittance (shadow)
   V3 thr{1, 1, 1}, L{0, 0, 0};
   bool lost = false;
