@@ -334,9 +334,9 @@ static int sm_count() {
 
 int tracer_sm_count() { return sm_count(); }
 
-int paths_per_fetch(int64_t total) {
+int paths_per_fetch(int64_t total, int most) {
   const int64_t share = total / (int64_t(sm_count()) * 24 * 8);
-  return (int)(share < 2 ? 2 : (share > 64 ? 64 : share));
+  return share < most ? (int)(share < 2 ? (most < 2 ? most : 2) : share) : most;
 }
 
 void warm_launch_config() {
@@ -399,8 +399,9 @@ int make_queue(int mode, const VolJob* jobs, int njobs, int64_t total, const rcv
   Q.jobs = jobs;
   Q.njobs = njobs;
   Q.total = total;
-  Q.batch = (o != nullptr && o->batch > 0) ? o->batch : paths_per_fetch(total);
-  RCV_REQUIRE(Q.batch <= (1 << 20), "batch must be <= 2^20");
+  const int most = (o != nullptr && o->batch > 0) ? o->batch : 64;
+  RCV_REQUIRE(most <= (1 << 20), "batch must be <= 2^20");
+  Q.batch = paths_per_fetch(total, most);
   Q.defer = (o != nullptr && o->defer > 0) ? o->defer : 8;
   RCV_REQUIRE(Q.defer <= 32, "defer must be in [1, 32]");
   if (!zeroed) RCV_TRY_CUDA(cudaMemsetAsync(Q.counter, 0, sizeof(unsigned long long), st), "queue reset");

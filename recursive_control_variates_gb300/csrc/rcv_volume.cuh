@@ -591,15 +591,15 @@ int launch_persistent(int mode, const VolJob& J, const VolJob* jobs, int njobs, 
                       const rcv_volpath_options* o, unsigned long long* queue_counter, float4* path_out,
                       const AdjBuffers* adj, uint64_t* counters, cudaStream_t st, bool supergrid,
                       bool zeroed = false);
-// Paths that a warp claims per queue fetch when the caller gives no number: an
-// eighth of a warp's share of the launch, 2 to 64.  A warp that claims more
+// Paths that a warp claims per queue fetch: `most`, the caller's number (by
+// default 64), or in small launches an eighth of a warp's share, 2 at least.  A warp that claims more
 // than its share leaves others without work and walks its paths in turns; with
 // few paths per warp the cooperative walk sets in at once.  Paired launch of
 // 64^2 x (4 + 4) spp on 16^3, 128^2 on 32^3 and five 107 x 83 x (6 + 6) views,
 // us: 64 per fetch 292 / 346 / 1003, a whole share (8 at least) 176 / 241 /
 // 1003, half 169 / 194 / 835, a quarter 166 / 193 / 801, an eighth (2 at
-// least) 131 / 193 / 811; films of 1.9 M paths or more keep 64.
-int paths_per_fetch(int64_t total);
+// least) 131 / 193 / 811; launches of 1.9 M paths or more keep 64.
+int paths_per_fetch(int64_t total, int most = 64);
 // Work queue of a persistent tracer launch (the arguments of
 // launch_persistent); zeroes its hand-out counter on `st` unless that is
 // known to be zero.
