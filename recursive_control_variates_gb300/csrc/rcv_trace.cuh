@@ -109,8 +109,9 @@ constexpr int kTraceBlock = 32 * kTraceWarps;
 // step itself.  Positions, remaining distances, null-collision weights and
 // transmittances are accumulated in step order with the operations of the
 // regular step, so a path gives the same bits whether it walks alone or with
-// helpers.  `m` holds the walking lanes (at most 8: G = 32 / 16 / 8 / 4 for
-// 1 / 2 / 3-4 / 5-8 paths); `org`, `dir`, `tmax` are the walk's ray and
+// helpers.  `m` holds the walking lanes (at most 16: G = 32 / 16 / 8 / 4 / 2 for
+// 1 / 2 / 3-4 / 5-8 / 9-16 paths; a limit of 4 / 8 / 16 gave 822 / 766 / 711 us
+// for the paired launch of five 107 x 83 views, 202 / 181 / 180 us at 128^2); `org`, `dir`, `tmax` are the walk's ray and
 // remaining distance, `c1`, `c2` its throughputs (main: bn, bo) or
 // transmittances (shadow: trn, tro in .x); `s_t`, `s_w1`, `s_w2` are the
 // warp's 32-float shared arrays for the steps' distances and weights.
@@ -119,38 +120,45 @@ constexpr int kTraceBlock = 32 * kTraceWarps;
 // the lane that evaluated it appends to the tape with the owner's reference
 // `ref`; `lost` is set on an owner whose events did not fit.
 template <int kMode, bool kTable>
-__device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJob& single, const VolJob* Jp, Pcg32& rng, float mu,
-                                         float inv_mu, float half_inv_mu, V3& org, const V3& dir, float& tmax,
-                                         V3& c1, V3& c2, float* s_t, float* s_w1, float* s_w2, const Queue& Q,
-                                         TapeCursor& tc, uint32_t ref, bool& lost) {
+__device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJob& single, const VolJob* Jp,
+                                         Pcg32& rng, float mu, float inv_mu, float half_inv_mu, V3& org,
+                                         const V3& dir, float& tmax, V3& c1, V3& c2, float* s_t, float* s_w1,
+                                         float* s_w2, const Queue& Q, TapeCursor& tc, uint32_t ref, bool& lost) {
   constexpr unsigned kFull = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u;
   const int n = __popc(m);
-  const int G = n == 1 ? 32 : (n == 2 ? 16 : (n <= 4 ? 8 : 4));
+  const int G = coop_group(n);
   const int grp = (int)lane / G;
   const int k = (int)lane & (G - 1);
   const int base = grp * G;
   const bool busy = grp < n;
   // owner of this lane's group: the grp-th walking lane (lanes of idle groups
   // read their own registers and touch no memory)
-  unsigned mm = m;
-  for (int i = 0; i < grp && mm != 0u; ++i) mm &= mm - 1u;
-  const int owner = mm != 0u ? __ffs(mm) - 1 : (int)lane;
+  const int owner = coop_owner(m, grp, (int)lane);
 
   const bool g_main = __shfl_sync(kFull, (int)main_walk, owner) != 0;
   const VolJob& J = kTable ? *(const VolJob*)__shfl_sync(kFull, (unsigned long long)Jp, owner) : single;
   Pcg32 r;
   r.state = __shfl_sync(kFull, (unsigned long long)rng.state, owner);
   r.inc = __shfl_sync(kFull, (unsigned long long)rng.inc, owner);
-  const float g_mu = __shfl_sync(kFull, mu, owner);
-  const float g_inv = __shfl_sync(kFull, inv_mu, owner);
-  const float g_hinv = __shfl_sync(kFull, half_inv_mu, owner);
+  // (every path of a single job has its majorant)
+  const float g_mu = kTable ? __shfl_sync(kFull, mu, owner) : mu;
+  const float g_inv = kTable ? __shfl_sync(kFull, inv_mu, owner) : inv_mu;
+  const float g_hinv = kTable ? __shfl_sync(kFull, half_inv_mu, owner) : half_inv_mu;
+  // throughputs (transmittances in .x) before the group's first step
+  V3 b1{__shfl_sync(kFull, c1.x, owner), 0.0f, 0.0f}, b2{0.0f, 0.0f, 0.0f};
+  if (kMode == kTwoState) {
+    b1.y = __shfl_sync(kFull, c1.y, owner);
+    b1.z = __shfl_sync(kFull, c1.z, owner);
+    b2 = V3{__shfl_sync(kFull, c2.x, owner), __shfl_sync(kFull, c2.y, owner), __shfl_sync(kFull, c2.z, owner)};
+  }
   const V3 dv{__shfl_sync(kFull, dir.x, owner), __shfl_sync(kFull, dir.y, owner), __shfl_sync(kFull, dir.z, owner)};
   float px = __shfl_sync(kFull, org.x, owner), py = __shfl_sync(kFull, org.y, owner);
   float pz = __shfl_sync(kFull, org.z, owner), tr = __shfl_sync(kFull, tmax, owner);
 
   // this lane's step: its draws, distance and real/null variable
-  r.state = pcg_jump(r.state, r.inc, (g_main ? 3u : 1u) * (uint32_t)k);
+  const ulonglong2 jump = __ldg(reinterpret_cast<const ulonglong2*>(kCoopJumps.j) + (g_main ? 3 * k : k));
+  r.state = jump.x * r.state + jump.y * r.inc;
   if (g_main) pcg_skip1(r);  // roulette draw, unused below the roulette depth
   const float t = free_flight(next1d(r), g_mu, g_inv);
   const float ur = g_main ? next1d(r) : 0.0f;
@@ -179,7 +187,7 @@ __device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJo
     st_n = J.scale * rho_n;
   }
   bool term;
-  float w1 = 0.0f, w2 = 0.0f;  // main: null-collision weights (two-state); shadow: transmittance factors
+  float w1 = 1.0f, w2 = 1.0f;  // main: null-collision weights (two-state); shadow: transmittance factors
   if (g_main) {
     const float prob = kMode == kTwoState ? (st_n + st_o) * g_hinv : st_n * g_inv;
     term = !(valid && ur >= prob);
@@ -194,46 +202,37 @@ __device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJo
     if (kMode == kTwoState) w2 = (g_mu - st_o) * g_inv;
   }
   s_w1[lane] = w1;
-  s_w2[lane] = w2;
-  const unsigned tb_all = __ballot_sync(kFull, term);
+  if (kMode == kTwoState) s_w2[lane] = w2;
   __syncwarp();
+  // throughputs before and after this lane's step, in step order (the owner
+  // alone took them one after the other while the group waited); a step is
+  // not taken when the regular one would end the path before it (throughput
+  // zero) or the shadow walk with it (transmittance zero)
+#pragma unroll 4
+  for (int j = 0; j < k; ++j) {
+    const float x1 = s_w1[base + j];
+    b1.x *= x1;
+    if (kMode == kTwoState) {
+      const float x2 = s_w2[base + j];
+      b1.y *= x1;
+      b1.z *= x1;
+      b2 = V3{b2.x * x2, b2.y * x2, b2.z * x2};
+    }
+  }
+  if (kMode == kTwoState && g_main) term = term || !nonzero<kMode>(b1, b2);
+  b1 = V3{b1.x * w1, b1.y * w1, b1.z * w1};
+  if (kMode == kTwoState) b2 = V3{b2.x * w2, b2.y * w2, b2.z * w2};
+  if (!g_main) term = term || (b1.x == 0.0f && (kMode != kTwoState || b2.x == 0.0f));
+  const unsigned tb_all = __ballot_sync(kFull, term);
 
-  // the owner takes the steps before the first one that is not a null step
-  // (main) or that ends the shadow walk, with its throughputs (main) or
-  // transmittances (shadow) multiplied in step order
+  // the owner takes the steps before the first one that is not
   const bool own = (m >> lane) & 1u;
   int f = 0, src = (int)lane;
   const int ob = __popc(m & ((1u << lane) - 1u)) * G;
   const unsigned gmask = G == 32 ? kFull : ((1u << G) - 1u);
   if (own) {
     const unsigned tb = (tb_all >> ob) & gmask;
-    const int f0 = tb != 0u ? __ffs(tb) - 1 : G;
-    f = f0;
-    for (int j = 0; j < f0; ++j) {
-      const float x1 = s_w1[ob + j], x2 = s_w2[ob + j];
-      if (main_walk) {
-        // the regular step begins with the roulette's throughput test
-        bool alive = c1.x != 0.0f || c1.y != 0.0f || c1.z != 0.0f;
-        if (kMode == kTwoState) alive = alive || (c2.x != 0.0f || c2.y != 0.0f || c2.z != 0.0f);
-        if (!alive) {
-          f = j;
-          break;
-        }
-        if (kMode == kTwoState) {
-          c1 = V3{c1.x * x1, c1.y * x1, c1.z * x1};
-          c2 = V3{c2.x * x2, c2.y * x2, c2.z * x2};
-        }
-      } else {
-        const float n1 = c1.x * x1, n2 = c2.x * x2;
-        const bool done = kMode == kTwoState ? (n1 == 0.0f && n2 == 0.0f) : n1 == 0.0f;
-        if (done) {
-          f = j;  // the regular step takes this step and ends the walk
-          break;
-        }
-        c1.x = n1;
-        if (kMode == kTwoState) c2.x = n2;
-      }
-    }
+    f = tb != 0u ? __ffs(tb) - 1 : G;
     if (f > 0) src = ob + f - 1;
   }
   // state after f steps: position, remaining distance and stream after step
@@ -241,6 +240,12 @@ __device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJo
   const V3 xs{__shfl_sync(kFull, x.x, src), __shfl_sync(kFull, x.y, src), __shfl_sync(kFull, x.z, src)};
   const float ts = __shfl_sync(kFull, tr - t, src);
   const unsigned long long ss = __shfl_sync(kFull, (unsigned long long)r.state, src);
+  b1.x = __shfl_sync(kFull, b1.x, src);
+  if (kMode == kTwoState) {
+    b1.y = __shfl_sync(kFull, b1.y, src);
+    b1.z = __shfl_sync(kFull, b1.z, src);
+    b2 = V3{__shfl_sync(kFull, b2.x, src), __shfl_sync(kFull, b2.y, src), __shfl_sync(kFull, b2.z, src)};
+  }
   if (kMode == kTape) {
     // the group's steps before the first that ends the run are events
     const int fg = __shfl_sync(kFull, f, owner);
@@ -254,6 +259,14 @@ __device__ __forceinline__ int coop_walk(unsigned m, bool main_walk, const VolJo
   org = xs;
   tmax = ts;
   rng.state = ss;
+  c1.x = b1.x;
+  if (kMode == kTwoState) {
+    c2.x = b2.x;
+    if (main_walk) {
+      c1 = b1;
+      c2 = b2;
+    }
+  }
   return f;
 }
 
@@ -695,7 +708,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       }
       const unsigned m_coop = __ballot_sync(0xffffffffu, elig);
       const int n_coop = __popc(m_coop);
-      if (n_coop >= 1 && n_coop <= 8) {
+      if (n_coop >= 1 && n_coop <= kCoopMost) {
         const bool mw = phase == kMain;
         float* s = s_coop + (threadIdx.x >> 5) * 96;
         const int f = coop_walk<kMode, kTable>(m_coop, mw, single, Jp, rng, mu, inv_mu, 0.5f * inv_mu, x, dir, rem, bn,

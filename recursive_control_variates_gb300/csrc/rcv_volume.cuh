@@ -225,6 +225,22 @@ __device__ __forceinline__ void tape_close(const Queue& Q, const TapeCursor& tc)
     __stcs(Q.tape + i, make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(kTapeEmpty)));
 }
 
+// The jumps of the cooperative walk's lanes (up to 3 x 31 draws), read through
+// the L1: 16 bytes per lane instead of up to seven rounds of 64-bit squarings.
+static __device__ const PcgJumpTable kCoopJumps = make_pcg_jumps();
+
+// Lanes per path of a cooperative walk of n paths.
+constexpr int kCoopMost = 16;
+__device__ __forceinline__ int coop_group(int n) {
+  return n == 1 ? 32 : (n == 2 ? 16 : (n <= 4 ? 8 : (n <= 8 ? 4 : 2)));
+}
+
+// Owner of group `grp`: the grp-th lane of m, or the lane itself.
+__device__ __forceinline__ int coop_owner(unsigned m, int grp, int lane) {
+  for (int i = 0; i < grp && m != 0u; ++i) m &= m - 1u;
+  return m != 0u ? __ffs(m) - 1 : lane;
+}
+
 // Buffers of the two adjoint launches.
 struct AdjBuffers {
   float4* ckpt;

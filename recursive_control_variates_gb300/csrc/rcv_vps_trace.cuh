@@ -65,6 +65,91 @@ __device__ __forceinline__ uint32_t vps_sid(const VolJob& J, uint32_t path, int&
   return (uint32_t)pix * (uint32_t)J.spp + (local - k * (uint32_t)J.spp);
 }
 
+// Cooperative walk of a warp's last paths (see coop_walk in rcv_trace.cuh):
+// groups of lanes take the next steps of one path each, with this tracer's two
+// draws per main step, its quotients and its walked distance `acc` (of a shadow
+// walk: its transmittance).
+template <int kMode>
+__device__ __forceinline__ void vps_coop(unsigned m, bool main_walk, const VolJob& J, Pcg32& rng, float mu,
+                                         float inv_mu, V3& org, const V3& dir, float& tmax, float& acc, float* s_t,
+                                         float* s_w, const Queue& Q, TapeCursor& tc, uint32_t rec, bool& lost) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const unsigned lane = threadIdx.x & 31u;
+  const int n = __popc(m), G = coop_group(n);
+  const int grp = (int)lane / G, k = (int)lane & (G - 1), base = grp * G;
+  const bool busy = grp < n;
+  const int owner = coop_owner(m, grp, (int)lane);
+  const bool g_main = __shfl_sync(kFull, (int)main_walk, owner) != 0;
+  Pcg32 r;
+  r.state = __shfl_sync(kFull, (unsigned long long)rng.state, owner);
+  r.inc = __shfl_sync(kFull, (unsigned long long)rng.inc, owner);
+  const V3 dv{__shfl_sync(kFull, dir.x, owner), __shfl_sync(kFull, dir.y, owner), __shfl_sync(kFull, dir.z, owner)};
+  float px = __shfl_sync(kFull, org.x, owner), py = __shfl_sync(kFull, org.y, owner);
+  float pz = __shfl_sync(kFull, org.z, owner), tr = __shfl_sync(kFull, tmax, owner);
+  float a = __shfl_sync(kFull, acc, owner);
+
+  const ulonglong2 jump = __ldg(reinterpret_cast<const ulonglong2*>(kCoopJumps.j) + (g_main ? 2 * k : k));
+  r.state = jump.x * r.state + jump.y * r.inc;
+  const float t = free_flight(next1d(r), mu, inv_mu);
+  const float ur = g_main ? next1d(r) : 0.0f;
+  s_t[lane] = t;
+  __syncwarp();
+#pragma unroll 4
+  for (int j = 0; j < k; ++j) {
+    const float tj = s_t[base + j];
+    px = fmaf(tj, dv.x, px);
+    py = fmaf(tj, dv.y, py);
+    pz = fmaf(tj, dv.z, pz);
+    tr = tr - tj;
+    if (g_main) a = a + tj;
+  }
+  const bool valid = busy && t <= tr;
+  const V3 x{fmaf(t, dv.x, px), fmaf(t, dv.y, py), fmaf(t, dv.z, pz)};
+  const float st = valid ? J.scale * density_new(J, locate(J, x)) : 0.0f;
+  const float sn = mu - st;
+  bool term = !valid;
+  float w = 1.0f;
+  if (g_main)
+    term = term || ur < (mu != 0.0f ? div_by(st, mu, inv_mu) : 0.0f);
+  else
+    w = mu != 0.0f ? div_by(sn, mu, inv_mu) : sn;
+  s_w[lane] = w;
+  __syncwarp();
+  if (!g_main) {
+#pragma unroll 4
+    for (int j = 0; j < k; ++j) a *= s_w[base + j];
+  }
+  a = g_main ? a + t : a * w;
+  term = term || (!g_main && a == 0.0f);
+  const unsigned tb_all = __ballot_sync(kFull, term);
+
+  const bool own = (m >> lane) & 1u;
+  const int ob = __popc(m & ((1u << lane) - 1u)) * G;
+  const unsigned gmask = G == 32 ? kFull : ((1u << G) - 1u);
+  int f = 0, src = (int)lane;
+  if (own) {
+    const unsigned tb = (tb_all >> ob) & gmask;
+    f = tb != 0u ? __ffs(tb) - 1 : G;
+    if (f > 0) src = ob + f - 1;
+  }
+  const V3 xs{__shfl_sync(kFull, x.x, src), __shfl_sync(kFull, x.y, src), __shfl_sync(kFull, x.z, src)};
+  const float ts = __shfl_sync(kFull, tr - t, src), as = __shfl_sync(kFull, a, src);
+  const unsigned long long ss = __shfl_sync(kFull, (unsigned long long)r.state, src);
+  if (kMode == kVpsTape) {
+    const int fg = __shfl_sync(kFull, f, owner);
+    const uint32_t rg = __shfl_sync(kFull, rec, owner);
+    const bool kept = __shfl_sync(kFull, (int)lost, owner) == 0;
+    const bool ok = tape_append(Q, tc, busy && kept && k < fg && !g_main && w > 0.0f, x, rg, sn);
+    const unsigned bad = __ballot_sync(kFull, !ok);
+    if (own && ((bad >> ob) & gmask) != 0u) lost = true;
+  }
+  if (f == 0) return;
+  org = xs;
+  tmax = ts;
+  acc = as;
+  rng.state = ss;
+}
+
 template <int kMode, bool kSG, bool kEnv>
 __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
   constexpr bool kDrt = kMode == kVpsDrt;
@@ -82,6 +167,7 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
   constexpr int cTask = 0, cNee = 1, cDist = 4;
   constexpr int cEnv = kDrt ? 5 : 13;
 
+  __shared__ float s_coop[kSG ? 1 : kVpsWarps * 64];
   const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
   const unsigned defer = (unsigned)Q.defer;
   const float mu = J.scale * bits_to_float(__ldg(J.maxbits + 1)), inv_mu = 1.0f / mu;
@@ -360,6 +446,15 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
         acc = 0.0f;
         if (!kDrt) F(cMax) = rem;
         phase = kVMain;
+      }
+    }
+
+    // ------------------------------ cooperative walk of the warp's last paths
+    if (!kSG && queue_empty) {
+      const unsigned m_coop = __ballot_sync(0xffffffffu, !finished && (phase == kVMain || phase == kVNee));
+      if (m_coop != 0u && __popc(m_coop) <= kCoopMost) {
+        float* s = s_coop + (threadIdx.x >> 5) * 64;
+        vps_coop<kMode>(m_coop, phase == kVMain, J, rng, mu, inv_mu, p, w, rem, acc, s, s + 32, Q, tc, rec, lost);
       }
     }
 
