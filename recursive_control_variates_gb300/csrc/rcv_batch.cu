@@ -517,6 +517,7 @@ extern "C" int rcv_batch_job_init(const rcv_batch_job* job, void* stream) {
   if (rc) return rc;
   OrderJob O;
   O.J = J;
+  O.head = nullptr;
   O.npix = J.width * J.height;
   O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
   O.order = reinterpret_cast<uint32_t*>(ws + L.order);

@@ -74,8 +74,17 @@ __global__ void tape_weights_kernel(const __grid_constant__ VolJob single, const
                                     float4* __restrict__ w, const float4* __restrict__ ltot,
                                     const uint32_t* __restrict__ entered, float2* __restrict__ cam_w,
                                     const unsigned long long* __restrict__ entered_count,
-                                    unsigned long long* replay_counter) {
+                                    int64_t clear_cells, int64_t clear_albedo, unsigned long long* replay_counter) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *replay_counter = 0ull;
+  // the gradient records, for the scatter that follows (a clear of their own
+  // cost a launch each)
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < clear_cells;
+       i += int64_t(gridDim.x) * blockDim.x)
+    single.grad_cells[i] = zero;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < clear_albedo;
+       i += int64_t(gridDim.x) * blockDim.x)
+    single.grad_albedo[i] = zero;
   const int64_t paths = (int64_t)*entered_count;
   const int64_t nrec = min((int64_t)*rec_count, rec_cap);
   const int64_t n = max(nrec, paths);
@@ -179,10 +188,11 @@ int launch_tape_gradient(const VolJob& single, const VolJob* jobs, int njobs, co
                          unsigned long long* replay_counter, uint64_t* counters, int sms, cudaStream_t st) {
   const int block = 256;
   // grid-stride: the numbers of records and paths are known on the device only
-  const unsigned need = grid_for(A.ckpt_cap, block), most = (unsigned)(sms > 0 ? sms : 1) * 16u;
+  const unsigned need = grid_for(A.ckpt_cap + A.clear_cells, block), most = (unsigned)(sms > 0 ? sms : 1) * 16u;
   tape_weights_kernel<<<need < most ? need : most, block, 0, st>>>(single, jobs, njobs, A.ckpt, A.ckpt_count,
                                                                    A.ckpt_cap, weights, A.path_ltot, A.entered,
-                                                                   A.cam_w, A.entered_count, replay_counter);
+                                                                   A.cam_w, A.entered_count, A.clear_cells,
+                                                                   A.clear_albedo, replay_counter);
   int rc = launched("tape_weights launch");
   if (rc) return rc;
   const unsigned grid = (unsigned)(sms > 0 ? sms : 1) * 8u;

@@ -256,6 +256,9 @@ struct AdjBuffers {
   uint32_t* entered;  // paths that entered the medium
   unsigned long long* entered_count;
   float2* cam_w;  // their camera segments' weights
+  // gradient records that the weights pass clears (single jobs; a batch clears
+  // them as it packs): float4s of the density's and of the albedo's
+  int64_t clear_cells, clear_albedo;
 };
 
 struct Counts {
@@ -546,15 +549,18 @@ int make_volume_job(const rcv_medium* m, const rcv_sensor* s, const rcv_volpath_
 // Pixel hand-out of one job: `order` receives its pixels, most expensive
 // first, by `cost` (the per-pixel path lengths of the previous call, cleared
 // here) or, when cost is null, by the chord length of the pixel's centre ray
-// through the medium.  buckets: 2 x 256 zeroed uint32 of scratch.
+// through the medium.  head: the workspace's head (kRenderHeadBytes), cleared
+// before, or null when the caller cleared the buckets.  buckets: 2 x 256 uint32
+// of scratch.
 struct OrderJob {
   VolJob J;
+  void* head;
   int32_t npix;
   uint32_t* buckets;
   uint32_t* order;
   uint32_t* cost;
 };
-// Orders the pixels of one job or of two, in the same two launches.
+// Orders the pixels of one job or of two, in the same launches.
 int order_pixels(const OrderJob* jobs, int n, cudaStream_t st);
 // Clears the medium workspace's cell (and albedo) gradient accumulators.
 int reset_gradients(const rcv_medium* m, bool albedo, cudaStream_t st);

@@ -632,11 +632,11 @@ static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, cha
     // call would order a little better but would tie the scratch to the caller
     OrderJob O;
     O.J = J;
+    O.head = ws;
     O.npix = (int32_t)npix;
     O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
     O.order = reinterpret_cast<uint32_t*>(ws + L.order);
     O.cost = nullptr;
-    RCV_TRY_CUDA(cudaMemsetAsync(ws, 0, kRenderHeadBytes, st), "counters reset");
     rc = order_pixels(&O, 1, st);
     if (rc) return rc;
     J.pixel_order = O.order;

@@ -7,9 +7,11 @@
 // launch took 13.1 ms at a few lanes per instruction.  Here the adjoint is
 // two persistent launches with one free-flight step per loop iteration for
 // every lane, whatever its phase (as in rcv_trace.cuh), and two flat passes;
-// on the same film 1.14 + 0.88 + 0.26 + 0.11 ms (GB300).  The tracers are
+// on the same film 0.94 + 0.80 + 0.26 + 0.11 ms (GB300).  The tracers are
 // bound by the issue of divergent instructions and end on their longest
-// paths, the flat passes by the vector reductions into the gradient:
+// paths (a DRT path that follows its first path in the same lane and launch
+// gives 2.0 ms for the two tracers), the flat passes by the vector reductions
+// into the gradient:
 //   kVpsTape  traces each path once.  It records every segment (64 bytes:
 //             the path, the NEE radiance gathered before it, its ray, its
 //             length, the NEE contribution at its end) and every step of a
