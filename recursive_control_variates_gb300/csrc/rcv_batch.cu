@@ -181,22 +181,18 @@ __global__ void batch_pack_kernel(const BatchEntry* __restrict__ E, const int32_
   const float* nd = B.d.density[cur];
   const float* od = B.d.density[cur ^ 1];
   const int dx = B.d.dims[0], dy = B.d.dims[1], dz = B.d.dims[2];
-  float mo = 0.0f, mn = 0.0f;
+  float mo, mn;
+  pack_cells(i, B.nc, dx, dy, dz, od, nd, B.cells, mo, mn);
   if (i < B.nc) {
-    pack_cell(i, dx, dy, dz, od, nd, B.cells);
-    B.grad_cells[i * 2 + 0] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    B.grad_cells[i * 2 + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    store_pair(B.grad_cells + i * 2, zero, zero);
     if (B.opt_albedo) {
       // the albedo grid has the density's resolution: one 6-float4 record per cell
 #pragma unroll
-      for (int q = 0; q < 6; ++q) B.grad_albedo[i * 6 + q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      for (int q = 0; q < 6; q += 2) store_pair(B.grad_albedo + i * 6 + q, zero, zero);
     }
   }
-  if (i < B.nv) {
-    mo = od[i];
-    mn = nd[i];
-    if (B.has_albedo) pack_albedo(i, B.d.albedo[cur ^ 1], B.d.albedo[cur], B.albedo);
-  }
+  if (i < B.nv && B.has_albedo) pack_albedo(i, B.d.albedo[cur ^ 1], B.d.albedo[cur], B.albedo);
   reduce_majorants(mo, mn, B.maxbits);
 }
 
@@ -313,7 +309,9 @@ __global__ void batch_update_kernel(const BatchEntry* __restrict__ E, const int3
   const float b1 = B.d.adam_beta1, b2 = B.d.adam_beta2, eps = B.d.adam_eps;
   const float omb1 = 1.0f - b1, omb2 = 1.0f - b2;
   // the single-job path accumulates the fold into a zeroed gradient: 0 + g
-  const float g = 0.0f + fold_voxel(i, B.d.dims[0], B.d.dims[1], B.d.dims[2],
+  int x, y, z;
+  voxel_of(i, B.d.dims[0], B.d.dims[1], x, y, z);
+  const float g = 0.0f + fold_voxel(x, y, z, B.d.dims[0], B.d.dims[1], B.d.dims[2],
                                     reinterpret_cast<const float*>(B.grad_cells));
   {
     float m = B.d.density_m[i], v = B.d.density_v[i];
@@ -323,7 +321,7 @@ __global__ void batch_update_kernel(const BatchEntry* __restrict__ E, const int3
     B.d.density_v[i] = v;
   }
   if (B.opt_albedo) {
-    const V3 ga = fold_voxel_rgb(i, B.d.dims[0], B.d.dims[1], B.d.dims[2],
+    const V3 ga = fold_voxel_rgb(x, y, z, B.d.dims[0], B.d.dims[1], B.d.dims[2],
                                  reinterpret_cast<const float*>(B.grad_albedo));
     const float gs[3] = {0.0f + ga.x, 0.0f + ga.y, 0.0f + ga.z};
     const float* pin = B.d.albedo[cur];

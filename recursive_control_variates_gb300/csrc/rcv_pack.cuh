@@ -7,29 +7,46 @@
 
 namespace rcv {
 
-// Cell i of a (dx+1)(dy+1)(dz+1) lattice: the 8 clamped corner voxels of the
+// Cells of a (dx+1)(dy+1)(dz+1) lattice: the 8 clamped corner voxels of the
 // old and the new density, x pairs as value and difference (trilerp_diff).
+// Called by whole warps with consecutive i, one cell per lane (none from nc
+// on); mo and mn receive maxima of voxels of the old and of the new density,
+// which over all cells cover every voxel.
+// Bound by the stores, 64 bytes per cell.  Two lanes write a cell, one per
+// state, so that a warp's store is 1024 consecutive bytes (256^3: 200 us, 6.1
+// TB/s); a lane that wrote its own cell in two such stores took 243 us, in
+// four of 16 bytes, half sectors of 32 lines each, 309.
 // 32-bit index arithmetic: 4 (dx+1)(dy+1)(dz+1) < 2^32 is enforced on the host.
-__device__ __forceinline__ void pack_cell(int64_t i, int dx, int dy, int dz, const float* __restrict__ old_d,
-                                          const float* __restrict__ new_d, float4* __restrict__ cells) {
+__device__ __forceinline__ void pack_cells(int64_t i, int64_t nc, int dx, int dy, int dz,
+                                           const float* __restrict__ old_d, const float* __restrict__ new_d,
+                                           float4* __restrict__ cells, float& mo, float& mn) {
   const uint32_t ex = (uint32_t)(dx + 1), ey = (uint32_t)(dy + 1);
-  const uint32_t row = (uint32_t)i / ex;
-  const int cx = int((uint32_t)i - row * ex);
-  const uint32_t cz_u = row / ey;
-  const int cy = int(row - cz_u * ey);
-  const int cz = int(cz_u);
-  const int x0 = clampi(cx - 1, dx - 1), x1 = clampi(cx, dx - 1);
-  const int y0 = clampi(cy - 1, dy - 1), y1 = clampi(cy, dy - 1);
-  const int z0 = clampi(cz - 1, dz - 1), z1 = clampi(cz, dz - 1);
-  auto idx = [&](int x, int y, int z) { return (int64_t(z) * dy + y) * dx + x; };
-  const int64_t i000 = idx(x0, y0, z0), i100 = idx(x1, y0, z0), i010 = idx(x0, y1, z0), i110 = idx(x1, y1, z0),
-                i001 = idx(x0, y0, z1), i101 = idx(x1, y0, z1), i011 = idx(x0, y1, z1), i111 = idx(x1, y1, z1);
-  float4* c = cells + i * 4;
-  const auto pairs = [](float a0, float a1, float b0, float b1) { return make_float4(a0, a1 - a0, b0, b1 - b0); };
-  c[0] = pairs(old_d[i000], old_d[i100], old_d[i010], old_d[i110]);
-  c[1] = pairs(old_d[i001], old_d[i101], old_d[i011], old_d[i111]);
-  c[2] = pairs(new_d[i000], new_d[i100], new_d[i010], new_d[i110]);
-  c[3] = pairs(new_d[i001], new_d[i101], new_d[i011], new_d[i111]);
+  const int lane = threadIdx.x & 31, state = lane & 1;
+  const float* __restrict__ d = state ? new_d : old_d;
+  float m = 0.0f;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int64_t c = i - lane + 16 * half + (lane >> 1);
+    if (c >= nc) break;
+    const uint32_t row = (uint32_t)c / ex;
+    const int cx = int((uint32_t)c - row * ex);
+    const uint32_t cz_u = row / ey;
+    const int cy = int(row - cz_u * ey), cz = int(cz_u);
+    const uint32_t x0 = (uint32_t)clampi(cx - 1, dx - 1), x1 = (uint32_t)clampi(cx, dx - 1);
+    const uint32_t y0 = (uint32_t)clampi(cy - 1, dy - 1), y1 = (uint32_t)clampi(cy, dy - 1);
+    const uint32_t z0 = (uint32_t)clampi(cz - 1, dz - 1) * (uint32_t)dy,
+                   z1 = (uint32_t)clampi(cz, dz - 1) * (uint32_t)dy;
+    const auto pairs = [&](uint32_t r0, uint32_t r1) {  // rows of the corners
+      const float a0 = d[r0 + x0], a1 = d[r0 + x1], b0 = d[r1 + x0], b1 = d[r1 + x1];
+      m = fmaxf(m, fmaxf(fmaxf(a0, a1), fmaxf(b0, b1)));
+      return make_float4(a0, a1 - a0, b0, b1 - b0);
+    };
+    const float4 lo = pairs((z0 + y0) * (uint32_t)dx, (z0 + y1) * (uint32_t)dx);
+    const float4 hi = pairs((z1 + y0) * (uint32_t)dx, (z1 + y1) * (uint32_t)dx);
+    store_pair(cells + c * 4 + 2 * state, lo, hi);
+  }
+  mo = state ? 0.0f : m;
+  mn = state ? m : 0.0f;
 }
 
 // Voxels whose trilinear weight can be non-zero inside supergrid cell c of
@@ -78,8 +95,8 @@ __device__ __forceinline__ void supergrid_cell(int64_t i, const int sg[3], int d
 // Voxel i of the old and the new RGB albedo as one 32-byte pair.
 __device__ __forceinline__ void pack_albedo(int64_t i, const float* __restrict__ old_a,
                                             const float* __restrict__ new_a, float4* __restrict__ albedo) {
-  albedo[i * 2 + 0] = make_float4(old_a[i * 3 + 0], old_a[i * 3 + 1], old_a[i * 3 + 2], 0.0f);
-  albedo[i * 2 + 1] = make_float4(new_a[i * 3 + 0], new_a[i * 3 + 1], new_a[i * 3 + 2], 0.0f);
+  store_pair(albedo + i * 2, make_float4(old_a[i * 3 + 0], old_a[i * 3 + 1], old_a[i * 3 + 2], 0.0f),
+             make_float4(new_a[i * 3 + 0], new_a[i * 3 + 1], new_a[i * 3 + 2], 0.0f));
 }
 
 // Sum of a pixel's per-path radiance slots in sample order, divided by spp
@@ -181,64 +198,66 @@ __device__ __forceinline__ bool fold_uses(int c, int bit, int v, int D) {
   return c <= D && clampi(c - 1 + bit, D - 1) == v;
 }
 
-// Gradient of voxel i: the sum of its corner entries in every cell that uses
-// it, in the order z, y, x candidate, each by cell and then corner bit.  The
-// candidate slots are fixed (cell v or v + 1, bit 0 or 1) and unrolled, so
-// everything stays in registers.
-__device__ __forceinline__ float fold_voxel(int64_t i, int dx, int dy, int dz, const float* __restrict__ gcells) {
-  // 32-bit index arithmetic (the voxel count is below the cell count, < 2^30)
-  const uint32_t row = (uint32_t)i / (uint32_t)dx;
-  const int x = int((uint32_t)i - row * (uint32_t)dx);
-  const uint32_t z_u = row / (uint32_t)dy;
-  const int y = int(row - z_u * (uint32_t)dy), z = int(z_u);
-  float g = 0.0f;
-#pragma unroll
-  for (int kz = 0; kz < 4; ++kz) {
-    const int cz = z + (kz >> 1), bz = kz & 1;
-    if (!fold_uses(cz, bz, z, dz)) continue;
-#pragma unroll
-    for (int ky = 0; ky < 4; ++ky) {
-      const int cy = y + (ky >> 1), by = ky & 1;
-      if (!fold_uses(cy, by, y, dy)) continue;
-#pragma unroll
-      for (int kx = 0; kx < 4; ++kx) {
-        const int cx = x + (kx >> 1), bx = kx & 1;
-        if (!fold_uses(cx, bx, x, dx)) continue;
-        const int64_t cell = (int64_t(cz) * (dy + 1) + cy) * (dx + 1) + cx;
-        g += gcells[cell * 8 + bx + 2 * by + 4 * bz];
-      }
-    }
+// Calls f(entry) with the address of each corner entry (C floats; 8 per cell)
+// of voxel (x, y, z), in the order z, y, x candidate, each by cell and then
+// corner bit.  Along an axis those are the cell's corner 1 and the next one's
+// corner 0, and at the grid's faces, where cells clamp, the other corners.
+// The x faces are two predicated entries (one lane of a warp has one); trying
+// all 64 candidate slots for every voxel was bound by their tests, a branch
+// for inner voxels by its divergence (256^3, with the tiles of
+// fold_density_kernel: 194 -> 148 us; 96-byte records of 64^3: 13.7 -> 13.4).
+template <int C, class F>
+__device__ __forceinline__ void fold_entries(int x, int y, int z, int dx, int dy, int dz,
+                                             const float* __restrict__ gcells, F f) {
+  const int64_t row = int64_t(dx + 1) * (8 * C), plane = row * (dy + 1);
+  const float* own = gcells + z * plane + y * row + int64_t(x) * (8 * C);
+  const auto along_x = [&](const float* r) {
+    if (x == 0) f(r);
+    f(r + C);
+    f(r + 8 * C);
+    if (x == dx - 1) f(r + 9 * C);
+  };
+  if (y > 0 && y < dy - 1 && z > 0 && z < dz - 1) {
+    along_x(own + 6 * C);
+    along_x(own + row + 4 * C);
+    along_x(own + plane + 2 * C);
+    along_x(own + plane + row);
+    return;
   }
+  for (int kz = 0; kz < 4; ++kz) {
+    if (!fold_uses(z + (kz >> 1), kz & 1, z, dz)) continue;
+    for (int ky = 0; ky < 4; ++ky)
+      if (fold_uses(y + (ky >> 1), ky & 1, y, dy))
+        along_x(own + (kz >> 1) * plane + (ky >> 1) * row + (2 * (ky & 1) + 4 * (kz & 1)) * C);
+  }
+}
+
+// Voxel i of a grid (32-bit index arithmetic: fewer than 2^30 voxels).
+__device__ __forceinline__ void voxel_of(int64_t i, int dx, int dy, int& x, int& y, int& z) {
+  const uint32_t row = (uint32_t)i / (uint32_t)dx;
+  x = int((uint32_t)i - row * (uint32_t)dx);
+  const uint32_t z_u = row / (uint32_t)dy;
+  y = int(row - z_u * (uint32_t)dy);
+  z = int(z_u);
+}
+
+// Gradient of a voxel: the sum of its corner entries (8 floats per cell).
+__device__ __forceinline__ float fold_voxel(int x, int y, int z, int dx, int dy, int dz,
+                                            const float* __restrict__ gcells) {
+  float g = 0.0f;
+  fold_entries<1>(x, y, z, dx, dy, dz, gcells, [&](const float* r) { g += *r; });
   return g;
 }
 
-// RGB gradient of albedo voxel i from the albedo cell records (24 floats per
+// RGB gradient of an albedo voxel from the albedo cell records (24 floats per
 // cell: corner k = bx + 2 by + 4 bz, then R, G, B), summed in the order of
 // fold_voxel.
-__device__ __forceinline__ V3 fold_voxel_rgb(int64_t i, int dx, int dy, int dz, const float* __restrict__ gcells) {
-  const uint32_t row = (uint32_t)i / (uint32_t)dx;
-  const int x = int((uint32_t)i - row * (uint32_t)dx);
-  const uint32_t z_u = row / (uint32_t)dy;
-  const int y = int(row - z_u * (uint32_t)dy), z = int(z_u);
+__device__ __forceinline__ V3 fold_voxel_rgb(int x, int y, int z, int dx, int dy, int dz,
+                                             const float* __restrict__ gcells) {
   V3 g{0.0f, 0.0f, 0.0f};
-#pragma unroll
-  for (int kz = 0; kz < 4; ++kz) {
-    const int cz = z + (kz >> 1), bz = kz & 1;
-    if (!fold_uses(cz, bz, z, dz)) continue;
-#pragma unroll
-    for (int ky = 0; ky < 4; ++ky) {
-      const int cy = y + (ky >> 1), by = ky & 1;
-      if (!fold_uses(cy, by, y, dy)) continue;
-#pragma unroll
-      for (int kx = 0; kx < 4; ++kx) {
-        const int cx = x + (kx >> 1), bx = kx & 1;
-        if (!fold_uses(cx, bx, x, dx)) continue;
-        const int64_t cell = (int64_t(cz) * (dy + 1) + cy) * (dx + 1) + cx;
-        const float* r = gcells + cell * 24 + (bx + 2 * by + 4 * bz) * 3;
-        g = V3{g.x + r[0], g.y + r[1], g.z + r[2]};
-      }
-    }
-  }
+  fold_entries<3>(x, y, z, dx, dy, dz, gcells, [&](const float* r) {
+    g = V3{g.x + r[0], g.y + r[1], g.z + r[2]};
+  });
   return g;
 }
 

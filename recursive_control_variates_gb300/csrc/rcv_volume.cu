@@ -15,20 +15,15 @@
 namespace rcv {
 
 // ------------------------------------------------------------------ packing
-// One thread per cell / voxel / albedo voxel (na: albedo grid voxels).
+// One thread per cell / albedo voxel (na: albedo grid voxels).
 __global__ void pack_medium_kernel(int dx, int dy, int dz, const float* __restrict__ old_d,
                                    const float* __restrict__ new_d, float4* __restrict__ cells,
                                    const float* __restrict__ old_a, const float* __restrict__ new_a,
                                    float4* __restrict__ albedo, int64_t na, uint32_t* __restrict__ maxbits) {
   const int64_t nc = int64_t(dx + 1) * (dy + 1) * (dz + 1);
-  const int64_t nv = int64_t(dx) * dy * dz;
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  float mo = 0.0f, mn = 0.0f;
-  if (i < nc) pack_cell(i, dx, dy, dz, old_d, new_d, cells);
-  if (i < nv) {
-    mo = old_d[i];
-    mn = new_d[i];
-  }
+  float mo, mn;
+  pack_cells(i, nc, dx, dy, dz, old_d, new_d, cells, mo, mn);
   if (albedo != nullptr && i < na) pack_albedo(i, old_a, new_a, albedo);
   // majorant: maximum density of each state (non-negative part)
   reduce_majorants(mo, mn, maxbits);
@@ -179,23 +174,47 @@ __global__ void __launch_bounds__(kReduceBlock) reduce_paths_kernel(const float4
 }
 
 // ------------------------------------------------------------ gradient fold
-__global__ void fold_density_kernel(int dx, int dy, int dz, const float* __restrict__ gcells,
-                                    float* __restrict__ grad) {
-  const int64_t nv = int64_t(dx) * dy * dz;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  grad[i] += fold_voxel(i, dx, dy, dz, gcells);
+// Blocks take tiles of kFoldX x kFoldY x kFoldZ voxels, so that the cells that
+// neighbouring rows share come from the L1 (256^3: 148 us, 4.1 TB/s of records
+// read once; in runs of 256 voxels of one row 215, in tiles of 32 x 4 x 4 171;
+// 32 x 4 x 2 and 32 x 2 x 1 as good).  A lane that took its neighbour's corner
+// by a shuffle in place of a load was slower (214 to 243).
+constexpr int kFoldX = 32, kFoldY = 2, kFoldZ = 2, kFoldBlock = kFoldX * kFoldY * kFoldZ;
+
+static unsigned fold_grid(const int32_t d[3]) {
+  // ceil per axis in 64 bits; fewer than 2^30 voxels, so the product fits
+  return unsigned(((int64_t(d[0]) + kFoldX - 1) / kFoldX) * ((int64_t(d[1]) + kFoldY - 1) / kFoldY) *
+                  ((int64_t(d[2]) + kFoldZ - 1) / kFoldZ));
 }
 
-__global__ void fold_albedo_kernel(int adx, int ady, int adz, const float* __restrict__ gcells,
-                                   float* __restrict__ grad) {
-  const int64_t nv = int64_t(adx) * ady * adz;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  const V3 g = fold_voxel_rgb(i, adx, ady, adz, gcells);
-  grad[i * 3 + 0] += g.x;
-  grad[i * 3 + 1] += g.y;
-  grad[i * 3 + 2] += g.z;
+// The block's voxel of this thread; false outside the grid.
+__device__ __forceinline__ bool fold_tile(int dx, int dy, int dz, int& x, int& y, int& z) {
+  const uint32_t nx = (uint32_t(dx) + kFoldX - 1) / kFoldX, ny = (uint32_t(dy) + kFoldY - 1) / kFoldY;
+  const uint32_t row = blockIdx.x / nx, plane = row / ny;
+  x = int(blockIdx.x - row * nx) * kFoldX + int(threadIdx.x % kFoldX);
+  y = int(row - plane * ny) * kFoldY + int(threadIdx.x / kFoldX % kFoldY);
+  z = int(plane) * kFoldZ + int(threadIdx.x / (kFoldX * kFoldY));
+  return x < dx && y < dy && z < dz;
+}
+
+__global__ void __launch_bounds__(kFoldBlock) fold_density_kernel(int dx, int dy, int dz,
+                                                                  const float* __restrict__ gcells,
+                                                                  float* __restrict__ grad) {
+  int x, y, z;
+  if (!fold_tile(dx, dy, dz, x, y, z)) return;
+  grad[(int64_t(z) * dy + y) * dx + x] += fold_voxel(x, y, z, dx, dy, dz, gcells);
+}
+
+__global__ void __launch_bounds__(kFoldBlock) fold_albedo_kernel(int adx, int ady, int adz,
+                                                                 const float* __restrict__ gcells,
+                                                                 float* __restrict__ grad) {
+  int x, y, z;
+  if (!fold_tile(adx, ady, adz, x, y, z)) return;
+  const V3 g = fold_voxel_rgb(x, y, z, adx, ady, adz, gcells);
+  float* r = grad + ((int64_t(z) * ady + y) * adx + x) * 3;
+  r[0] += g.x;
+  r[1] += g.y;
+  r[2] += g.z;
 }
 
 // Forward mode: the tangent of the density packed like a cell gradient
@@ -496,18 +515,14 @@ int launch_reduce(bool two, const float4* po, int64_t path_begin, int64_t npix, 
 int launch_fold(const rcv_medium* m, float* grad_density, float* grad_albedo, cudaStream_t st) {
   const MediumLayout L = medium_layout(m);
   const char* ws = static_cast<const char*>(m->workspace);
-  const int64_t nv = int64_t(m->dims[0]) * m->dims[1] * m->dims[2];
-  const int block = 256;
-  fold_density_kernel<<<grid_for(nv, block), block, 0, st>>>(
-      m->dims[0], m->dims[1], m->dims[2], reinterpret_cast<const float*>(ws + L.grad_cells),
-      grad_density);
+  fold_density_kernel<<<fold_grid(m->dims), kFoldBlock, 0, st>>>(
+      m->dims[0], m->dims[1], m->dims[2], reinterpret_cast<const float*>(ws + L.grad_cells), grad_density);
   int rc = launched("fold_density launch");
   if (rc) return rc;
   if (grad_albedo != nullptr && m->albedo_old != nullptr) {
     int32_t ad[3];
     albedo_dims_of(m, ad);
-    const int64_t na = (int64_t)albedo_voxels_of(m);
-    fold_albedo_kernel<<<grid_for(na, block), block, 0, st>>>(
+    fold_albedo_kernel<<<fold_grid(ad), kFoldBlock, 0, st>>>(
         ad[0], ad[1], ad[2], reinterpret_cast<const float*>(ws + L.grad_albedo), grad_albedo);
     rc = launched("fold_albedo launch");
   }
@@ -698,8 +713,8 @@ static int64_t gradient_float4s(const VolJob& J, bool albedo) {
 }
 
 // Whether the tape's weights pass clears the gradient records: up to 64 MB,
-// where the launches saved count; beyond, cudaMemsetAsync (256^3: the clear
-// inside cost 0.1 ms more, the scatter after it included).
+// where the launches saved count; beyond, cudaMemsetAsync (256^3: the clear is
+// bound by memory either way, 104 + 85 us apart and 184 together).
 static bool clears_in_weights(const VolJob& J) {
   return gradient_float4s(J, false) + gradient_float4s(J, true) <= (int64_t(1) << 22);
 }
