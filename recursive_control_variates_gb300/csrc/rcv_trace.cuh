@@ -409,6 +409,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
           break;
         }
       }
+      __syncwarp();  // lane 0's last write of *next, seen by all (a shuffle or ballot orders no memory)
       const unsigned take = min((unsigned)__popc(need), left);
       const unsigned rank = (unsigned)__popc(need & lt_mask);
       if (((need >> lane) & 1u) && rank < take) {
