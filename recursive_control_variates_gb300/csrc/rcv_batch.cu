@@ -520,6 +520,7 @@ extern "C" int rcv_batch_job_init(const rcv_batch_job* job, void* stream) {
   O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
   O.order = reinterpret_cast<uint32_t*>(ws + L.order);
   O.cost = nullptr;
+  O.chord = true;  // nothing is packed yet
   RCV_TRY_CUDA(cudaMemsetAsync(O.buckets, 0, 2 * kRenderOrderBuckets * sizeof(uint32_t), st), "order reset");
   rc = order_pixels(&O, 1, st);
   if (rc) return rc;

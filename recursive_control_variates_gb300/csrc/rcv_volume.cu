@@ -70,8 +70,31 @@ __global__ void supergrid_kernel(int sx, int sy, int sz, int dx, int dy, int dz,
 // (bucket 0 = longest; misses last).
 constexpr int kOrderBuckets = 256;
 
-__device__ __forceinline__ int order_key(const VolJob& J, int pix, const uint32_t* cost) {
-  return cost != nullptr ? cost_bucket(cost[pix]) : chord_key(J, pix);
+// Pixels without a cost (a workspace's first call, samples that left at once,
+// the volpathsimple adjoint, which keeps none): the chord through the cube,
+// times one plus the optical depth along it (8 points of the pixel's central
+// ray).  A first call in the order of the film's rows ended on whatever its
+// last rows held: first step of 512^2 x 16 spp 2060 -> 1892 us (by the chord
+// alone 1946), of five 107 x 83 views 1486 -> 1362 (1400), first target of
+// 512^2 x 256 spp 9.3 -> 8.8 ms.
+__device__ __forceinline__ int estimated_key(const VolJob& J, int pix) {
+  V3 o, d;
+  camera_ray(J, pix % J.width, pix / J.width, 0.5f, 0.5f, o, d);
+  float tn, tf;
+  slab(o, recip(d), tn, tf);
+  tn = fmaxf(tn, 0.0f);
+  if (!(tn < tf)) return cost_bucket(0u);
+  const float step = (tf - tn) * 0.125f;
+  float sum = 0.0f;
+  for (int k = 0; k < 8; ++k) sum += density_new(J, locate(J, advance(o, tn + ((float)k + 0.5f) * step, d)));
+  const float est = (tf - tn) * 16.0f * (1.0f + J.scale * sum * step);
+  return cost_bucket((uint32_t)fminf(fmaxf(est, 0.0f), 1e9f) + 1u);
+}
+
+__device__ __forceinline__ int order_key(const OrderJob& O, int pix) {
+  const uint32_t c = O.cost != nullptr ? O.cost[pix] : 0u;
+  if (c != 0u) return cost_bucket(c);
+  return O.chord ? chord_key(O.J, pix) : estimated_key(O.J, pix);
 }
 
 __global__ void order_count_kernel(const __grid_constant__ OrderJob A, const __grid_constant__ OrderJob B) {
@@ -80,7 +103,7 @@ __global__ void order_count_kernel(const __grid_constant__ OrderJob A, const __g
   for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x) hist[k] = 0;
   __syncthreads();
   const int pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix < O.npix) atomicAdd(&hist[order_key(O.J, pix, O.cost)], 1u);
+  if (pix < O.npix) atomicAdd(&hist[order_key(O, pix)], 1u);
   __syncthreads();
   for (int k = threadIdx.x; k < kOrderBuckets; k += blockDim.x)
     if (hist[k]) atomicAdd(O.buckets + k, hist[k]);
@@ -103,7 +126,7 @@ __global__ void __launch_bounds__(kOrderSmallBlock) order_small_kernel(const __g
       reinterpret_cast<uint32_t*>(O.head)[i] = 0u;
   if (t < kOrderBuckets) next[t] = 0u;
   __syncthreads();
-  for (int pix = t; pix < O.npix; pix += kOrderSmallBlock) atomicAdd(&next[order_key(O.J, pix, O.cost)], 1u);
+  for (int pix = t; pix < O.npix; pix += kOrderSmallBlock) atomicAdd(&next[order_key(O, pix)], 1u);
   __syncthreads();
   if (t < 32) {  // exclusive prefix sum, 8 buckets per lane
     uint32_t n[kOrderBuckets / 32], own = 0u;
@@ -121,7 +144,7 @@ __global__ void __launch_bounds__(kOrderSmallBlock) order_small_kernel(const __g
   }
   __syncthreads();
   for (int pix = t; pix < O.npix; pix += kOrderSmallBlock) {
-    O.order[atomicAdd(&next[order_key(O.J, pix, O.cost)], 1u)] = (uint32_t)pix;
+    O.order[atomicAdd(&next[order_key(O, pix)], 1u)] = (uint32_t)pix;
     if (O.cost != nullptr) O.cost[pix] = 0u;  // the next tracer call accumulates afresh
   }
 }
@@ -147,7 +170,7 @@ __global__ void __launch_bounds__(kOrderBuckets) order_place_kernel(const __grid
   __syncthreads();
   const int pix = blockIdx.x * blockDim.x + t;
   const bool valid = pix < O.npix;
-  place_block(valid ? order_key(O.J, pix, O.cost) : 0, valid, (uint32_t)pix, O.buckets + kOrderBuckets, O.order, first);
+  place_block(valid ? order_key(O, pix) : 0, valid, (uint32_t)pix, O.buckets + kOrderBuckets, O.order, first);
   if (valid && O.cost != nullptr) O.cost[pix] = 0u;  // the next tracer call accumulates afresh
 }
 
@@ -692,6 +715,7 @@ static int order_job(VolJob& J, const rcv_volpath_options* o, char* ws, const Re
     O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
     O.order = reinterpret_cast<uint32_t*>(ws + L.order);
     O.cost = cost;
+    O.chord = order == RCV_ORDER_LONGEST_FIRST;
   }
   J.pixel_order = reinterpret_cast<const uint32_t*>(ws + L.order);
   J.pixel_cost = cost;

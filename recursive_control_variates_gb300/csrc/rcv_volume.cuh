@@ -548,8 +548,9 @@ int make_volume_job(const rcv_medium* m, const rcv_sensor* s, const rcv_volpath_
                     int spp, VolJob* J);
 // Pixel hand-out of one job: `order` receives its pixels, most expensive
 // first, by `cost` (the per-pixel path lengths of the previous call, cleared
-// here) or, when cost is null, by the chord length of the pixel's centre ray
-// through the medium.  head: the workspace's head (kRenderHeadBytes), cleared
+// here) where there is one, else by an estimate from the pixel's centre ray:
+// its chord through the cube, and unless `chord` is set the density along it
+// (the medium is packed).  head: the workspace's head (kRenderHeadBytes), cleared
 // before, or null when the caller cleared the buckets.  buckets: 2 x 256 uint32
 // of scratch.
 struct OrderJob {
@@ -559,6 +560,7 @@ struct OrderJob {
   uint32_t* buckets;
   uint32_t* order;
   uint32_t* cost;
+  bool chord;
 };
 // Orders the pixels of one job or of two, in the same launches.
 int order_pixels(const OrderJob* jobs, int n, cudaStream_t st);

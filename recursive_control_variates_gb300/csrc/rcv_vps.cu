@@ -628,8 +628,8 @@ static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, cha
   unsigned long long* qc = reinterpret_cast<unsigned long long*>(ws + L.counters);
   int rc = RCV_OK;
   if (o->order != RCV_ORDER_ROW_MAJOR) {
-    // longest chord through the medium first: the path lengths of an earlier
-    // call would order a little better but would tie the scratch to the caller
+    // by the estimate: the path lengths of an earlier call would order a little
+    // better but would tie the scratch to the caller
     OrderJob O;
     O.J = J;
     O.head = ws;
@@ -637,6 +637,7 @@ static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, cha
     O.buckets = reinterpret_cast<uint32_t*>(ws + L.buckets);
     O.order = reinterpret_cast<uint32_t*>(ws + L.order);
     O.cost = nullptr;
+    O.chord = o->order == RCV_ORDER_LONGEST_FIRST;
     rc = order_pixels(&O, 1, st);
     if (rc) return rc;
     J.pixel_order = O.order;
