@@ -137,7 +137,8 @@ typedef struct rcv_volpath_options {
   int32_t max_depth;     /* path length limit (real scattering events), -1 = none */
   int32_t rr_depth;      /* Russian roulette applies when depth > this            */
   int32_t hide_emitters; /* skip directly visible environment                     */
-  int32_t batch;         /* most paths a warp claims per queue fetch, 0 = 64; small
+  int32_t batch;         /* most paths a warp claims per queue fetch, 0 = 64 (single
+                            jobs of more than 15 M paths: up to 256); small
                             launches: an eighth of a warp's share                */
   int32_t blocks_per_sm; /* persistent blocks per SM, 0 = occupancy limit        */
   int32_t defer;         /* lanes that must wait before a path-start or
