@@ -123,8 +123,17 @@ __global__ void tape_weights_kernel(const __grid_constant__ VolJob single, const
   }
 }
 
-template <bool kCount>
-__global__ void __launch_bounds__(256) tape_scatter_kernel(const __grid_constant__ VolJob single,
+// Gradient of the tape's events.  Bound by the reductions at L2 (they go
+// pairwise, see scatter_density_warp) and by the chain slot -> weight -> lookup:
+// the next slot is loaded a round ahead, and a single job is read from the
+// parameter bank (kTable false).  64 registers, 4 blocks per SM, and as many
+// blocks as are resident: a second wave would go through the tape again after
+// the first, away from the cells in L2 (1024^2 x 16 spp on 256^3: 8 blocks per
+// SM 8.82 ms, 4 8.75, 2 8.73; 512^2 on 64^3 2.01 / 2.00 / 2.18).  24 jobs / 512^2
+// step: 17.02 -> 16.77 ms / 2.01 -> 1.95 by the slot ahead; 5 blocks (48
+// registers, spills) 17.87 / 2.02.
+template <bool kCount, bool kTable>
+__global__ void __launch_bounds__(256, 4) tape_scatter_kernel(const __grid_constant__ VolJob single,
                                                            const VolJob* __restrict__ jobs,
                                                            const float4* __restrict__ tape,
                                                            const unsigned long long* __restrict__ tape_count,
@@ -134,44 +143,53 @@ __global__ void __launch_bounds__(256) tape_scatter_kernel(const __grid_constant
                                                            unsigned long long* counters) {
   const int64_t n = min((int64_t)*tape_count, tape_cap);
   uint32_t ge = 0, ae = 0;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const float4 ev = __ldcs(tape + i);
+  // (whole warps: the reductions go pairwise)
+  const int64_t first = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u);
+  const auto event = [&](int64_t i, float& f) {
+    f = i < n ? __ldcs(tape_f + i) : 0.0f;  // sigma_t (scattering event) or sigma_n
+    return i < n ? __ldcs(tape + i) : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(kTapeEmpty));
+  };
+  float next_f;
+  float4 next = event(first + (threadIdx.x & 31u), next_f);
+  for (int64_t base = first; base < n; base += int64_t(gridDim.x) * blockDim.x) {
+    const float4 ev = next;
+    const float f = next_f;
+    next = event(base + int64_t(gridDim.x) * blockDim.x + (threadIdx.x & 31u), next_f);
     const uint32_t ref = __float_as_uint(ev.w);
-    if (ref == kTapeEmpty) continue;
     const uint32_t kind = ref >> 30, idx = ref & kTapeIndexMask;
-    float s;
-    int j;
-    if (kind == kEvCamera) {
-      const float2 c = __ldg(cam_w + idx);
-      s = c.x;
-      j = __float_as_int(c.y);
-    } else {
-      const float4 wr = __ldg(w + 2 * (int64_t)idx);
-      s = kind == kEvSegment ? wr.x : (kind == kEvShadow ? wr.y : wr.z);
-      j = __float_as_int(wr.w);
+    int j = -1;
+    float s = 0.0f;
+    if (ref != kTapeEmpty) {
+      if (kind == kEvCamera) {
+        const float2 c = __ldg(cam_w + idx);
+        s = c.x;
+        j = __float_as_int(c.y);
+      } else {
+        const float4 wr = __ldg(w + 2 * (int64_t)idx);
+        s = kind == kEvSegment ? wr.x : (kind == kEvShadow ? wr.y : wr.z);
+        j = __float_as_int(wr.w);
+      }
     }
-    if (j < 0) continue;
-    const VolJob& J = jobs != nullptr ? jobs[j] : single;
+    const VolJob& J = kTable ? jobs[j < 0 ? 0 : j] : single;
     const V3 x{ev.x, ev.y, ev.z};
     const Lookup lk = locate(J, x);
-    const float f = __ldcs(tape_f + i);  // sigma_t (scattering event) or sigma_n
-    if (kind == kEvScatter) {
-      scatter_density(J, lk, (J.scale * s) / f);
-      if (kCount) ++ge;
-      if (J.grad_albedo != nullptr) {
-        const AlbedoLookup alk = albedo_lookup(J, lk, x);
+    {
+      const float g = (J.scale * s) / f;
+      const bool on = j >= 0 && (kind != kEvShadow || f > 0.0f);
+      if (kCount && on) ++ge;
+      scatter_density_warp(on, J.grad_cells, lk, kind == kEvScatter ? g : -g);
+    }
+    const bool alb = j >= 0 && kind == kEvScatter && J.grad_albedo != nullptr;
+    if (__any_sync(0xffffffffu, alb)) {
+      const AlbedoLookup alk = albedo_lookup(J, lk, x);
+      V3 ga{0.0f, 0.0f, 0.0f};
+      if (alb) {
         const V3 an = albedo_at(J, alk, 1);
-        const float4 ga = __ldg(w + 2 * (int64_t)idx + 1);
-        scatter_albedo(J, alk,
-                       V3{ga.x / fmaxf(an.x, 1e-8f), ga.y / fmaxf(an.y, 1e-8f), ga.z / fmaxf(an.z, 1e-8f)});
+        const float4 q = __ldg(w + 2 * (int64_t)idx + 1);
+        ga = V3{q.x / fmaxf(an.x, 1e-8f), q.y / fmaxf(an.y, 1e-8f), q.z / fmaxf(an.z, 1e-8f)};
         if (kCount) ++ae;
       }
-    } else {
-      const float sn = f;
-      if (kind != kEvShadow || sn > 0.0f) {
-        scatter_density(J, lk, -(J.scale * s) / sn);
-        if (kCount) ++ge;
-      }
+      scatter_albedo_warp(alb, albedo_record(J, alk), alk, ga);
     }
   }
   if (kCount && counters != nullptr) {
@@ -195,14 +213,11 @@ int launch_tape_gradient(const VolJob& single, const VolJob* jobs, int njobs, co
                                                                    A.clear_albedo, replay_counter);
   int rc = launched("tape_weights launch");
   if (rc) return rc;
-  const unsigned grid = (unsigned)(sms > 0 ? sms : 1) * 8u;
+  const unsigned grid = (unsigned)(sms > 0 ? sms : 1) * 4u;
   unsigned long long* c = reinterpret_cast<unsigned long long*>(counters);
-  if (counters != nullptr)
-    tape_scatter_kernel<true><<<grid, block, 0, st>>>(single, jobs, A.tape, A.tape_count, A.tape_cap, weights,
-                                                       A.cam_w, A.tape_f, c);
-  else
-    tape_scatter_kernel<false><<<grid, block, 0, st>>>(single, jobs, A.tape, A.tape_count, A.tape_cap, weights,
-                                                        A.cam_w, A.tape_f, c);
+  const auto kernel = jobs != nullptr ? (counters != nullptr ? tape_scatter_kernel<true, true> : tape_scatter_kernel<false, true>)
+                                      : (counters != nullptr ? tape_scatter_kernel<true, false> : tape_scatter_kernel<false, false>);
+  kernel<<<grid, block, 0, st>>>(single, jobs, A.tape, A.tape_count, A.tape_cap, weights, A.cam_w, A.tape_f, c);
   return launched("tape_scatter launch");
 }
 

@@ -465,6 +465,11 @@ __device__ __forceinline__ void scatter_density(const VolJob& J, const Lookup& l
   red_add_v4(dst + 1, b0 * gx0, b0 * fx, b1 * gx0, b1 * fx);
 }
 
+__device__ __forceinline__ float4* albedo_record(const VolJob& J, const AlbedoLookup& l) {
+  const int64_t cell = ((int64_t)l.az.cell * (J.ady + 1) + l.ay.cell) * (J.adx + 1) + l.ax.cell;
+  return J.grad_albedo + cell * 6;
+}
+
 // Scatters g (RGB) * (trilinear weight of each corner) into the albedo
 // cell's gradient record (8 corners x RGB = 24 floats, 96 bytes): six vector
 // reductions of consecutive floats, none of them padding.  The fold resolves
@@ -474,8 +479,7 @@ __device__ __forceinline__ void scatter_albedo(const VolJob& J, const AlbedoLook
   const float gx0 = 1.0f - fx, gy0 = 1.0f - fy, gz0 = 1.0f - fz;
   const float w0 = gz0 * gy0, w1 = gz0 * fy, w2 = fz * gy0, w3 = fz * fy;
   const float w[8] = {w0 * gx0, w0 * fx, w1 * gx0, w1 * fx, w2 * gx0, w2 * fx, w3 * gx0, w3 * fx};
-  const int64_t cell = ((int64_t)l.az.cell * (J.ady + 1) + l.ay.cell) * (J.adx + 1) + l.ax.cell;
-  float4* dst = J.grad_albedo + cell * 6;
+  float4* dst = albedo_record(J, l);
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
     float v[4];
@@ -486,6 +490,61 @@ __device__ __forceinline__ void scatter_albedo(const VolJob& J, const AlbedoLook
       v[e] = (c == 0 ? g.x : (c == 1 ? g.y : g.z)) * w[f / 3];
     }
     red_add_v4(dst + q, v[0], v[1], v[2], v[3]);
+  }
+}
+
+// The same scatters for a whole converged warp (every lane calls; `on` = false:
+// nothing to add).  The lanes of a pair exchange halves, so that one
+// instruction adds 32 consecutive bytes of the even lane's record (one sector
+// for two lanes) and the next one those of the odd lane's, instead of half a
+// sector for each lane twice: L2 gets half as many requests for the
+// reductions, which bound the flat gradient passes (batched step of 24 jobs
+// 17.76 -> 17.03 ms, 1024^2 x 16 spp on 256^3 9.53 -> 9.25).
+__device__ __forceinline__ unsigned long long pair_record(bool on, float4* dst) {
+  return on ? reinterpret_cast<unsigned long long>(dst) : 0ull;
+}
+
+// One 32-byte piece (lo, hi) at record + piece of each lane of a pair; mine, other: the lanes' records (0: none).
+__device__ __forceinline__ void red_pair(unsigned long long mine, unsigned long long other, int piece, const float4& lo,
+                                         const float4& hi) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const bool odd = (threadIdx.x & 1u) != 0u;
+  const float4 give = odd ? lo : hi, keep = odd ? hi : lo;
+  const float4 got{__shfl_xor_sync(kFull, give.x, 1), __shfl_xor_sync(kFull, give.y, 1),
+                   __shfl_xor_sync(kFull, give.z, 1), __shfl_xor_sync(kFull, give.w, 1)};
+  const unsigned long long even_rec = odd ? other : mine, odd_rec = odd ? mine : other;
+  const float4 e = odd ? got : keep, o = odd ? keep : got;
+  const int at = piece * 2 + (odd ? 1 : 0);
+  if (even_rec != 0ull) red_add_v4(reinterpret_cast<float4*>(even_rec) + at, e.x, e.y, e.z, e.w);
+  if (odd_rec != 0ull) red_add_v4(reinterpret_cast<float4*>(odd_rec) + at, o.x, o.y, o.z, o.w);
+}
+
+__device__ __forceinline__ void scatter_density_warp(bool on, float4* grad_cells, const Lookup& l, float g) {
+  const float fx = l.ax.f, fy = l.ay.f, fz = l.az.f;
+  const float gx0 = 1.0f - fx, gy0 = 1.0f - fy, gz0 = 1.0f - fz;
+  const float a = g * gz0, b = g * fz;
+  const float a0 = a * gy0, a1 = a * fy, b0 = b * gy0, b1 = b * fy;
+  const unsigned long long rec = pair_record(on, grad_cells + int64_t(l.cell) * 2);
+  red_pair(rec, __shfl_xor_sync(0xffffffffu, rec, 1), 0, make_float4(a0 * gx0, a0 * fx, a1 * gx0, a1 * fx),
+           make_float4(b0 * gx0, b0 * fx, b1 * gx0, b1 * fx));
+}
+
+__device__ __forceinline__ void scatter_albedo_warp(bool on, float4* rec_of_cell, const AlbedoLookup& l, const V3& g) {
+  const float fx = l.ax.f, fy = l.ay.f, fz = l.az.f;
+  const float gx0 = 1.0f - fx, gy0 = 1.0f - fy, gz0 = 1.0f - fz;
+  const float w0 = gz0 * gy0, w1 = gz0 * fy, w2 = fz * gy0, w3 = fz * fy;
+  const float w[8] = {w0 * gx0, w0 * fx, w1 * gx0, w1 * fx, w2 * gx0, w2 * fx, w3 * gx0, w3 * fx};
+  const unsigned long long rec = pair_record(on, rec_of_cell);
+  const unsigned long long other = __shfl_xor_sync(0xffffffffu, rec, 1);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int f = q * 8 + e, c = f % 3;  // corner f / 3, channel f % 3
+      v[e] = (c == 0 ? g.x : (c == 1 ? g.y : g.z)) * w[f / 3];
+    }
+    red_pair(rec, other, q, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]));
   }
 }
 

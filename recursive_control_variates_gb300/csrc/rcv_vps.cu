@@ -422,86 +422,116 @@ __device__ __forceinline__ V3 vps_dL(const VolJob& J, int pix) {
 // term of every segment (4 uniform samples of the second stream), the
 // scattering term at its end, the weight of its shadow walk (for the pass
 // over the tape), and the DRT term of every task.
-__global__ void __launch_bounds__(256) vps_segments_kernel(const __grid_constant__ VolJob J,
+__global__ void __launch_bounds__(256, 4) vps_segments_kernel(const __grid_constant__ VolJob J,
                                                            const __grid_constant__ VpsParams P,
                                                            const __grid_constant__ Queue Q, float* __restrict__ wn) {
   const int64_t nrec = min((int64_t)*Q.ckpt_count, Q.ckpt_cap), ntask = P.use_drt ? (int64_t)*P.task_count : 0;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x, first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (int64_t i = first; i < nrec; i += stride) {
-    const float4* r = Q.ckpt + i * kVpsRec;
-    const float4 r0 = __ldcs(r), r1 = __ldcs(r + 1), r2 = __ldcs(r + 2), r3 = __ldcs(r + 3);
-    const uint32_t path = __float_as_uint(r0.x);
-    const float4 lt = __ldg(Q.path_ltot + path);
-    if (lt.w != 0.0f) {  // lost: the path is taken whole by vps_kernel
-      wn[i] = 0.0f;
-      continue;
+  // (whole warps: the reductions go pairwise)
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  const int64_t first = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u);
+  const unsigned lane = threadIdx.x & 31u;
+  for (int64_t base = first; base < nrec; base += stride) {
+    const int64_t i = base + lane;
+    bool on = false, event = false;  // the record counts; it ends at a scattering event
+    V3 o{0, 0, 0}, d{0, 0, 0}, ga{0, 0, 0};
+    float interval = 0.0f, coef = 0.0f, ge = 0.0f;
+    Pcg32 alt{0ull, 0ull};
+    Lookup l{};
+    AlbedoLookup al{};
+    if (i < nrec) {
+      const float4* r = Q.ckpt + i * kVpsRec;
+      const float4 r0 = __ldcs(r), r1 = __ldcs(r + 1), r2 = __ldcs(r + 2), r3 = __ldcs(r + 3);
+      const uint32_t path = __float_as_uint(r0.x);
+      const float4 lt = __ldg(Q.path_ltot + path);
+      on = lt.w == 0.0f;
+      if (!on) {  // lost: the path is taken whole by vps_kernel
+        wn[i] = 0.0f;
+      } else {
+        int pix;
+        const uint32_t sid = vps_sid(J, path, pix);
+        const V3 dL = vps_dL(J, pix);
+        const V3 res{lt.x - r0.y, lt.y - r0.z, lt.z - r0.w};
+        wn[i] = (dL.x * r3.x + dL.y * r3.y) + dL.z * r3.z;
+        o = V3{r1.x, r1.y, r1.z};
+        d = V3{r2.x, r2.y, r2.z};
+        interval = r1.w;
+        const uint32_t kf = __float_as_uint(r2.w);
+        event = (kf & 1u) == 0u && (!P.use_drt || P.use_drt_mis);
+        if (event) {
+          const V3 x = advance(o, interval, d);
+          l = locate(J, x);
+          al = albedo_lookup(J, l, x);
+          const float st = J.scale * density_new(J, l);
+          const V3 a = albedo_at(J, al, 1);
+          const float mis = P.use_drt ? (st * st) / (1.0f + st * st) : 1.0f;
+          const float inv_pdf = 1.0f / st;
+          const V3 k{((mis * dL.x) * (res.x / fmaxf(1e-8f, a.x))) * inv_pdf,
+                     ((mis * dL.y) * (res.y / fmaxf(1e-8f, a.y))) * inv_pdf,
+                     ((mis * dL.z) * (res.z / fmaxf(1e-8f, a.z))) * inv_pdf};
+          ge = J.scale * ((k.x * a.x + k.y * a.y) + k.z * a.z);
+          ga = V3{k.x * st, k.y * st, k.z * st};
+        }
+        seed_lane(alt, P.alt_seed, sid);
+        alt.state = pcg_jump(alt.state, alt.inc, (uint32_t)P.draws * (kf >> 1) + (uint32_t)(P.draws - 4));
+        const float w = (dL.x * res.x + dL.y * res.y) + dL.z * res.z;
+        coef = -(w * (interval * 0.25f));
+      }
     }
-    int pix;
-    const uint32_t sid = vps_sid(J, path, pix);
-    const V3 dL = vps_dL(J, pix);
-    const V3 res{lt.x - r0.y, lt.y - r0.z, lt.z - r0.w};
-    wn[i] = (dL.x * r3.x + dL.y * r3.y) + dL.z * r3.z;
-    const V3 o{r1.x, r1.y, r1.z}, d{r2.x, r2.y, r2.z};
-    const float interval = r1.w;
-    const uint32_t kf = __float_as_uint(r2.w);
-    if ((kf & 1u) == 0u && (!P.use_drt || P.use_drt_mis)) {
-      const V3 x = advance(o, interval, d);
-      const Lookup l = locate(J, x);
-      const AlbedoLookup al = albedo_lookup(J, l, x);
-      const float st = J.scale * density_new(J, l);
-      const V3 a = albedo_at(J, al, 1);
-      const float mis = P.use_drt ? (st * st) / (1.0f + st * st) : 1.0f;
-      const float inv_pdf = 1.0f / st;
-      const V3 k{((mis * dL.x) * (res.x / fmaxf(1e-8f, a.x))) * inv_pdf,
-                 ((mis * dL.y) * (res.y / fmaxf(1e-8f, a.y))) * inv_pdf,
-                 ((mis * dL.z) * (res.z / fmaxf(1e-8f, a.z))) * inv_pdf};
-      scatter_density(J, l, J.scale * ((k.x * a.x + k.y * a.y) + k.z * a.z));
-      if (J.grad_albedo != nullptr) scatter_albedo(J, al, V3{k.x * st, k.y * st, k.z * st});
+    if (__any_sync(0xffffffffu, event)) {
+      scatter_density_warp(event, J.grad_cells, l, ge);
+      if (J.grad_albedo != nullptr) scatter_albedo_warp(event, albedo_record(J, al), al, ga);
     }
-    Pcg32 alt;
-    seed_lane(alt, P.alt_seed, sid);
-    alt.state = pcg_jump(alt.state, alt.inc, (uint32_t)P.draws * (kf >> 1) + (uint32_t)(P.draws - 4));
-    const float w = (dL.x * res.x + dL.y * res.y) + dL.z * res.z;
-    const float coef = -(w * (interval * 0.25f));
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float tj = next1d(alt) * interval;
-      scatter_density(J, locate(J, advance(o, tj, d)), J.scale * coef);
+      scatter_density_warp(on, J.grad_cells, locate(J, advance(o, tj, d)), J.scale * coef);
     }
   }
   if (!(J.scale * bits_to_float(__ldg(J.maxbits + 1)) > 0.0f)) return;  // empty medium: no DRT
-  for (int64_t i = first; i < ntask; i += stride) {
-    const float4* t = P.task + i * kVpsTask;
-    const float4 t0 = __ldcs(t), t1 = __ldcs(t + 1), t2 = __ldcs(t + 2);
-    int pix;
-    vps_sid(J, __float_as_uint(t0.x), pix);
-    const V3 dL = vps_dL(J, pix), x{t2.x, t2.y, t2.z};
-    const Lookup l = locate(J, x);
-    const AlbedoLookup al = albedo_lookup(J, l, x);
-    const float st = J.scale * density_new(J, l);
-    const V3 a = albedo_at(J, al, 1);
-    const float mis = P.use_drt_mis ? 1.0f / (1.0f + st * st) : 1.0f;
-    const float k0 = mis * t1.w;
-    const V3 k{(k0 * (t1.x * dL.x)) * t0.y, (k0 * (t1.y * dL.y)) * t0.z, (k0 * (t1.z * dL.z)) * t0.w};
-    scatter_density(J, l, J.scale * ((k.x * a.x + k.y * a.y) + k.z * a.z));
-    if (J.grad_albedo != nullptr) scatter_albedo(J, al, V3{k.x * st, k.y * st, k.z * st});
+  for (int64_t base = first; base < ntask; base += stride) {
+    const int64_t i = base + lane;
+    const bool on = i < ntask;
+    Lookup l{};
+    AlbedoLookup al{};
+    float ge = 0.0f;
+    V3 ga{0, 0, 0};
+    if (on) {
+      const float4* t = P.task + i * kVpsTask;
+      const float4 t0 = __ldcs(t), t1 = __ldcs(t + 1), t2 = __ldcs(t + 2);
+      int pix;
+      vps_sid(J, __float_as_uint(t0.x), pix);
+      const V3 dL = vps_dL(J, pix), x{t2.x, t2.y, t2.z};
+      l = locate(J, x);
+      al = albedo_lookup(J, l, x);
+      const float st = J.scale * density_new(J, l);
+      const V3 a = albedo_at(J, al, 1);
+      const float mis = P.use_drt_mis ? 1.0f / (1.0f + st * st) : 1.0f;
+      const float k0 = mis * t1.w;
+      const V3 k{(k0 * (t1.x * dL.x)) * t0.y, (k0 * (t1.y * dL.y)) * t0.z, (k0 * (t1.z * dL.z)) * t0.w};
+      ge = J.scale * ((k.x * a.x + k.y * a.y) + k.z * a.z);
+      ga = V3{k.x * st, k.y * st, k.z * st};
+    }
+    scatter_density_warp(on, J.grad_cells, l, ge);
+    if (J.grad_albedo != nullptr) scatter_albedo_warp(on, albedo_record(J, al), al, ga);
   }
 }
 
 // Flat pass over the shadow-walk steps on the tape: -(weight of the walk) /
 // sigma_n at each.
-__global__ void __launch_bounds__(256) vps_shadow_kernel(const __grid_constant__ VolJob J,
+__global__ void __launch_bounds__(256, 6) vps_shadow_kernel(const __grid_constant__ VolJob J,
                                                          const __grid_constant__ Queue Q,
                                                          const float* __restrict__ wn) {
   const int64_t n = min((int64_t)*Q.tape_count, Q.tape_cap);
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const float4 ev = __ldcs(Q.tape + i);
+  const int64_t first = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u);
+  for (int64_t base = first; base < n; base += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t i = base + (threadIdx.x & 31u);
+    const float4 ev = i < n ? __ldcs(Q.tape + i) : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(kTapeEmpty));
     const uint32_t ref = __float_as_uint(ev.w);
-    if (ref == kTapeEmpty) continue;
-    const float w = __ldg(wn + ref);
-    if (w == 0.0f) continue;
-    const float sn = __ldcs(Q.tape_f + i);
-    scatter_density(J, locate(J, V3{ev.x, ev.y, ev.z}), -(J.scale * w) / sn);
+    const float w = ref != kTapeEmpty ? __ldg(wn + ref) : 0.0f;
+    const bool on = w != 0.0f;
+    float g = 0.0f;
+    if (on) g = -(J.scale * w) / __ldcs(Q.tape_f + i);
+    scatter_density_warp(on, J.grad_cells, locate(J, V3{ev.x, ev.y, ev.z}), g);
   }
 }
 
@@ -681,10 +711,12 @@ static int vps_recorded(VolJob J, VpsParams P, const rcv_volpath_options* o, cha
       rc = launched("volpathsimple tracer launch");
       if (rc) return rc;
     }
-    vps_segments_kernel<<<(unsigned)sms * 8u, 256, 0, st>>>(J, P, Q, wn);
+    // as many blocks as are resident, so that the pass goes through its records
+    // once (8 blocks per SM in two waves: DRT step of 512^2 x 16 spp 2978 us, so 2923)
+    vps_segments_kernel<<<(unsigned)sms * 4u, 256, 0, st>>>(J, P, Q, wn);
     rc = launched("volpathsimple segments launch");
     if (rc) return rc;
-    vps_shadow_kernel<<<(unsigned)sms * 8u, 256, 0, st>>>(J, Q, wn);
+    vps_shadow_kernel<<<(unsigned)sms * 6u, 256, 0, st>>>(J, Q, wn);
     rc = launched("volpathsimple shadow launch");
     if (rc) return rc;
     VpsParams R = P;
