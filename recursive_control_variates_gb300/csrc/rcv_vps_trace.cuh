@@ -236,6 +236,9 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
       thr = V3{1, 1, 1};
       L = V3{0, 0, 0};
       if (kDrt) {
+        // last task first: the first launch's longest paths ended last, and
+        // theirs are the tasks that take longest
+        path = (uint32_t)*P.task_count - 1u - path;
         U(cTask) = path;
         const float4 t0 = P.task[(int64_t)path * kVpsTask];
         const float4* r = Q.ckpt + (int64_t)__float_as_uint(t0.y) * kVpsRec;
