@@ -153,23 +153,31 @@ __global__ void __launch_bounds__(256) surface_tape_scatter_kernel(const __grid_
                                                                    int64_t tape_cap,
                                                                    const float4* __restrict__ ltot) {
   const int64_t n = min((int64_t)*tape_count, tape_cap) / 2;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const float4 a = __ldcs(tape + 2 * i);
-    if (__float_as_uint(a.w) == kTapeEmpty) continue;
-    const float4 b = __ldcs(tape + 2 * i + 1);
-    const uint32_t path = __float_as_uint(a.z);
-    const float4 lt = __ldg(ltot + path);
-    if (lt.w != 0.0f) continue;
-    const int pix = (int)(path / (uint32_t)S.spp);
-    const float fs = (float)S.spp;
-    const float* g = S.grad_img + (int64_t)pix * 3;
-    const V3 dL{g[0] / fs, g[1] / fs, g[2] / fs};
-    const TexLookup tl = tex_locate(S, V3{a.x, 0.0f, a.y});
-    const V3 an = tex_eval(S, tl, 1);
-    const V3 lr{lt.x - b.x, lt.y - b.y, lt.z - b.z};
-    tex_scatter(S, tl,
-                V3{(dL.x * lr.x) / fmaxf(an.x, 1e-8f), (dL.y * lr.y) / fmaxf(an.y, 1e-8f),
-                   (dL.z * lr.z) / fmaxf(an.z, 1e-8f)});
+  const int64_t first = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u);
+  for (int64_t base = first; base < n; base += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t i = base + (threadIdx.x & 31u);
+    bool on = false;
+    TexLookup tl{};
+    V3 gt{0.0f, 0.0f, 0.0f};
+    if (i < n) {
+      const float4 a = __ldcs(tape + 2 * i);
+      if (__float_as_uint(a.w) != kTapeEmpty) {
+        const float4 b = __ldcs(tape + 2 * i + 1);
+        const uint32_t path = __float_as_uint(a.z);
+        const float4 lt = __ldg(ltot + path);
+        on = lt.w == 0.0f;
+        const int pix = (int)(path / (uint32_t)S.spp);
+        const float fs = (float)S.spp;
+        const float* g = S.grad_img + (int64_t)pix * 3;
+        const V3 dL{g[0] / fs, g[1] / fs, g[2] / fs};
+        tl = tex_locate(S, V3{a.x, 0.0f, a.y});
+        const V3 an = tex_eval(S, tl, 1);
+        const V3 lr{lt.x - b.x, lt.y - b.y, lt.z - b.z};
+        gt = V3{(dL.x * lr.x) / fmaxf(an.x, 1e-8f), (dL.y * lr.y) / fmaxf(an.y, 1e-8f),
+                (dL.z * lr.z) / fmaxf(an.z, 1e-8f)};
+      }
+    }
+    tex_scatter_warp(on, S, tl, gt);
   }
 }
 
