@@ -438,13 +438,9 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     bool finished = false;  // the lane's current path (or task) ends this iteration
     // the shadow walk ends in this iteration (handled below, after the tape)
     bool nee_done = false;
-    // kTape: this iteration's events, appended where the warp has
-    // reconverged: a walk step at x (null collision or shadow-walk step) with
-    // its reference and sigma_n, and the scattering event at the cold vertex
-    // processed in this iteration with its sigma_t
-    bool ev_walk = false;
-    uint32_t ev_ref = 0;
-    float ev_f = 0.0f, ev_sf = 0.0f;
+    // kTape: the scattering event at the cold vertex processed in this iteration,
+    // with its sigma_t
+    float ev_sf = 0.0f;
     bool ev_scat = false;
 
     // ------------------------------------------------------------ path start
@@ -727,153 +723,164 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     }
 
     // --------------------------------------------------- free-flight step
-    if (phase == kMain || phase == kNee || phase == kNeeAdj) {
-      const VolJob& J = kTable ? *Jp : single;
-      // whole-path replay: the second shadow walk draws from the saved stream
-      // (chosen by value, not through a pointer, which would put both
-      // streams in local memory)
-      const bool nee_stream = kRep && phase == kNeeAdj && task == kTaskWhole;
-      if (phase == kMain && !roulette<kMode>(J, rng, depth, bn, bo)) {
-        finished = true;
-      } else {
-        // majorant of this collision: global, or the supergrid cell it lies in
-        float mu_c = mu, inv_c = inv_mu, hinv_c = 0.5f * inv_mu;
-        float t;
-        if (kSG && J.sg[0] > 0) {
-          const float tau = -log_unit(1.0f - (nee_stream ? next1d_state(nee_state, rng.inc) : next1d(rng)));
-          t = supergrid_flight(J, kMode == kTwoState ? J.sg_two : J.sg_new, x, dir, rem, tau, mu_c);
-          inv_c = 1.0f / mu_c;
-          hinv_c = 0.5f * inv_c;
-        } else {
-          t = free_flight(nee_stream ? next1d_state(nee_state, rng.inc) : next1d(rng), mu, inv_mu);
-        }
-        const bool valid = t <= rem;
-        Lookup lk;
-        float rho_o = 0.0f, rho_n = 0.0f;
-        if (valid) {
-          x = advance(x, t, dir);  // the step's end, whatever happens there
-          lk = locate(J, x);
-          if (kMode == kTwoState)
-            density2(J, lk, rho_o, rho_n);
-          else
-            rho_n = density_new(J, lk);
-          if (kCount) {
-            if (phase == kMain)
-              ++cnt.lookups;
-            else
-              ++cnt.nee_lookups;
-          }
-        }
-        const float st_o = J.scale * rho_o, st_n = J.scale * rho_n;
-
-        bool walk_done = false;  // the shadow walk ends
-        if (valid) {
-          // factors of the step if it is not a scattering event: ratio
-          // tracking of a shadow ray (plugins/twostatevolpath.py:443-452), or
-          // the weights of a null collision (:227-231, 256-257; they sum to 2,
-          // equal states give exactly 1)
-          const float sn_n = mu_c - st_n;
-          float fn = sn_n * inv_c, fo = kMode == kTwoState ? (mu_c - st_o) * inv_c : 1.0f;
-          bool null = true;
-          if (phase == kMain) {
-            const float ur = next1d(rng);
-            // real-collision probability: mean of both states' sigma_t / mu
-            // (plugins/twostatevolpath.py:222-225); equal states give exactly
-            // the single-state sigma_t / mu
-            float prob;
-            if (kMode == kTwoState)
-              prob = (st_n + st_o) * hinv_c;
-            else
-              prob = st_n * inv_c;
-            null = ur >= prob;
-            fn = 1.0f;
-            if (kMode == kTwoState) {
-              const float den = sn_n + (mu_c - st_o);
-              fn = (2.0f * sn_n) / den;
-              fo = 2.0f - fn;
-            }
-          }
-          if (null) {
-            bn.x *= fn;  // (of a shadow ray: its transmittance)
-            if (kMode == kTwoState) {
-              bo.x *= fo;
-              const float gn = phase == kMain ? fn : 1.0f, go = phase == kMain ? fo : 1.0f;
-              bn.y *= gn;
-              bn.z *= gn;
-              bo.y *= go;
-              bo.z *= go;
-            }
-            if (kRep && phase != kNee && (phase == kMain || sn_n > 0.0f)) {
-              if (kMode == kForward) {
-                const V3 Lr = phase == kMain ? Lrem : cn_task;
-                const float f = -(J.scale * tangent_density(J, lk)) / sn_n;
-                dL = V3{dL.x + Lr.x * f, dL.y + Lr.y * f, dL.z + Lr.z * f};
-              } else {
-                scatter_density(J, lk, -(J.scale * (phase == kMain ? s_main : s_nee)) / sn_n);
-              }
-              if (kCount) ++cnt.grad_events;
-            }
-            rem = rem - t;
-            if (kMode == kTape) {
-              ev_walk = true;
-              ev_ref = tref;
-              ev_f = sn_n;
-            }
-            walk_done = phase != kMain && ((kMode == kTwoState) ? (trn == 0.0f && tro == 0.0f) : (trn == 0.0f));
-          } else {
-            // real scattering event (plugins/twostatevolpath.py:249-253)
-            depth += 1;
-            if (depth >= J.max_depth) {
-              finished = true;
-            } else {
-              if (kCount) ++cnt.scatters;
-              F(cScn) = st_n;
-              if (kMode == kTwoState) F(cSco) = st_o;
-              phase = kScatter;
-            }
-          }
-        } else if (phase == kMain) {
-          // leaves the cube: null BSDF sample, outside iteration RR, environment
-          pcg_skip3(rng);
-          if (roulette<kMode>(J, rng, depth, bn, bo) && !(J.hide_emitters && depth == 0)) {
-            V3 Ln = get3(cLn), Lo{0, 0, 0};
-            if (kMode == kTwoState) Lo = get3(cLo);
-            if (kEnv) {
-              // environment map hit after a phase sample: power heuristic
-              // against NEE (plugins/twostatevolpath.py:288-308)
-              float pdf;
-              const V3 Le = env_radiance_dir(J, dir, pdf);
-              const float k = depth == 0 ? 1.0f : env_mis(kInvFourPi, pdf);
-              Ln = V3{Ln.x + (bn.x * Le.x) * k, Ln.y + (bn.y * Le.y) * k, Ln.z + (bn.z * Le.z) * k};
-              if (kMode == kTwoState)
-                Lo = V3{Lo.x + (bo.x * Le.x) * k, Lo.y + (bo.y * Le.y) * k, Lo.z + (bo.z * Le.z) * k};
-            } else {
-              const float k = depth == 0 ? 1.0f : mis;
-              Ln = V3{Ln.x + bn.x * k, Ln.y + bn.y * k, Ln.z + bn.z * k};
-              if (kMode == kTwoState) Lo = V3{Lo.x + bo.x * k, Lo.y + bo.y * k, Lo.z + bo.z * k};
-            }
-            put3(cLn, Ln);
-            if (kMode == kTwoState) put3(cLo, Lo);
-          }
+    const int steps = kRep || kSG || queue_empty ? 1 : kWalkSteps;
+#pragma unroll 1
+    for (int sub = 1;; ++sub) {
+      // kTape: this step's event, appended where the warp has reconverged (null
+      // collision or shadow-walk step at x), with its reference and sigma_n
+      bool ev_walk = false;
+      uint32_t ev_ref = 0;
+      float ev_f = 0.0f;
+      if (!finished && !nee_done && (phase == kMain || phase == kNee || phase == kNeeAdj)) {
+        const VolJob& J = kTable ? *Jp : single;
+        // whole-path replay: the second shadow walk draws from the saved stream
+        // (chosen by value, not through a pointer, which would put both
+        // streams in local memory)
+        const bool nee_stream = kRep && phase == kNeeAdj && task == kTaskWhole;
+        if (phase == kMain && !roulette<kMode>(J, rng, depth, bn, bo)) {
           finished = true;
         } else {
-          walk_done = true;
-        }
-        if (!kRep || phase == kNee) {
-          nee_done = walk_done;
-        } else if (walk_done) {
-          // kNeeAdj: the shadow walk with gradients ends
-          bn.x = F(cBn);
-          x = get3(cP);
-          dir = get3(cWo);
-          rem = F(cT);
-          phase = kMain;
+          // majorant of this collision: global, or the supergrid cell it lies in
+          float mu_c = mu, inv_c = inv_mu, hinv_c = 0.5f * inv_mu;
+          float t;
+          if (kSG && J.sg[0] > 0) {
+            const float tau = -log_unit(1.0f - (nee_stream ? next1d_state(nee_state, rng.inc) : next1d(rng)));
+            t = supergrid_flight(J, kMode == kTwoState ? J.sg_two : J.sg_new, x, dir, rem, tau, mu_c);
+            inv_c = 1.0f / mu_c;
+            hinv_c = 0.5f * inv_c;
+          } else {
+            t = free_flight(nee_stream ? next1d_state(nee_state, rng.inc) : next1d(rng), mu, inv_mu);
+          }
+          const bool valid = t <= rem;
+          Lookup lk;
+          float rho_o = 0.0f, rho_n = 0.0f;
+          if (valid) {
+            x = advance(x, t, dir);  // the step's end, whatever happens there
+            lk = locate(J, x);
+            if (kMode == kTwoState)
+              density2(J, lk, rho_o, rho_n);
+            else
+              rho_n = density_new(J, lk);
+            if (kCount) {
+              if (phase == kMain)
+                ++cnt.lookups;
+              else
+                ++cnt.nee_lookups;
+            }
+          }
+          const float st_o = J.scale * rho_o, st_n = J.scale * rho_n;
+
+          bool walk_done = false;  // the shadow walk ends
+          if (valid) {
+            // factors of the step if it is not a scattering event: ratio
+            // tracking of a shadow ray (plugins/twostatevolpath.py:443-452), or
+            // the weights of a null collision (:227-231, 256-257; they sum to 2,
+            // equal states give exactly 1)
+            const float sn_n = mu_c - st_n;
+            float fn = sn_n * inv_c, fo = kMode == kTwoState ? (mu_c - st_o) * inv_c : 1.0f;
+            bool null = true;
+            if (phase == kMain) {
+              const float ur = next1d(rng);
+              // real-collision probability: mean of both states' sigma_t / mu
+              // (plugins/twostatevolpath.py:222-225); equal states give exactly
+              // the single-state sigma_t / mu
+              float prob;
+              if (kMode == kTwoState)
+                prob = (st_n + st_o) * hinv_c;
+              else
+                prob = st_n * inv_c;
+              null = ur >= prob;
+              fn = 1.0f;
+              if (kMode == kTwoState) {
+                const float den = sn_n + (mu_c - st_o);
+                fn = (2.0f * sn_n) / den;
+                fo = 2.0f - fn;
+              }
+            }
+            if (null) {
+              bn.x *= fn;  // (of a shadow ray: its transmittance)
+              if (kMode == kTwoState) {
+                bo.x *= fo;
+                const float gn = phase == kMain ? fn : 1.0f, go = phase == kMain ? fo : 1.0f;
+                bn.y *= gn;
+                bn.z *= gn;
+                bo.y *= go;
+                bo.z *= go;
+              }
+              if (kRep && phase != kNee && (phase == kMain || sn_n > 0.0f)) {
+                if (kMode == kForward) {
+                  const V3 Lr = phase == kMain ? Lrem : cn_task;
+                  const float f = -(J.scale * tangent_density(J, lk)) / sn_n;
+                  dL = V3{dL.x + Lr.x * f, dL.y + Lr.y * f, dL.z + Lr.z * f};
+                } else {
+                  scatter_density(J, lk, -(J.scale * (phase == kMain ? s_main : s_nee)) / sn_n);
+                }
+                if (kCount) ++cnt.grad_events;
+              }
+              rem = rem - t;
+              if (kMode == kTape) {
+                ev_walk = true;
+                ev_ref = tref;
+                ev_f = sn_n;
+              }
+              walk_done = phase != kMain && ((kMode == kTwoState) ? (trn == 0.0f && tro == 0.0f) : (trn == 0.0f));
+            } else {
+              // real scattering event (plugins/twostatevolpath.py:249-253)
+              depth += 1;
+              if (depth >= J.max_depth) {
+                finished = true;
+              } else {
+                if (kCount) ++cnt.scatters;
+                F(cScn) = st_n;
+                if (kMode == kTwoState) F(cSco) = st_o;
+                phase = kScatter;
+              }
+            }
+          } else if (phase == kMain) {
+            // leaves the cube: null BSDF sample, outside iteration RR, environment
+            pcg_skip3(rng);
+            if (roulette<kMode>(J, rng, depth, bn, bo) && !(J.hide_emitters && depth == 0)) {
+              V3 Ln = get3(cLn), Lo{0, 0, 0};
+              if (kMode == kTwoState) Lo = get3(cLo);
+              if (kEnv) {
+                // environment map hit after a phase sample: power heuristic
+                // against NEE (plugins/twostatevolpath.py:288-308)
+                float pdf;
+                const V3 Le = env_radiance_dir(J, dir, pdf);
+                const float k = depth == 0 ? 1.0f : env_mis(kInvFourPi, pdf);
+                Ln = V3{Ln.x + (bn.x * Le.x) * k, Ln.y + (bn.y * Le.y) * k, Ln.z + (bn.z * Le.z) * k};
+                if (kMode == kTwoState)
+                  Lo = V3{Lo.x + (bo.x * Le.x) * k, Lo.y + (bo.y * Le.y) * k, Lo.z + (bo.z * Le.z) * k};
+              } else {
+                const float k = depth == 0 ? 1.0f : mis;
+                Ln = V3{Ln.x + bn.x * k, Ln.y + bn.y * k, Ln.z + bn.z * k};
+                if (kMode == kTwoState) Lo = V3{Lo.x + bo.x * k, Lo.y + bo.y * k, Lo.z + bo.z * k};
+              }
+              put3(cLn, Ln);
+              if (kMode == kTwoState) put3(cLo, Lo);
+            }
+            finished = true;
+          } else {
+            walk_done = true;
+          }
+          if (!kRep || phase == kNee) {
+            nee_done = walk_done;
+          } else if (walk_done) {
+            // kNeeAdj: the shadow walk with gradients ends
+            bn.x = F(cBn);
+            x = get3(cP);
+            dir = get3(cWo);
+            rem = F(cT);
+            phase = kMain;
+          }
         }
       }
+      if (kMode == kTape && !tape_append(Q, tc, ev_walk && !ck_lost, x, ev_ref, ev_f)) ck_lost = true;
+      if (sub >= steps) break;
+      ++n_iter;  // (a path's cost counts its steps)
     }
 
-    if (kMode == kTape) {
-      if (!tape_append(Q, tc, ev_walk && !ck_lost, x, ev_ref, ev_f)) ck_lost = true;
+    if (kMode == kTape && run_scat) {
       if (!tape_append(Q, tc, ev_scat && !ck_lost, get3(cP), (kEvScatter << 30) | (tref & kTapeIndexMask), ev_sf))
         ck_lost = true;
     }
