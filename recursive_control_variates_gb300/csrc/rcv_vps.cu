@@ -405,8 +405,10 @@ __global__ void __launch_bounds__(128) vps_kernel(const __grid_constant__ VolJob
   }
 }
 
+// Resident blocks per SM: 7 without spills for the DRT paths (72 registers), 6
+// for the first (80; at 7, which spills, a DRT step is 2 % slower).
 template <int kMode, bool kSG, bool kEnv>
-__global__ void __launch_bounds__(kVpsBlock, 6) vps_trace_kernel(const __grid_constant__ VolJob J,
+__global__ void __launch_bounds__(kVpsBlock, kMode == kVpsDrt ? 7 : 6) vps_trace_kernel(const __grid_constant__ VolJob J,
                                                                  const __grid_constant__ VpsParams P,
                                                                  const __grid_constant__ Queue Q) {
   trace_vps<kMode, kSG, kEnv>(J, P, Q);

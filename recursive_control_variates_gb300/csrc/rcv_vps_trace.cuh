@@ -465,81 +465,85 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
     }
 
     // ---------------------------------------------------- free-flight step
-    bool ev = false;  // kVpsTape: a shadow-walk step with a gradient, at p
-    float ev_sn = 0.0f;
-    if (!finished && (phase == kVMain || phase == kVNee)) {
-      float m = mu, inv_m = inv_mu, t;
-      const float uf = next1d(rng);
-      if (kSG) {
-        m = mu;
-        t = supergrid_flight(J, J.sg_new, p, w, rem, -log_unit(1.0f - uf), m);
-        inv_m = 1.0f / m;
-      } else {
-        t = free_flight(uf, mu, inv_mu);
-      }
-      const bool valid = t <= rem;
-      float st = 0.0f;
-      V3 x;
-      if (valid) {
-        x = advance(p, t, w);
-        st = J.scale * density_new(J, locate(J, x));
-      }
-      if (phase == kVMain) {
+    // (several before the next look at the lanes that wait, see kWalkSteps)
+    const int steps = kSG || queue_empty ? 1 : kWalkSteps;
+#pragma unroll 1
+    for (int sub = 1;; ++sub) {
+      bool ev = false;  // kVpsTape: a shadow-walk step with a gradient, at p
+      float ev_sn = 0.0f;
+      if (!finished && (phase == kVMain || phase == kVNee)) {
+        float m = mu, inv_m = inv_mu, t;
+        const float uf = next1d(rng);
+        if (kSG) {
+          m = mu;
+          t = supergrid_flight(J, J.sg_new, p, w, rem, -log_unit(1.0f - uf), m);
+          inv_m = 1.0f / m;
+        } else {
+          t = free_flight(uf, mu, inv_mu);
+        }
+        const bool valid = t <= rem;
+        float st = 0.0f;
+        V3 x;
         if (valid) {
-          const float ratio = m != 0.0f ? div_by(st, m, inv_m) : 0.0f;
-          const float u = next1d(rng);
-          acc = acc + t;
-          if (u < ratio) {
-            phase = kVVertex;
+          x = advance(p, t, w);
+          st = J.scale * density_new(J, locate(J, x));
+        }
+        if (phase == kVMain) {
+          if (valid) {
+            const float ratio = m != 0.0f ? div_by(st, m, inv_m) : 0.0f;
+            const float u = next1d(rng);
+            acc = acc + t;
+            if (u < ratio) {
+              phase = kVVertex;
+            } else {
+              p = x;
+              rem = rem - t;
+            }
           } else {
-            p = x;
-            rem = rem - t;
+            phase = kVEscape;
           }
         } else {
-          phase = kVEscape;
-        }
-      } else {
-        bool done = !valid;
-        if (valid) {
-          const float sn = m - st;
-          const float contrib = m != 0.0f ? div_by(sn, m, inv_m) : sn;
-          acc = acc * contrib;
-          p = x;
-          rem = rem - t;
-          if (!kDrt) {
-            ev = contrib > 0.0f && !lost;
-            ev_sn = sn;
+          bool done = !valid;
+          if (valid) {
+            const float sn = m - st;
+            const float contrib = m != 0.0f ? div_by(sn, m, inv_m) : sn;
+            acc = acc * contrib;
+            p = x;
+            rem = rem - t;
+            if (!kDrt) {
+              ev = contrib > 0.0f && !lost;
+              ev_sn = sn;
+            }
+            done = acc == 0.0f;
           }
-          done = acc == 0.0f;
-        }
-        if (done) {
-          if (kDrt && stage == 0) {
-            phase = kVVertex;
-          } else {
-            V3 c;
-            if (kEnv) {
-              c = V3{(thr.x * F(cEnv)) * acc, (thr.y * F(cEnv + 1)) * acc, (thr.z * F(cEnv + 2)) * acc};
+          if (done) {
+            if (kDrt && stage == 0) {
+              phase = kVVertex;
             } else {
-              const float mis = 0.5f, en = (1.0f / kInvFourPi) * acc;
-              c = V3{((thr.x * kInvFourPi) * mis) * en, ((thr.y * kInvFourPi) * mis) * en,
-                     ((thr.z * kInvFourPi) * mis) * en};
+              V3 c;
+              if (kEnv) {
+                c = V3{(thr.x * F(cEnv)) * acc, (thr.y * F(cEnv + 1)) * acc, (thr.z * F(cEnv + 2)) * acc};
+              } else {
+                const float mis = 0.5f, en = (1.0f / kInvFourPi) * acc;
+                c = V3{((thr.x * kInvFourPi) * mis) * en, ((thr.y * kInvFourPi) * mis) * en,
+                       ((thr.z * kInvFourPi) * mis) * en};
+              }
+              if (kDrt && stage == 1) {
+                F(cNee) = c.x;
+                F(cNee + 1) = c.y;
+                F(cNee + 2) = c.z;
+              } else {
+                L = V3{L.x + c.x, L.y + c.y, L.z + c.z};
+                if (!kDrt && !lost)
+                  __stcs(Q.ckpt + (int64_t)rec * kVpsRec + 3, make_float4(c.x, c.y, c.z, 0.0f));
+              }
+              phase = kVDir;
             }
-            if (kDrt && stage == 1) {
-              F(cNee) = c.x;
-              F(cNee + 1) = c.y;
-              F(cNee + 2) = c.z;
-            } else {
-              L = V3{L.x + c.x, L.y + c.y, L.z + c.z};
-              if (!kDrt && !lost)
-                __stcs(Q.ckpt + (int64_t)rec * kVpsRec + 3, make_float4(c.x, c.y, c.z, 0.0f));
-            }
-            phase = kVDir;
           }
         }
       }
-    }
-    if (!kDrt) {
-      if (!tape_append(Q, tc, ev, p, rec, ev_sn)) lost = true;
+      if (!kDrt && !tape_append(Q, tc, ev, p, rec, ev_sn)) lost = true;
+      if (sub >= steps) break;
     }
 
     // -------------------------------------------------------------- path end
