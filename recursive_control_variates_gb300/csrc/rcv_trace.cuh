@@ -690,6 +690,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     }
 
     // ------------------------- cooperative walk of the last paths (see above)
+    bool many = false;  // too many lanes walk for it
     if (kCoop && queue_empty) {
       const VolJob& J = kTable ? *Jp : single;
       bool elig = false;
@@ -705,6 +706,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       }
       const unsigned m_coop = __ballot_sync(0xffffffffu, elig);
       const int n_coop = __popc(m_coop);
+      many = n_coop > kCoopMost;
       if (n_coop >= 1 && n_coop <= kCoopMost) {
         const bool mw = phase == kMain;
         float* s = s_coop + (threadIdx.x >> 5) * 96;
@@ -723,7 +725,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
     }
 
     // --------------------------------------------------- free-flight step
-    const int steps = kRep || kSG || queue_empty ? 1 : kWalkSteps;
+    const int steps = kRep || kSG || (queue_empty && !many) ? 1 : kWalkSteps;
 #pragma unroll 1
     for (int sub = 1;; ++sub) {
       // kTape: this step's event, appended where the warp has reconverged (null

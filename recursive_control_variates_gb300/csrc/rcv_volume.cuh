@@ -675,15 +675,17 @@ int launch_persistent(int mode, const VolJob& J, const VolJob* jobs, int njobs, 
                       const AdjBuffers* adj, uint64_t* counters, cudaStream_t st, bool supergrid,
                       bool zeroed = false);
 // Free-flight steps that a tracer's walking lanes take in a row while paths are
-// left to hand out.  Tracers are bound by instruction issue; handing paths out,
-// looking at the phases and the ends of walks and paths (few lanes each) cost
-// about a third of an iteration, and a lane that stops early waits for a few
-// steps at most.  1 / 2 / 3 / 4 / 6 steps: 512^2 x 256-spp target 9.73 / 8.15 /
-// 7.98 / 7.87 / 7.83 ms, 24 jobs 16.76 / 15.70 / 15.60 / 15.63 / 15.92, 512^2 x 16
-// spp 1.785 / 1.671 / 1.638 / 1.630 / 1.630, 1024^2 on 256^3 9.13 / 8.74 / 8.65 / 8.59
-// / 8.59.  Going on while 2/3, 3/4 or 7/8 of the lanes still walk was slower (16.1
-// to 16.4 ms for the 24 jobs).  A supergrid's step is long and its walks are
-// short: 1 (829 us at 1, 836 / 863 / 876 at 2 / 3 / 4).
+// left to hand out or too many lanes walk for the cooperative walk.  Tracers are
+// bound by instruction issue; handing paths out, looking at the phases and the
+// ends of walks and paths (few lanes each) cost about a third of an iteration,
+// and a lane that stops early waits for a few steps at most.  1 / 2 / 3 / 4 / 6
+// steps: 512^2 x 256-spp target 9.73 / 8.15 / 7.98 / 7.87 / 7.83 ms, 24 jobs 16.76 /
+// 15.70 / 15.60 / 15.63 / 15.92, 512^2 x 16 spp 1.785 / 1.671 / 1.638 / 1.630 /
+// 1.630, 1024^2 on 256^3 9.13 / 8.74 / 8.65 / 8.59 / 8.59.  One step as soon as the
+// queue is empty: 24 jobs 15.63 against 15.50 ms, three map-lit DRT views 1.875
+// against 1.835.  Going on while 2/3, 3/4 or 7/8 of the lanes still walk was slower
+// (16.1 to 16.4 ms for the 24 jobs).  A supergrid's step is long and its walks
+// are short: 1 (829 us at 1, 836 / 863 / 876 at 2 / 3 / 4).
 constexpr int kWalkSteps = 4;
 
 // Paths that a warp claims per queue fetch: `most`, the caller's number (by

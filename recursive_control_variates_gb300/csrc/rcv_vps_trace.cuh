@@ -456,8 +456,10 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
     }
 
     // ------------------------------ cooperative walk of the warp's last paths
+    bool many = false;  // too many lanes walk for it
     if (!kSG && queue_empty) {
       const unsigned m_coop = __ballot_sync(0xffffffffu, !finished && (phase == kVMain || phase == kVNee));
+      many = __popc(m_coop) > kCoopMost;
       if (m_coop != 0u && __popc(m_coop) <= kCoopMost) {
         float* s = s_coop + (threadIdx.x >> 5) * 64;
         vps_coop<kMode>(m_coop, phase == kVMain, J, rng, mu, inv_mu, p, w, rem, acc, s, s + 32, Q, tc, rec, lost);
@@ -466,7 +468,7 @@ __device__ void trace_vps(const VolJob& J, const VpsParams& P, const Queue& Q) {
 
     // ---------------------------------------------------- free-flight step
     // (several before the next look at the lanes that wait, see kWalkSteps)
-    const int steps = kSG || queue_empty ? 1 : kWalkSteps;
+    const int steps = kSG || (queue_empty && !many) ? 1 : kWalkSteps;
 #pragma unroll 1
     for (int sub = 1;; ++sub) {
       bool ev = false;  // kVpsTape: a shadow-walk step with a gradient, at p
