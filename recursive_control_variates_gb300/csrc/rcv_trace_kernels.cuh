@@ -26,12 +26,13 @@ __device__ __forceinline__ void add_counts(unsigned long long* counters, const C
 
 // Resident blocks per SM that a tracer's registers are bounded for.  More
 // warps hide more of the walk's latency but slow each of the longest paths, on
-// which a launch ends: the single-state tracer of target renders (56 registers
-// suffice) 5 / 6 / 7 / 8 / 9 blocks 17.3 / 16.6 / 15.5 / 14.8 / 14.5 ms at 512^2
-// x 256 spp; the other primal passes alone end on their tails from 7 on; the
-// replays spill below 96 registers.
+// which a launch ends: the single-state tracer of target renders 8 (64
+// registers; 512^2 x 256 spp 7.80 ms, 9 blocks 7.85; with one step per iteration 5 /
+// 6 / 7 / 8 / 9 blocks were 17.3 / 16.6 / 15.5 / 14.8 / 14.5 ms); the other primal
+// passes alone end on their tails from 7 on (three map-lit DRT views 1.818 ms at
+// 6, 1.837 at 7); the replays spill below 96 registers.
 constexpr int tracer_blocks(int mode) {
-  return mode == kSingle ? 9 : (mode == kReplay || mode == kForward ? 5 : 6);
+  return mode == kSingle ? 8 : (mode == kReplay || mode == kForward ? 5 : 6);
 }
 
 template <int kMode, bool kSG, bool kCount, bool kEnv, bool kTable>
