@@ -228,12 +228,13 @@ int rcv_medium_prepare(const rcv_medium* medium, void* stream);
 /* ------------------------------------------------------------- tracers  */
 /* Scratch a tracer call needs (work-queue counter, pixel order, per-pixel
  * cost and, for the primal tracers, one radiance slot per path; for the
- * adjoint 476 B per path: total radiance, 2 scatter checkpoints or event
+ * adjoint 480 B per path: total radiance, 2 scatter checkpoints or event
  * records with their weights, 16 tape slots of 16 B each with a 4-B
- * extinction term, camera-segment weight, entered- and lost-path lists): 256-B aligned device memory of this size, passed as
- * `workspace`.  The per-pixel cost persists from call to call
- * (RCV_ORDER_COST); pass the same workspace to the calls of one image size.
- * mode = RCV_MODE_*. */
+ * extinction term, camera-segment weight, entered- and lost-path lists; calls
+ * of 4.2 M paths or fewer have 4 times the slots and checkpoints, 1.8 KB):
+ * 256-B aligned device memory of this size, passed as `workspace`.  The
+ * per-pixel cost persists from call to call (RCV_ORDER_COST); pass the same
+ * workspace to the calls of one image size.  mode = RCV_MODE_*. */
 uint64_t rcv_render_workspace_bytes(int32_t width, int32_t height, int32_t spp, int32_t mode);
 
 /* Two-state primal: renders the previous (img_old = H) and current

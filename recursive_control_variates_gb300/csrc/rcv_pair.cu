@@ -22,10 +22,11 @@
 namespace rcv {
 
 // kBlocks: resident blocks per SM that the registers are bounded for: 7 (72
-// registers, none spilled) but under an environment map, whose launches end on
-// longer paths, 6.  Paired launch at 6 / 7 / 8 blocks: 512^2 x (16 + 16) spp on
-// 64^3 1477 / 1430 / 1466 us, 1024^2 on 256^3 5.79 / 5.25 / 5.62 ms, 24 mixed
-// jobs 12.8 / 12.5 / 13.5 ms, five map-lit 107 x 83 views 791 / 817 / 846 us.
+// registers, up to 80 bytes spilled) but under an environment map, whose launches
+// end on longer paths, 6.  Steps at 6 / 7 blocks: 512^2 x (16 + 16) spp on 64^3
+// 1663 / 1630 us, 1024^2 on 256^3 8.84 / 8.66 ms, 24 mixed jobs 15.85 / 15.63 ms,
+// five map-lit 107 x 83 views 839 / 865 us; at 8 the paired launch was 2 to 8 %
+// slower than at 7 (with one step per iteration).
 template <bool kSG, bool kEnv, bool kTable, int kBlocks>
 __global__ void __launch_bounds__(kTraceBlock, kBlocks)
     trace_pair_kernel(const __grid_constant__ VolJob JA, const __grid_constant__ Queue QA,

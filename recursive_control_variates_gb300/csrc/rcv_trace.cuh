@@ -3,7 +3,8 @@
 // Every warp pulls batches of path indices from one global counter and hands
 // them to idle lanes.  A lane is always in one of these phases:
 //   kStart    path (or adjoint replay pass) waiting to be initialised
-//   kMain     walking the main path: one free-flight step per iteration
+//   kMain     walking the main path: up to kWalkSteps free-flight steps per
+//             iteration
 //   kScatter  real scattering event waiting to be processed (albedo lookups,
 //             phase and NEE direction sampling, adjoint scatter)
 //   kNee      walking the NEE shadow ray (ratio tracking)

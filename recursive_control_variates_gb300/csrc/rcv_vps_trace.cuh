@@ -5,9 +5,11 @@
 // inside a segment, segments of a path, the paths traced twice and a third
 // one for differential ratio tracking).  At 512^2, 16 spp, depth 64 that
 // launch took 13.1 ms at a few lanes per instruction.  Here the adjoint is
-// two persistent launches with one free-flight step per loop iteration for
+// two persistent launches with a few free-flight steps per loop iteration for
 // every lane, whatever its phase (as in rcv_trace.cuh), and two flat passes;
-// on the same film 0.94 + 0.80 + 0.26 + 0.11 ms (GB300).  The tracers are
+// on the same film 0.94 + 0.80 + 0.26 + 0.11 ms (GB300; with one step per
+// iteration, before the reductions went pairwise: the whole step has gone from
+// 2.97 to 2.50 ms since).  The tracers are
 // bound by the issue of divergent instructions and end on their longest
 // paths (a DRT path that follows its first path in the same lane and launch
 // gives 2.0 ms for the two tracers), the flat passes by the vector reductions
