@@ -26,6 +26,16 @@ def _twostate_types():
     return (TwoStatePRBIntegrator, TwoStatePRBVolpathIntegrator)
 
 
+def _prefetch(adjoint, primal, twostates: bool, scene, sensor, seed: int, spp: int):
+    """The adjoint's ``prefetch_adjoint`` (None without one); ``twostates``: the
+    step's primal render is a ``render_twostates`` of ``primal``, which takes
+    the adjoint's radiance pass when both are one volume integrator."""
+    if twostates and adjoint is primal and type(adjoint) is TwoStatePRBVolpathIntegrator:
+        return adjoint._prefetch(scene, sensor, seed, spp, True)
+    pre = getattr(adjoint, "prefetch_adjoint", None)
+    return pre(scene, sensor, seed, spp) if pre is not None else None
+
+
 class _CVState:
     """Device buffers of the control variate: img, w_s, v_n plus the
     statistics (all zero-initialised like the reference's scalar zeros)."""
@@ -123,8 +133,7 @@ class CVIntegrator:
         return self.adjoint_integrator.render_backward(scene, params, grad_in, sensor, seed, spp)
 
     def prefetch_adjoint(self, scene, sensor=0, seed: int = 0, spp: int = 0):
-        pre = getattr(self.adjoint_integrator, "prefetch_adjoint", None)
-        return pre(scene, sensor, seed, spp) if pre is not None else None
+        return _prefetch(self.adjoint_integrator, self.integrator, True, scene, sensor, seed, spp)
 
 
 class MetaIntegrator:
@@ -203,5 +212,4 @@ class MetaIntegrator:
         return self.adjoint_integrator.render_backward(scene, params, grad_in, sensor, seed, spp)
 
     def prefetch_adjoint(self, scene, sensor=0, seed: int = 0, spp: int = 0):
-        pre = getattr(self.adjoint_integrator, "prefetch_adjoint", None)
-        return pre(scene, sensor, seed, spp) if pre is not None else None
+        return _prefetch(self.adjoint_integrator, self.integrator, self.method == "cv_ps", scene, sensor, seed, spp)

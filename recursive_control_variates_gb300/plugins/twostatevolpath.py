@@ -153,6 +153,12 @@ class _VolumeIntegratorBase:
         medium state, sensor and options called before that function runs
         the pass in its own launch instead, and the function does nothing.
         ``render_backward`` with the same arguments then only replays."""
+        return self._prefetch(scene, sensor, seed, spp, False)
+
+    def _prefetch(self, scene, sensor, seed: int, spp: int, twostates_next: bool):
+        """``prefetch_adjoint``; with ``twostates_next`` the caller goes on with
+        a ``render_twostates`` of this integrator, which takes the pass: the
+        event that only the side stream would wait for is then not recorded."""
         if not self.overlap_adjoint:
             return None
         medium = self._checked_medium(scene)
@@ -168,11 +174,8 @@ class _VolumeIntegratorBase:
         counters = self.counters_ptr(dev)
         pending = {"key": key, "seed": seed, "spp": spp, "ws": ws, "used": False}
         self._pending = pending if self.pair_adjoint else None
-        # where a render_twostates will most likely take the pass, the point
-        # that a pass on the side stream has to wait for is not recorded now:
-        # should it go there after all, it waits for the launches up to then
         packed = None
-        if not (self.pair_adjoint and self.two_state):
+        if not (twostates_next and self.pair_adjoint):
             packed = torch.cuda.Event()
             packed.record(main)
 
@@ -185,7 +188,7 @@ class _VolumeIntegratorBase:
             side = self._side.get(dev)
             if side is None:
                 side = self._side[dev] = torch.cuda.Stream(dev)
-            if packed is None:
+            if packed is None:  # the render did not take the pass after all
                 side.wait_stream(main)
             else:
                 side.wait_event(packed)
