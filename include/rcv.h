@@ -428,6 +428,12 @@ typedef struct rcv_surface_scene {
 /* Workspace of a surface scene: texture state pairs and gradient. */
 uint64_t rcv_surface_workspace_bytes(int32_t tex_width, int32_t tex_height);
 
+/* Scratch of a surface call (256-B aligned device memory): the primal modes as
+ * rcv_render_workspace_bytes; RCV_MODE_ADJOINT (both adjoints and forward
+ * mode) 276 B per path: total radiance, 16 tape slots of 16 B, lost-path
+ * list. */
+uint64_t rcv_render_surface_workspace_bytes(int32_t width, int32_t height, int32_t spp, int32_t mode);
+
 /* Packs the old / new textures after a state rotation
  * (TwoStateBSDF.parameters_changed, plugins/twostatebsdf.py:46-56). */
 int rcv_surface_prepare(const rcv_surface_scene* scene, void* stream);
@@ -435,8 +441,8 @@ int rcv_surface_prepare(const rcv_surface_scene* scene, void* stream);
 /* Two-state surface primal (H = old, F = new), replacing
  * TwoStatePRBIntegrator.render_twostates / sample_twostates
  * (plugins/twostatepath.py:179-223, 225-364) with the two-state BSDF of
- * plugins/twostatebsdf.py:25-38.  Scratch: rcv_render_workspace_bytes(...,
- * RCV_MODE_TWOSTATE). */
+ * plugins/twostatebsdf.py:25-38.  Scratch:
+ * rcv_render_surface_workspace_bytes(..., RCV_MODE_TWOSTATE). */
 int rcv_render_twostates_surface(const rcv_surface_scene* scene, const rcv_sensor* sensor,
                                  const rcv_volpath_options* opts, uint32_t seed, int32_t spp,
                                  float* img_old, float* img_new, void* workspace,
@@ -454,7 +460,7 @@ int rcv_render_surface(const rcv_surface_scene* scene, const rcv_sensor* sensor,
  * opts->adjoint: RCV_ADJOINT_TAPE traces each path once, recording its
  * texture vertices (2 of the 16 tape slots per path each), and scatters them
  * once L is known; RCV_ADJOINT_REPLAY traces each path a second time.
- * Scratch: rcv_render_workspace_bytes(..., RCV_MODE_ADJOINT). */
+ * Scratch: rcv_render_surface_workspace_bytes(..., RCV_MODE_ADJOINT). */
 int rcv_render_backward_surface(const rcv_surface_scene* scene, const rcv_sensor* sensor,
                                 const rcv_volpath_options* opts, uint32_t seed, int32_t spp,
                                 const float* grad_img, float* grad_texture, void* workspace,

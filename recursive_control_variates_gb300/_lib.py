@@ -269,6 +269,7 @@ SIGNATURES = {
         [P(Medium), P(Sensor), P(VolpathOptions), P(VpsFlags), C.c_uint32, C.c_int32, vp, vp, vp, vp, C.c_uint64, vp],
     ),
     "rcv_surface_workspace_bytes": (C.c_uint64, [C.c_int32, C.c_int32]),
+    "rcv_render_surface_workspace_bytes": (C.c_uint64, [C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "rcv_surface_prepare": (C.c_int, [P(SurfaceScene), vp]),
     "rcv_render_twostates_surface": (
         C.c_int, [P(SurfaceScene), P(Sensor), P(VolpathOptions), C.c_uint32, C.c_int32, vp, vp, vp, vp, vp]

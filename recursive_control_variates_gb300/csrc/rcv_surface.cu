@@ -214,17 +214,44 @@ static int launch_surface(int mode, const SurfJob& S, const Queue& Q, const rcv_
   return launched("trace_surface launch");
 }
 
+// The tape adjoint's slots are 32-bit indices.
+static bool surface_tape_fits(int64_t paths) { return paths < (int64_t(1) << 28); }
+
+// Scratch of one call (256-byte aligned sections): counters | primal passes:
+// the sections of render_layout | tape adjoint: per-path radiance | tape (16 bytes
+// a slot, kTapeSlotsPerPath per path) | lost list.  Replay and forward mode
+// need the counters alone.
+struct SurfCallLayout {
+  uint64_t path_out, ltot, tape, lost, total;
+};
+
+static SurfCallLayout surf_call_layout(int64_t npix, int64_t paths, int mode) {
+  SurfCallLayout L{};
+  if (mode != RCV_MODE_ADJOINT) {
+    const RenderLayout R = render_layout(npix, paths, mode);
+    L.path_out = R.path_out;
+    L.total = R.total;
+    return L;
+  }
+  const uint64_t n = surface_tape_fits(paths) ? (uint64_t)paths : 0u;
+  L.ltot = 256;
+  L.tape = align256(L.ltot + n * 16u);
+  L.lost = align256(L.tape + uint64_t(tape_capacity((int64_t)n, kTapeSlotsPerPath)) * 16u);
+  L.total = align256(L.lost + n * 4u);
+  return L;
+}
+
 static int run_surface(int mode, const SurfJob& S, const rcv_volpath_options* o, void* workspace,
                        uint64_t* counters, float* img_new, float* img_old, cudaStream_t st) {
   RCV_REQUIRE(workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0,
               "render workspace must be non-NULL and 256-byte aligned");
   const int64_t npix = int64_t(S.width) * S.height;
-  const RenderLayout L = render_layout(npix, S.path_count, mode);
+  const bool adj = mode == kAdjoint || mode == kForward;
+  const SurfCallLayout L = surf_call_layout(npix, S.path_count, adj ? RCV_MODE_ADJOINT : mode);
   char* ws = static_cast<char*>(workspace);
   Queue Q;
   std::memset(&Q, 0, sizeof(Q));
-  Q.counter = reinterpret_cast<unsigned long long*>(ws + L.counter);
-  const bool adj = mode == kAdjoint || mode == kForward;
+  Q.counter = reinterpret_cast<unsigned long long*>(ws);
   Q.path_out = adj ? nullptr : reinterpret_cast<float4*>(ws + L.path_out);
   Q.counters = reinterpret_cast<unsigned long long*>(counters);
   Q.total = S.path_count;
@@ -233,7 +260,7 @@ static int run_surface(int mode, const SurfJob& S, const rcv_volpath_options* o,
   Q.defer = 1;
   const int adjoint = o == nullptr ? RCV_ADJOINT_TAPE : o->adjoint;
   RCV_REQUIRE(adjoint == RCV_ADJOINT_TAPE || adjoint == RCV_ADJOINT_REPLAY, "unknown adjoint %d", adjoint);
-  if (mode == kAdjoint && adjoint == RCV_ADJOINT_TAPE && S.path_count < (int64_t(1) << 28)) {
+  if (mode == kAdjoint && adjoint == RCV_ADJOINT_TAPE && surface_tape_fits(S.path_count)) {
     // one pass records the texture vertices, one flat pass scatters them, and
     // the replay takes the paths whose vertices did not fit (2 slots each)
     const int per_path = (o == nullptr || o->tape_events_per_path == 0) ? int(kTapeSlotsPerPath)
@@ -271,6 +298,12 @@ using namespace rcv;
 extern "C" uint64_t rcv_surface_workspace_bytes(int32_t tex_width, int32_t tex_height) {
   if (tex_width <= 0 || tex_height <= 0) return 0;
   return surf_layout(tex_width, tex_height).total;
+}
+
+extern "C" uint64_t rcv_render_surface_workspace_bytes(int32_t width, int32_t height, int32_t spp, int32_t mode) {
+  if (width <= 0 || height <= 0 || spp <= 0 || mode < 0 || mode > 2) return 0;
+  const int64_t npix = int64_t(width) * height;
+  return surf_call_layout(npix, npix * spp, mode).total;
 }
 
 extern "C" int rcv_surface_prepare(const rcv_surface_scene* sc, void* stream) {

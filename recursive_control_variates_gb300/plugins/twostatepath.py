@@ -65,7 +65,7 @@ class TwoStatePRBIntegrator:
     def scratch(self, device, sensor, spp: int, mode: int) -> int:
         device = torch.device(device)
         f = sensor.film()
-        need = int(_lib.load().rcv_render_workspace_bytes(f.width, f.height, spp, mode)) + 256
+        need = int(_lib.load().rcv_render_surface_workspace_bytes(f.width, f.height, spp, mode)) + 256
         buf = self._scratch.get(device)
         if buf is None or buf.numel() < need:
             buf = torch.empty(need, dtype=torch.uint8, device=device)
