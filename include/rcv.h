@@ -161,9 +161,11 @@ typedef struct rcv_volpath_options {
    * and jobs (or batches) of 2^28 gradient paths or more always replay.  The
    * batched engine takes the same choice. */
   int32_t adjoint;
-  /* Tape slots per path, 1..16 (0 = the room that the adjoint workspace
-   * holds: 16 per path, up to 64 in single-job calls of 4.2 M paths or
-   * fewer): paths whose events do not fit are replayed whole. */
+  /* Tape slots per path: paths whose events do not fit are replayed whole.  0 =
+   * the most: max(16 per path, min(64 per path, 2^28)) in single-job calls, 16
+   * per path in batches.  1..16 bounds the slots in use and asks for scratch
+   * of 16 per path (rcv_render_adjoint_workspace_bytes).  The calls of one
+   * gradient (radiance pass, replay) take the same value. */
   int32_t tape_events_per_path;
   /* The two-state pass and the adjoint's radiance pass of a step as two
    * launches (1; the batched engine runs them on two streams) instead of one
@@ -228,14 +230,22 @@ int rcv_medium_prepare(const rcv_medium* medium, void* stream);
 /* ------------------------------------------------------------- tracers  */
 /* Scratch a tracer call needs (work-queue counter, pixel order, per-pixel
  * cost and, for the primal tracers, one radiance slot per path; for the
- * adjoint 480 B per path: total radiance, 2 scatter checkpoints or event
- * records with their weights, 16 tape slots of 16 B each with a 4-B
- * extinction term, camera-segment weight, entered- and lost-path lists; calls
- * of 4.2 M paths or fewer have 4 times the slots and checkpoints, 1.8 KB):
+ * adjoint, whatever its options, total radiance, scatter checkpoints of 64 B
+ * or event records with their weights, tape slots of 16 B each with a 4-B
+ * extinction term, camera-segment weight, entered- and lost-path lists: n
+ * paths have max(16 n, min(64 n, 2^28)) slots and one checkpoint for every 8,
+ * i.e. 1.8 KB per path up to 4.2 M paths, 7.5 GB and 32 B per path up to
+ * 16.8 M and 480 B per path beyond):
  * 256-B aligned device memory of this size, passed as `workspace`.  The
  * per-pixel cost persists from call to call (RCV_ORDER_COST); pass the same
  * workspace to the calls of one image size.  mode = RCV_MODE_*. */
 uint64_t rcv_render_workspace_bytes(int32_t width, int32_t height, int32_t spp, int32_t mode);
+
+/* Scratch of the volume adjoint and forward-mode calls with these options, at
+ * most the RCV_MODE_ADJOINT size above: 480 B per path (and 4.2 MB) with
+ * tape_events_per_path from 1 to 16, less with RCV_ADJOINT_REPLAY. */
+uint64_t rcv_render_adjoint_workspace_bytes(int32_t width, int32_t height, int32_t spp,
+                                            const rcv_volpath_options* opts);
 
 /* Two-state primal: renders the previous (img_old = H) and current
  * (img_new = F) parameters with shared random numbers.  Images are

@@ -82,7 +82,7 @@ class VolpathOptions(C.Structure):
         ("count_events", C.c_int32),
         ("envmap", C.c_void_p),  # const rcv_envmap* or NULL (constant environment)
         ("adjoint", C.c_int32),  # ADJOINT_TAPE / ADJOINT_REPLAY
-        ("tape_events_per_path", C.c_int32),  # 1..16, 0 = 16
+        ("tape_events_per_path", C.c_int32),  # 1..16, 0 = the room of the scratch (up to 64)
         ("separate_tracers", C.c_int32),  # 1: two-state and adjoint radiance passes as two launches
     ]
 
@@ -225,6 +225,7 @@ SIGNATURES = {
     "rcv_envmap_workspace_bytes": (C.c_uint64, [C.c_int32, C.c_int32]),
     "rcv_envmap_prepare": (C.c_int, [P(Envmap), vp]),
     "rcv_render_workspace_bytes": (C.c_uint64, [C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "rcv_render_adjoint_workspace_bytes": (C.c_uint64, [C.c_int32, C.c_int32, C.c_int32, P(VolpathOptions)]),
     "rcv_render_twostates_volume": (
         C.c_int,
         [P(Medium), P(Sensor), P(VolpathOptions), C.c_uint32, C.c_int32, vp, vp, vp, vp, vp],

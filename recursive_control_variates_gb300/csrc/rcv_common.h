@@ -161,30 +161,56 @@ inline int64_t tape_room(int64_t paths) {
 // replayed whole.  The tape adjoint keeps its 32-byte event records in the
 // first half of the same buffer and their 32-byte weights in the second.
 constexpr int64_t kCkptMargin = 65536;
-inline int64_t ckpt_capacity(int64_t paths) {
-  return within_budget(paths, kTapeSlotsPerPath / 8, kTapeSlotsMost / 8, kTapeSlotBudget / 8) + kCkptMargin;
+inline int64_t ckpt_capacity(int64_t paths, int64_t most) {
+  return within_budget(paths, kTapeSlotsPerPath / 8, most, kTapeSlotBudget / 8) + kCkptMargin;
+}
+
+// Room of a volume adjoint call: tape slots (0: no tape) and checkpoints.
+struct AdjRoom {
+  int64_t slots, ckpts;
+};
+
+// The tape's slots are 32-bit indices.
+inline bool tape_fits(int64_t paths) { return paths < (int64_t(1) << 28); }
+
+// The most that a call of these options can use.  tape_events_per_path from 1 to
+// 16 asks for 16 slots and 2 checkpoints per path (480 B in all: callers whose
+// GPU does not hold the room of 64, 1.8 KB).  Without a tape (replay, forward
+// mode) 7 checkpoints per path come to less than that.
+inline AdjRoom adjoint_room(int64_t paths, const rcv_volpath_options* o, bool forward) {
+  if (forward || !tape_fits(paths) || (o != nullptr && o->adjoint == RCV_ADJOINT_REPLAY))
+    return AdjRoom{0, ckpt_capacity(paths, 7)};
+  if (o != nullptr && o->tape_events_per_path > 0)
+    return AdjRoom{tape_capacity(paths, kTapeSlotsPerPath), ckpt_capacity(paths, 0)};
+  return AdjRoom{tape_room(paths), ckpt_capacity(paths, kTapeSlotsMost / 8)};
 }
 
 inline uint64_t path_out_bytes(int64_t paths, int mode) {
   return mode == RCV_MODE_ADJOINT ? 0u : uint64_t(paths) * (mode == RCV_MODE_TWOSTATE ? 32u : 16u);
 }
 
-inline RenderLayout render_layout(int64_t npix, int64_t paths, int mode) {
+inline RenderLayout render_layout(int64_t npix, int64_t paths, int mode, const AdjRoom& room) {
   RenderLayout L;
   L.counter = 0;
   L.buckets = 256;
   L.order = align256(kRenderHeadBytes);
   L.cost = align256(L.order + uint64_t(npix) * sizeof(uint32_t));
   L.path_out = align256(L.cost + uint64_t(npix) * sizeof(uint32_t));
-  const bool adj = mode == RCV_MODE_ADJOINT;
+  const uint64_t adj = mode == RCV_MODE_ADJOINT ? uint64_t(paths) : 0u;
+  const uint64_t tape = room.slots > 0 ? adj : 0u;
   L.ltot = align256(L.path_out + path_out_bytes(paths, mode));
-  L.ckpt = align256(L.ltot + (adj ? uint64_t(paths) * 16u : 0u));
-  L.tape = align256(L.ckpt + (adj ? uint64_t(ckpt_capacity(paths)) * 64u : 0u));
-  L.cam_w = align256(L.tape + (adj ? uint64_t(tape_room(paths)) * 20u : 0u));
-  L.entered = align256(L.cam_w + (adj ? uint64_t(paths) * 8u : 0u));
-  L.lost = align256(L.entered + (adj ? uint64_t(paths) * 4u : 0u));
-  L.total = align256(L.lost + (adj ? uint64_t(paths) * 4u : 0u));
+  L.ckpt = align256(L.ltot + adj * 16u);
+  L.tape = align256(L.ckpt + (adj > 0u ? uint64_t(room.ckpts) * 64u : 0u));
+  L.cam_w = align256(L.tape + (adj > 0u ? uint64_t(room.slots) * 20u : 0u));
+  L.entered = align256(L.cam_w + tape * 8u);
+  L.lost = align256(L.entered + tape * 4u);
+  L.total = align256(L.lost + tape * 4u);
   return L;
+}
+
+// The same for the primal passes, and for an adjoint with room for any options.
+inline RenderLayout render_layout(int64_t npix, int64_t paths, int mode) {
+  return render_layout(npix, paths, mode, AdjRoom{tape_room(paths), ckpt_capacity(paths, kTapeSlotsMost / 8)});
 }
 
 // Per-pixel sum of per-path radiance slots in sample order (rcv_volume.cu).

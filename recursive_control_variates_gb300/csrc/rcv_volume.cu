@@ -665,6 +665,15 @@ extern "C" uint64_t rcv_render_workspace_bytes(int32_t width, int32_t height, in
   return render_layout(npix, npix * spp, mode).total;
 }
 
+extern "C" uint64_t rcv_render_adjoint_workspace_bytes(int32_t width, int32_t height, int32_t spp,
+                                                       const rcv_volpath_options* o) {
+  if (width <= 0 || height <= 0 || spp <= 0) return 0;
+  const int64_t npix = int64_t(width) * height, paths = npix * spp;
+  const uint64_t forward = render_layout(npix, paths, kAdjoint, adjoint_room(paths, o, true)).total;
+  const uint64_t backward = render_layout(npix, paths, kAdjoint, adjoint_room(paths, o, false)).total;
+  return backward > forward ? backward : forward;
+}
+
 extern "C" int rcv_medium_prepare(const rcv_medium* m, void* stream) {
   int rc = validate_medium(m);
   if (rc) return rc;
@@ -734,11 +743,9 @@ static int order_job(VolJob& J, const rcv_volpath_options* o, char* ws, const Re
 }
 
 // The gradient comes from the event tape (RCV_ADJOINT_TAPE), except in forward
-// mode and for jobs of 2^28 paths or more, whose tape slots would not fit
-// 32-bit indices.
+// mode and for jobs of too many paths.
 static bool uses_tape(const VolJob& J, const rcv_volpath_options* o, int stage) {
-  return (o == nullptr || o->adjoint == RCV_ADJOINT_TAPE) && stage != kAdjForward &&
-         J.path_count < (int64_t(1) << 28);
+  return (o == nullptr || o->adjoint == RCV_ADJOINT_TAPE) && stage != kAdjForward && tape_fits(J.path_count);
 }
 
 // float4s of a job's density (or albedo) gradient records.
@@ -757,12 +764,13 @@ static bool clears_in_weights(const VolJob& J) {
 // Adjoint buffers of a job in its workspace (queue counters at qc: hand-out,
 // records, tape slots, lost paths).  *tape: the gradient comes from the tape.
 static int adjoint_buffers(const VolJob& J, const rcv_volpath_options* o, char* ws, const RenderLayout& L,
-                           unsigned long long* qc, int stage, AdjBuffers* out, bool* tape_out) {
+                           const AdjRoom& room, unsigned long long* qc, int stage, AdjBuffers* out,
+                           bool* tape_out) {
   AdjBuffers& A = *out;
   std::memset(&A, 0, sizeof(A));
   A.ckpt = reinterpret_cast<float4*>(ws + L.ckpt);
   A.ckpt_count = qc + 1;
-  A.ckpt_cap = ckpt_capacity(J.path_count);
+  A.ckpt_cap = room.ckpts;
   A.path_ltot = reinterpret_cast<float4*>(ws + L.ltot);
   const int adjoint = o == nullptr ? RCV_ADJOINT_TAPE : o->adjoint;
   const int per_path = o == nullptr ? 0 : o->tape_events_per_path;
@@ -773,10 +781,10 @@ static int adjoint_buffers(const VolJob& J, const rcv_volpath_options* o, char* 
   if (tape) {
     A.tape = reinterpret_cast<float4*>(ws + L.tape);
     A.tape_count = qc + 2;
-    A.tape_cap = per_path > 0 ? tape_capacity(J.path_count, per_path) : tape_room(J.path_count);
+    A.tape_cap = per_path > 0 ? tape_capacity(J.path_count, per_path) : room.slots;
     A.lost_list = reinterpret_cast<uint32_t*>(ws + L.lost);
     A.lost_count = qc + 3;
-    A.tape_f = tape_terms(ws + L.tape, tape_room(J.path_count));
+    A.tape_f = tape_terms(ws + L.tape, room.slots);
     A.cam_w = reinterpret_cast<float2*>(ws + L.cam_w);
     A.entered = reinterpret_cast<uint32_t*>(ws + L.entered);
     A.entered_count = qc + 5;
@@ -797,7 +805,8 @@ static int run_single_job(int mode, VolJob& J, const rcv_volpath_options* o, voi
   int rc = check_workspace(workspace);
   if (rc) return rc;
   const int64_t npix = int64_t(J.width) * J.height;
-  const RenderLayout L = render_layout(npix, J.path_count, mode);
+  const AdjRoom room = adjoint_room(J.path_count, o, stage == kAdjForward);
+  const RenderLayout L = render_layout(npix, J.path_count, mode, room);
   char* ws = static_cast<char*>(workspace);
   OrderJob sort[1];
   int nsort = 0;
@@ -809,7 +818,7 @@ static int run_single_job(int mode, VolJob& J, const rcv_volpath_options* o, voi
   if (mode == kAdjoint) {
     AdjBuffers A;
     bool tape = false;
-    rc = adjoint_buffers(J, o, ws, L, qc, stage, &A, &tape);
+    rc = adjoint_buffers(J, o, ws, L, room, qc, stage, &A, &tape);
     if (rc) return rc;
     if (stage != kAdjReplay) {
       rc = launch_persistent(tape ? kTape : kAdjoint, J, nullptr, 0, J.path_count, o, qc, nullptr, &A, counters,
@@ -877,14 +886,15 @@ extern "C" int rcv_render_twostates_volume_and_adjoint_radiance(
   if (rc) return rc;
   const int64_t npix = int64_t(JA.width) * JA.height;
   const RenderLayout LA = render_layout(npix, JA.path_count, kTwoState);
-  const RenderLayout LB = render_layout(npix, JB.path_count, kAdjoint);
+  const AdjRoom room = adjoint_room(JB.path_count, o, false);
+  const RenderLayout LB = render_layout(npix, JB.path_count, kAdjoint, room);
   char* wa = static_cast<char*>(workspace);
   char* wb = static_cast<char*>(adjoint_workspace);
   unsigned long long* qa = reinterpret_cast<unsigned long long*>(wa + LA.counter);
   unsigned long long* qb = reinterpret_cast<unsigned long long*>(wb + LB.counter);
   AdjBuffers A;
   bool tape = false;
-  rc = adjoint_buffers(JB, o, wb, LB, qb, kAdjRadiance, &A, &tape);
+  rc = adjoint_buffers(JB, o, wb, LB, room, qb, kAdjRadiance, &A, &tape);
   if (rc) return rc;
   if (counters != nullptr || !tape || (o != nullptr && o->separate_tracers)) {
     rc = run_single_job(kTwoState, JA, o, workspace, counters, img_new, img_old, st);

@@ -73,6 +73,7 @@ class _VolumeIntegratorBase:
         self._counters: dict[torch.device, torch.Tensor] = {}
         self._scratch: dict[torch.device, torch.Tensor] = {}
         self._adj_scratch: dict[torch.device, torch.Tensor] = {}
+        self._adj_refused: dict[torch.device, int] = {}  # smallest adjoint scratch that did not fit the GPU
         self._side: dict[torch.device, torch.cuda.Stream] = {}
         self._ticket = None  # (key, done event) of an adjoint radiance pass started ahead
         self._pending = None  # a prepared radiance pass the next two-state render may run with it
@@ -119,18 +120,35 @@ class _VolumeIntegratorBase:
             self._scratch[device] = buf
         return (buf.data_ptr() + 255) & ~255
 
-    def adjoint_scratch(self, device, sensor, spp: int) -> int:
+    def adjoint_scratch(self, device, sensor, spp: int, o: _lib.VolpathOptions | None = None) -> int:
         """256-B aligned scratch of the adjoint launches (its own buffer, so
         an adjoint radiance pass on the side stream never shares scratch with
-        a primal render)."""
+        a primal render), for the options `o`.  On a GPU without room for the
+        large event tape, `o` receives the 16 slots per path that the smaller
+        scratch has (more paths are replayed whole; the same gradient)."""
         device = torch.device(device)
         f = sensor.film()
-        need = int(_lib.load().rcv_render_workspace_bytes(f.width, f.height, spp, _lib.MODE_ADJOINT)) + 256
-        buf = self._adj_scratch.get(device)
-        if buf is None or buf.numel() < need:
+        o = self.options() if o is None else o
+        lib = _lib.load()
+        while True:
+            need = int(lib.rcv_render_adjoint_workspace_bytes(f.width, f.height, spp, C.byref(o))) + 256
+            buf = self._adj_scratch.get(device)
+            if buf is not None and buf.numel() >= need:
+                break
+            smaller = o.adjoint == _lib.ADJOINT_TAPE and o.tape_events_per_path == 0
+            if smaller and need >= self._adj_refused.get(device, need + 1):
+                o.tape_events_per_path = 16
+                continue
             self._drain_ticket(device)  # the old buffer may still be in use
-            buf = _new_scratch(need, f, device)
-            self._adj_scratch[device] = buf
+            del buf
+            self._adj_scratch.pop(device, None)
+            try:
+                buf = self._adj_scratch[device] = _new_scratch(need, f, device)
+                break
+            except torch.cuda.OutOfMemoryError:
+                if not smaller:
+                    raise
+                self._adj_refused[device] = need
         return (buf.data_ptr() + 255) & ~255
 
     def _drain_ticket(self, device):
@@ -169,10 +187,11 @@ class _VolumeIntegratorBase:
         m = medium.prepare(main.cuda_stream)
         s = sensor.c_struct()
         o = self.options(scene)
-        ws = self.adjoint_scratch(dev, sensor, spp)
         key = self._adjoint_key(o, medium, sensor, seed, spp)
+        ws = self.adjoint_scratch(dev, sensor, spp, o)
+        slots = o.tape_events_per_path
         counters = self.counters_ptr(dev)
-        pending = {"key": key, "seed": seed, "spp": spp, "ws": ws, "used": False}
+        pending = {"key": key, "seed": seed, "spp": spp, "ws": ws, "slots": slots, "used": False}
         self._pending = pending if self.pair_adjoint else None
         packed = None
         if not (twostates_next and self.pair_adjoint):
@@ -203,7 +222,7 @@ class _VolumeIntegratorBase:
             done = torch.cuda.Event()
             done.record(side)
             medium.add_reader(done)
-            self._ticket = (key, done)
+            self._ticket = (key, done, slots)
 
         return launch
 
@@ -287,10 +306,10 @@ class _VolumeIntegratorBase:
         dx, dy, dz = medium.dims
         gd = torch.zeros((dz, dy, dx, 1), dtype=torch.float32, device=dev)
         ga = medium.albedo_grad_buffer()
-        ws = self.adjoint_scratch(dev, sensor, spp)
+        ws = self.adjoint_scratch(dev, sensor, spp, o)
         # the radiance pass already ran for exactly these arguments: replay only
         fn = ("rcv_render_backward_replay" if ticket is not None and ticket[0] == key and medium.version == key[1]
-              else "rcv_render_backward_volume")
+              and ticket[2] == o.tape_events_per_path else "rcv_render_backward_volume")
         self.last_adjoint_call = fn
         with profiling.region("trace_adjoint", dev):
             _lib.check(
@@ -354,12 +373,13 @@ class _VolumeIntegratorBase:
         m = medium.prepare(st)
         s = sensor.c_struct()
         o = self.options(scene)
+        o.adjoint = _lib.ADJOINT_REPLAY  # forward mode replays: no room for a tape
         with profiling.region("trace_forward", dev):
             _lib.check(
                 _lib.load().rcv_render_forward_volume(
                     C.byref(m), C.byref(s), C.byref(o), seed & 0xFFFFFFFF, spp,
                     td.data_ptr() if td is not None else None, ta.data_ptr() if ta is not None else None,
-                    out.data_ptr(), self.adjoint_scratch(dev, sensor, spp), self.counters_ptr(dev), st,
+                    out.data_ptr(), self.adjoint_scratch(dev, sensor, spp, o), self.counters_ptr(dev), st,
                 ),
                 "rcv_render_forward_volume",
             )
@@ -417,6 +437,7 @@ class TwoStatePRBVolpathIntegrator(_VolumeIntegratorBase):
             else:
                 fn = "rcv_render_twostates_volume_and_adjoint_radiance"
                 self._drain_ticket(medium.device)  # the call overwrites the adjoint scratch
+                o.tape_events_per_path = pend["slots"]
                 rc = _lib.load().rcv_render_twostates_volume_and_adjoint_radiance(
                     C.byref(m), C.byref(s), C.byref(o), seed & 0xFFFFFFFF, spp, H.data_ptr(), F.data_ptr(), ws,
                     pend["seed"] & 0xFFFFFFFF, pend["spp"], pend["ws"], self.counters_ptr(medium.device), st,
@@ -427,7 +448,7 @@ class TwoStatePRBVolpathIntegrator(_VolumeIntegratorBase):
             done = torch.cuda.Event()
             done.record(torch.cuda.current_stream(medium.device))
             medium.add_reader(done)
-            self._ticket = (pend["key"], done)
+            self._ticket = (pend["key"], done, pend["slots"])
             pend["used"] = True
         self.primal_image_old, self.primal_image_new = self._post(H), self._post(F)
         return self.primal_image_old, self.primal_image_new
