@@ -7,7 +7,7 @@ primal images come from the two-state tracer, the gradients from this
 integrator's adjoint.  Switches (plugins/volpathsimple.py:33-48):
 ``use_nee``, ``use_drt``, ``use_drt_subsampling``, ``use_drt_mis``, all on
 by default.  ``render`` and ``render_backward`` run on the GPU through
-librcv (rcv_render_volpathsimple / rcv_render_backward_volpathsimple).
+librcv (rcv_render_volpathsimple / rcv_render_backward_volpathsimple_ws).
 """
 from __future__ import annotations
 
@@ -39,7 +39,7 @@ class VolpathSimpleIntegrator(PRBVolpathIntegrator):
                                   "use render_backward, or prbvolpath / twostateprbvolpath for forward mode")
 
     def prefetch_adjoint(self, scene, sensor=0, seed: int = 0, spp: int = 0):
-        """The DRT adjoint is one launch per call: nothing to start ahead."""
+        """The adjoint's tracers run in the backward call: nothing is started ahead."""
         return None
 
     def flags(self) -> _lib.VpsFlags:
@@ -60,11 +60,13 @@ class VolpathSimpleIntegrator(PRBVolpathIntegrator):
             self._vps_scratch[device] = buf
         return (buf.data_ptr() + 255) & ~255
 
-    @staticmethod
-    def _adjoint_scratch(device, sensor, spp: int):
+    def _adjoint_scratch(self, device, sensor, spp: int):
         """Scratch of one adjoint call: torch's allocator keeps it for the next
         call on the stream, or hands it to others.  On a nearly full GPU a
-        smaller one (more passes; too small for any, one thread per path)."""
+        smaller one (more passes; too small for any, one thread per path).
+        None for DRT without subsampling, which always runs one thread per path."""
+        if self.use_drt and not self.use_drt_subsampling:
+            return None
         f = sensor.film()
         need = int(_lib.load().rcv_volpathsimple_adjoint_workspace_bytes(f.width, f.height, spp)) + 256
         while need > (1 << 22):
@@ -117,13 +119,15 @@ class VolpathSimpleIntegrator(PRBVolpathIntegrator):
         gd = torch.zeros((dz, dy, dx, 1), dtype=torch.float32, device=medium.device)
         ga = medium.albedo_grad_buffer()
         ws = self._adjoint_scratch(medium.device, sensor, spp)
-        base = (ws.data_ptr() + 255) & ~255
+        base = nbytes = 0
+        if ws is not None:
+            base = (ws.data_ptr() + 255) & ~255
+            nbytes = ws.numel() - (base - ws.data_ptr())
         with profiling.region("vps_adjoint", medium.device):
             _lib.check(
                 _lib.load().rcv_render_backward_volpathsimple_ws(
                     C.byref(m), C.byref(s), C.byref(o), C.byref(fl), seed & 0xFFFFFFFF, spp, g.data_ptr(),
-                    gd.data_ptr(), ga.data_ptr() if ga is not None else None, base,
-                    ws.numel() - (base - ws.data_ptr()), st,
+                    gd.data_ptr(), ga.data_ptr() if ga is not None else None, base or None, nbytes, st,
                 ),
                 "rcv_render_backward_volpathsimple_ws",
             )
