@@ -10,7 +10,7 @@ from recursive_control_variates_gb300.plugins import twostatevolpath
 
 from test_gpu_volume import make_scene
 
-W, SPP = 512, 2
+W, SPP = 32, 512  # few pixels: what is zeroed stays below the size that torch splits over threads
 PATHS = W * W * SPP
 
 
