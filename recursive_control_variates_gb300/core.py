@@ -491,8 +491,8 @@ class _PackedMedium:
         grid = new.albedo_grid
         # what does not change from step to step, as bytes; a step fills in
         # the addresses of its states
-        key = (new.density.shape, None if grid is None else grid.shape, new.scale, new.albedo_value, self._factor(),
-               new.box)
+        key = (new.density.shape, None if grid is None else grid.shape, new.scale, tuple(new.albedo_value),
+               self._factor(), new.box)
         made = self.__dict__.get("_fixed")
         if made is None or made[0] != key:
             m = _lib.Medium()
