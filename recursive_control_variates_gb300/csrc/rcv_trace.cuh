@@ -880,7 +880,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
       }
       if (kMode == kTape && !tape_append(Q, tc, ev_walk && !ck_lost, x, ev_ref, ev_f)) ck_lost = true;
       if (sub >= steps) break;
-      ++n_iter;  // (a path's cost counts its steps)
+      ++n_iter;  // (a path's cost counts its steps, and those of its last round)
     }
 
     if (kMode == kTape && run_scat) {

@@ -26,8 +26,8 @@
 // one global counter and hands them to its idle lanes at the top of each loop
 // iteration, so a lane starts a new path as soon as its path ends and a warp
 // only drains at the end of the queue.  The main path and its NEE shadow walk
-// share one loop body ("one free-flight step per iteration") so that lanes in
-// different phases still execute the density lookup together.  Each path's
+// share one loop body (the same free-flight step, a few per iteration) so that
+// lanes in different phases still execute the density lookup together.  Each path's
 // radiance is written to a per-path slot; a separate pass sums a pixel's
 // samples in sample order, so results do not depend on the schedule.
 #pragma once
