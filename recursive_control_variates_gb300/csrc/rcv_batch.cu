@@ -383,18 +383,11 @@ static int validate_job(const rcv_batch_job* j, int idx) {
 // queue counters (two-state, adjoint radiance, replay, checkpoints / event
 // records, tape slots, lost paths, entered paths) | tracer counters | per-path radiance |
 // adjoint per-path total radiance | scatter checkpoints (tape: event records
-// and their weights) | event tape | camera-segment weights and paths
-// of those that entered the medium | lost-path list.
+// and their weights) | event tape | paths that entered the medium, replaced
+// by their camera-segment weights | lost-path list.
 struct PlanLayout {
-  uint64_t entries, two, adj, prefix, queue, counters, path_out, ltot, ckpt, tape, cam_w, entered, lost, total;
+  uint64_t entries, two, adj, prefix, queue, counters, path_out, ltot, ckpt, tape, cam_w, lost, total;
 };
-
-// A plan's scratch grows with its paths alone (the serving budget adds its
-// jobs' shares up): 2 checkpoints of 64 bytes per path, less the 4 bytes of the
-// entered paths' list, and kTapeSlotsPerPath tape slots.
-static int64_t batch_ckpt_capacity(int64_t paths) {
-  return kTapeSlotsPerPath / 8 * paths - paths / 16 + kCkptMargin;
-}
 
 static PlanLayout plan_layout(int n, int64_t total_two_paths, int64_t total_adj_paths) {
   PlanLayout L;
@@ -416,13 +409,11 @@ static PlanLayout plan_layout(int n, int64_t total_two_paths, int64_t total_adj_
   L.ltot = off;
   off = align256(off + uint64_t(total_adj_paths) * 16u);
   L.ckpt = off;
-  off = align256(off + uint64_t(batch_ckpt_capacity(total_adj_paths)) * 64u);
+  off = align256(off + uint64_t(ckpt_capacity(total_adj_paths, 0)) * 64u);
   L.tape = off;
   off = align256(off + uint64_t(tape_capacity(total_adj_paths, kTapeSlotsPerPath)) * 20u);
   L.cam_w = off;
   off = align256(off + uint64_t(total_adj_paths) * 8u);
-  L.entered = off;
-  off = align256(off + uint64_t(total_adj_paths) * 4u);
   L.lost = off;
   off = align256(off + uint64_t(total_adj_paths) * 4u);
   L.total = off;
@@ -679,7 +670,7 @@ extern "C" int rcv_batch_create(const rcv_batch_job* jobs, int32_t n, const rcv_
   b->path_out = reinterpret_cast<float4*>(w + P.path_out);
   b->adjbuf.ckpt = reinterpret_cast<float4*>(w + P.ckpt);
   b->adjbuf.ckpt_count = b->queue + 3;
-  b->adjbuf.ckpt_cap = batch_ckpt_capacity(adj_total);
+  b->adjbuf.ckpt_cap = ckpt_capacity(adj_total, 0);
   b->adjbuf.path_ltot = reinterpret_cast<float4*>(w + P.ltot);
   // (tape slots are 32-bit indices: batches of 2^28 gradient paths or more replay)
   b->tape = b->opt.adjoint == RCV_ADJOINT_TAPE && adj_total < (int64_t(1) << 28);
@@ -694,7 +685,7 @@ extern "C" int rcv_batch_create(const rcv_batch_job* jobs, int32_t n, const rcv_
     b->adjbuf.tape_f = tape_terms(w + P.tape, tape_capacity(adj_total, kTapeSlotsPerPath));
     b->tape_weights = reinterpret_cast<float4*>(w + P.ckpt + uint64_t(b->adjbuf.ckpt_cap) * 32u);
     b->adjbuf.cam_w = reinterpret_cast<float2*>(w + P.cam_w);
-    b->adjbuf.entered = reinterpret_cast<uint32_t*>(w + P.entered);
+    b->adjbuf.entered = reinterpret_cast<uint32_t*>(w + P.cam_w);  // (in place of the weights to come)
     b->adjbuf.entered_count = b->queue + 6;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);

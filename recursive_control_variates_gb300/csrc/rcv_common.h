@@ -161,6 +161,8 @@ inline int64_t tape_room(int64_t paths) {
 // replayed whole.  The tape adjoint keeps its 32-byte event records in the
 // first half of the same buffer and their 32-byte weights in the second.
 constexpr int64_t kCkptMargin = 65536;
+// (most 0: 2 per path, and the plan of a batch, whose scratch grows with its
+// paths alone: the serving budget adds its jobs' shares up)
 inline int64_t ckpt_capacity(int64_t paths, int64_t most) {
   return within_budget(paths, kTapeSlotsPerPath / 8, most, kTapeSlotBudget / 8) + kCkptMargin;
 }

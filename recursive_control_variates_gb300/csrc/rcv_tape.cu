@@ -72,7 +72,7 @@ __global__ void tape_weights_kernel(const __grid_constant__ VolJob single, const
                                     int njobs, const float4* __restrict__ rec,
                                     const unsigned long long* __restrict__ rec_count, int64_t rec_cap,
                                     float4* __restrict__ w, const float4* __restrict__ ltot,
-                                    const uint32_t* __restrict__ entered, float2* __restrict__ cam_w,
+                                    const uint32_t* entered, float2* cam_w,
                                     const unsigned long long* __restrict__ entered_count,
                                     int64_t clear_cells, int64_t clear_albedo, unsigned long long* replay_counter) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *replay_counter = 0ull;
@@ -109,7 +109,7 @@ __global__ void tape_weights_kernel(const __grid_constant__ VolJob single, const
       }
     }
     if (i < paths) {
-      const uint32_t path = entered[i];
+      const uint32_t path = entered[jobs != nullptr ? 2 * i : i];
       const float4 lt = ltot[path];
       float2 c = make_float2(0.0f, __int_as_float(-1));
       if (lt.w == 0.0f) {

@@ -541,7 +541,7 @@ __device__ void trace_persistent(const VolJob& single, const Queue& Q, Counts& c
             phase = kMain;
             if (kMode == kTape) {
               const uint32_t k = (uint32_t)atomicAdd(Q.entered_count, 1ull);
-              __stcs(Q.entered + k, (uint32_t)path);
+              __stcs(Q.entered + (kTable ? 2u * k : k), (uint32_t)path);
               tref = (kEvCamera << 30) | k;
             }
           }

@@ -131,7 +131,10 @@ struct Queue {
   // (scattering events), so that the gradient pass needs no grid lookup
   float* tape_f;
   // paths that entered the medium, and how many there are; the others have no
-  // events, and their total radiance is not kept either
+  // events, and their total radiance is not kept either.  A single job's list is
+  // kept from one replay call to the next; of a job table, whose step does both
+  // passes, it lies where each path's camera-segment weight will (every second
+  // word), so that a plan needs no memory for it
   uint32_t* entered;
   unsigned long long* entered_count;
 };

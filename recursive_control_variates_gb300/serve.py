@@ -96,8 +96,7 @@ class StepServer:
         gradient path (total radiance, scatter checkpoints or event records
         and their weights), and with the tape adjoint 16 x 20 + 8 + 4 bytes
         more (event slots with their extinction terms, camera-segment weight,
-        lost-path list; the list of paths that entered the medium takes its 4
-        bytes from the checkpoints)."""
+        whose place first holds the path, lost-path list)."""
         npix = job.width * job.height
         per_grad = 144 + (332 if self.options.adjoint == "tape" else 0)
         return job.nbytes() + 32 * npix * job.spp + per_grad * npix * job.spp_grad
