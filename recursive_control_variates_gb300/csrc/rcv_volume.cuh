@@ -231,6 +231,8 @@ __device__ __forceinline__ void tape_close(const Queue& Q, const TapeCursor& tc)
 // The jumps of the cooperative walk's lanes (up to 3 x 31 draws), read through
 // the L1: 16 bytes per lane instead of up to seven rounds of 64-bit squarings.
 static __device__ const PcgJumpTable kCoopJumps = make_pcg_jumps();
+static_assert(sizeof(PcgJump) == sizeof(ulonglong2) && alignof(PcgJump) >= alignof(ulonglong2),
+              "jumps are loaded as ulonglong2");
 
 // Lanes per path of a cooperative walk of n paths.
 constexpr int kCoopMost = 16;
