@@ -156,10 +156,8 @@ typedef struct rcv_volpath_options {
    * event of the radiance pass on a tape and scatters the gradient from it in
    * one flat pass; RCV_ADJOINT_REPLAY replays the paths' segments from
    * scattering checkpoints.  Both give the same gradient (up to the order of
-   * float additions).  Under a majorant supergrid the tape keeps each
-   * event's majorant beside it (at most 12 events per path); forward mode
-   * and jobs (or batches) of 2^28 gradient paths or more always replay.  The
-   * batched engine takes the same choice. */
+   * float additions).  Forward mode and jobs (or batches) of 2^28 gradient
+   * paths or more always replay.  The batched engine takes the same choice. */
   int32_t adjoint;
   /* Tape slots per path: paths whose events do not fit are replayed whole.  0 =
    * the most: max(16 per path, min(64 per path, 2^28)) in single-job calls, 16
@@ -650,8 +648,9 @@ typedef struct rcv_batch rcv_batch; /* opaque host handle of a batch plan */
 
 /* Shared device scratch of a batch: job tables, the per-path radiance of the
  * two-state launch (32 bytes per primal path of all jobs) and the adjoint's
- * per-path scratch (476 bytes per gradient path, as for
- * rcv_render_workspace_bytes).  opts->adjoint selects the tape or the replay
+ * per-path scratch (476 bytes per gradient path: total radiance, 2 scatter
+ * checkpoints or event records with their weights, 16 tape slots of 16 + 4
+ * bytes, camera-segment weight, lost-path list).  opts->adjoint selects the tape or the replay
  * tasks for the whole batch. */
 uint64_t rcv_batch_workspace_bytes(const rcv_batch_job* jobs, int32_t n);
 /* Plans a batch of n initialised jobs with launch options `opts` (batch,

@@ -22,8 +22,8 @@
 namespace rcv {
 
 // kBlocks: resident blocks per SM that the registers are bounded for: 7 (72
-// registers, up to 80 bytes spilled) but under an environment map, whose launches
-// end on longer paths, 6.  Steps at 6 / 7 blocks: 512^2 x (16 + 16) spp on 64^3
+// registers; without a supergrid 36 bytes spilled, 100 by job tables) but under
+// an environment map, whose launches end on longer paths, 6 (80, none spilled).  Steps at 6 / 7 blocks: 512^2 x (16 + 16) spp on 64^3
 // 1663 / 1630 us, 1024^2 on 256^3 8.84 / 8.66 ms, 24 mixed jobs 15.85 / 15.63 ms,
 // five map-lit 107 x 83 views 839 / 865 us; at 8 the paired launch was 2 to 8 %
 // slower than at 7 (with one step per iteration).

@@ -7,13 +7,12 @@
 // launch took 13.1 ms at a few lanes per instruction.  Here the adjoint is
 // two persistent launches with a few free-flight steps per loop iteration for
 // every lane, whatever its phase (as in rcv_trace.cuh), and two flat passes;
-// on the same film 0.94 + 0.80 + 0.26 + 0.11 ms (GB300; with one step per
-// iteration, before the reductions went pairwise: the whole step has gone from
-// 2.97 to 2.50 ms since).  The tracers are
+// on the same film 0.82 + 0.70 + 0.21 + 0.08 ms (GB300, launches one at a
+// time).  The tracers are
 // bound by the issue of divergent instructions and end on their longest
 // paths (a DRT path that follows its first path in the same lane and launch
-// gives 2.0 ms for the two tracers), the flat passes by the vector reductions
-// into the gradient:
+// gave 2.0 ms for the two tracers where two launches took 1.74), the flat
+// passes by the vector reductions into the gradient:
 //   kVpsTape  traces each path once.  It records every segment (64 bytes:
 //             the path, the NEE radiance gathered before it, its ray, its
 //             length, the NEE contribution at its end) and every step of a
